@@ -24,9 +24,9 @@ _dp = ctypes.POINTER(ctypes.c_double)
 
 
 def build():
-    """Compile the library from the reference tree (where it exists)."""
+    """Compile the library from the reference tree (where its sources are)."""
     import subprocess
-    if not os.path.isdir(REF_ROOT):
+    if not os.path.exists(os.path.join(REF_ROOT, "fmm3d_mpi", "kernel3d_mpi.cpp")):
         return False
     subprocess.check_call(["make", "-s", "-C", os.path.join(_HERE, "ref"), "REF=" + REF_ROOT])
     return os.path.exists(LIB_PATH)
