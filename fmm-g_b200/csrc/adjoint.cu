@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(AJ_THREADS)
 }
 
 // Multi-DOF transposed Hadamard step on the V-lists inverted per source slot:
-// out[s][f][j] = nrmfc * sum_{(t, id)} sum_i conj(T[id][f][j*TDM + i]) in[t][f][i].
+// out[s][j][f] = nrmfc * sum_{(t, id)} sum_i conj(T[id][f][j*TDM + i]) in[t][i][f].
 // A warp owns one source slot and 32 frequencies (lane = frequency).
 template <int SDM, int TDM>
 __global__ void __launch_bounds__(256)
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(256)
     const int2 en = lent[e];
     double2 d[TDM];
 #pragma unroll
-    for (int i = 0; i < TDM; i++) d[i] = in[((int64_t)en.x * nEff + f) * TDM + i];
+    for (int i = 0; i < TDM; i++) d[i] = in[((int64_t)en.x * TDM + i) * nEff + f];
     const double2* Tf = T + ((int64_t)en.y * nEff + f) * (SDM * TDM);
 #pragma unroll
     for (int j = 0; j < SDM; j++)
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(256)
   }
 #pragma unroll
   for (int j = 0; j < SDM; j++)
-    out[((int64_t)s * nEff + f) * SDM + j] = make_double2(acc[j].x * nrmfc, acc[j].y * nrmfc);
+    out[((int64_t)s * SDM + j) * nEff + f] = make_double2(acc[j].x * nrmfc, acc[j].y * nrmfc);
 }
 
 // Gradient of a scalar kernel with respect to the target position:

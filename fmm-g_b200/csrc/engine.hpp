@@ -68,6 +68,11 @@ struct DevState {
   // operators
   double *uc2ue = nullptr, *m2m = nullptr, *dc2de = nullptr, *l2l = nullptr;
   double2* m2lT = nullptr;
+  // translations of the vector kernels laid out for k_m2l_had_v64 / v32 (had_vec.cuh),
+  // and whether their 3 x 3 parts are symmetric
+  double2* hvT = nullptr;
+  float2* hvT32 = nullptr;
+  bool hvSym = true, hvSymOf64 = true, hvSymOf32 = true;  // of the tables; of the layouts held
   int16_t* transIdDev = nullptr;  // (rx+3)*49+(ry+3)*7+(rz+3) -> translation 0..315 or -1
   // per-evaluate work arrays
   double *den = nullptr, *val = nullptr, *uchk = nullptr, *uden = nullptr, *dchk = nullptr, *dden = nullptr;

@@ -28,11 +28,10 @@
 #include "gemm_tc.cuh"
 #include "had_pq.cuh"
 #include "had_smem.cuh"
+#include "had_vec.cuh"
 #include "kernels.hpp"
 
 namespace fmmg {
-
-__constant__ int16_t c_transId32[343];
 
 constexpr int MX_THREADS = 128;
 constexpr int MX_THREADS_FAR = 192;  // M2T: 2^6 x 3 also allows target groups of 24, 48, 96
@@ -816,237 +815,20 @@ __global__ void __launch_bounds__(32 * S2M_WARPS)
   }
 }
 
-// s += a b and s += a conj(b) as four FMAs into the accumulator (a product
-// formed first and then added costs a multiply and an add more: IEEE rules
-// keep the compiler from reassociating it)
-__device__ __forceinline__ void r8_cmac(float2& s, float2 a, float2 b) {
-  s.x = fmaf(a.x, b.x, s.x);
-  s.x = fmaf(-a.y, b.y, s.x);
-  s.y = fmaf(a.x, b.y, s.y);
-  s.y = fmaf(a.y, b.x, s.y);
-}
-__device__ __forceinline__ void r8_cmacc(float2& s, float2 a, float2 b) {
-  s.x = fmaf(a.x, b.x, s.x);
-  s.x = fmaf(a.y, b.y, s.x);
-  s.y = fmaf(a.y, b.x, s.y);
-  s.y = fmaf(-a.x, b.y, s.y);
-}
-
 // ------------------------------------------------------------------ FP32 M2L
-// grid (source slots, right-hand sides)
-template <int NP>
-__global__ void __launch_bounds__(128)
-    k_m2l_fwd32(const int32_t* __restrict__ nodes, const int32_t* __restrict__ depth, int rootLevel, Scale4 deg,
-                int sdm, const float* __restrict__ uden, int64_t udenRhs, const int32_t* __restrict__ ijk, int nUE,
-                float2* __restrict__ effDen, int64_t effRhs, int nEff) {
-  using F = FftDims32<NP>;
-  constexpr int N = F::N, NH = F::NH, H = F::H;
-  __shared__ float cube[NP * NP * NP];
-  __shared__ float2 X1[NP * NP * NH];
-  __shared__ float2 X2[NP * N * NH];
-  __shared__ float2 tw[N];
-  const int slot = blockIdx.x;
-  const int v = nodes[slot];
-  const int tid = threadIdx.x;
-  if (tid < N) {
-    double s, c;
-    sincospi(2.0 * tid / N, &s, &c);
-    tw[tid] = make_float2((float)c, (float)-s);
-  }
-  const int l = depth[v] + rootLevel;
-  const float* ud = uden + blockIdx.y * udenRhs + (int64_t)v * nUE * sdm;
-  float2* out = effDen + blockIdx.y * effRhs + (int64_t)slot * nEff * sdm;
-  for (int m = 0; m < sdm; m++) {
-    const float scl = (float)exp2(l * deg.v[m]);
-    for (int i = tid; i < NP * NP * NP; i += blockDim.x) cube[i] = 0.f;
-    __syncthreads();
-    for (int i = tid; i < nUE; i += blockDim.x) {
-      int p = ijk[i];
-      cube[((p >> 16) * NP + ((p >> 8) & 255)) * NP + (p & 255)] = ud[(int64_t)i * sdm + m] * scl;
-    }
-    __syncthreads();
-    for (int e = tid; e < NP * NP * NH; e += blockDim.x) {
-      int kx = e % NH, yb = (e / NH) % NP, zb = e / (NH * NP);
-      float2 s = make_float2(0.f, 0.f);
-      const float* row = &cube[(zb * NP + yb) * NP];
-#pragma unroll
-      for (int xb = 0; xb < NP; xb++) {
-        float2 w = tw[(kx * (xb + H)) % N];
-        s.x += row[xb] * w.x;
-        s.y += row[xb] * w.y;
-      }
-      X1[e] = s;
-    }
-    __syncthreads();
-    for (int e = tid; e < NP * N * NH; e += blockDim.x) {
-      int kx = e % NH, ky = (e / NH) % N, zb = e / (NH * N);
-      float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int yb = 0; yb < NP; yb++) {
-        r8_cmac(s, X1[(zb * NP + yb) * NH + kx], tw[(ky * (yb + H)) % N]);
-      }
-      X2[e] = s;
-    }
-    __syncthreads();
-    for (int e = tid; e < N * N * NH; e += blockDim.x) {
-      int kx = e % NH, ky = (e / NH) % N, kz = e / (NH * N);
-      float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int zb = 0; zb < NP; zb++) {
-        r8_cmac(s, X2[(zb * N + ky) * NH + kx], tw[(kz * (zb + H)) % N]);
-      }
-      out[(int64_t)e * sdm + m] = s;
-    }
-    __syncthreads();
-  }
-}
-
-// grid (target parents, 32-frequency chunks, RHS blocks); warp c owns child c;
-// each translation spectrum value is loaded once and applied to KB densities.
-// The parent's neighbour entries (the 8 input child slots resolved at setup,
-// the offset code) are staged in shared memory once for the CTA, 32 at a
-// time, so each (neighbour, child) pair starts on shared-memory reads instead
-// of a chain of dependent global loads (neighbour -> its children -> slot).
-template <int SDM, int TDM, int KB>
-__global__ void __launch_bounds__(256)
-    k_m2l_had32(const int32_t* __restrict__ rowOut, const int64_t* __restrict__ vPtr,
-                const int8_t* __restrict__ vOff, const int32_t* __restrict__ nIn,
-                const float2* __restrict__ effDen, int64_t denRhs, const float2* __restrict__ T,
-                float2* __restrict__ effVal, int64_t valRhs, int nEff, int nrhs, float nrmfc) {
-  __shared__ int sSl[32 * 8];
-  __shared__ int sOf[32];
-  const int b = blockIdx.x;
-  const int c = threadIdx.x >> 5;
-  const int f = blockIdx.y * 32 + (threadIdx.x & 31);
-  const int rhs0 = blockIdx.z * KB;
-  const int ts = rowOut[8 * b + c];
-  const int cx = c >> 2, cy = (c >> 1) & 1, cz = c & 1;
-  float2 acc[KB][TDM];
-#pragma unroll
-  for (int q = 0; q < KB; q++)
-#pragma unroll
-    for (int i = 0; i < TDM; i++) acc[q][i] = make_float2(0.f, 0.f);
-  const bool live = ts >= 0 && f < nEff;  // every thread stays for the CTA's barriers
-  const int64_t e1 = vPtr[b + 1];
-  for (int64_t e0 = vPtr[b]; e0 < e1; e0 += 32) {
-    const int ne = (int)min((int64_t)32, e1 - e0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < ne * 8; i += blockDim.x) sSl[i] = nIn[8 * e0 + i];
-    if (threadIdx.x < ne) sOf[threadIdx.x] = vOff[e0 + threadIdx.x];
-    __syncthreads();
-    if (!live) continue;
-    for (int j = 0; j < ne; j++) {
-      const int off = sOf[j];
-      const int dx = off / 9 - 1, dy = (off / 3) % 3 - 1, dz = off % 3 - 1;
-#pragma unroll 1
-      for (int c2 = 0; c2 < 8; c2++) {
-        const int s = sSl[j * 8 + c2];
-        if (s < 0) continue;
-        const int rx = 2 * dx + (c2 >> 2) - cx, ry = 2 * dy + ((c2 >> 1) & 1) - cy, rz = 2 * dz + (c2 & 1) - cz;
-        if (max(abs(rx), max(abs(ry), abs(rz))) <= 1) continue;
-        const int id = c_transId32[(rx + 3) * 49 + (ry + 3) * 7 + (rz + 3)];
-        const float2* Tf = T + ((int64_t)id * nEff + f) * (SDM * TDM);
-        float2 tv[SDM * TDM];
-#pragma unroll
-        for (int jj = 0; jj < SDM * TDM; jj++) tv[jj] = Tf[jj];
-#pragma unroll
-        for (int q = 0; q < KB; q++) {
-          if (rhs0 + q >= nrhs) break;
-          const float2* dp = effDen + (rhs0 + q) * denRhs + ((int64_t)s * nEff + f) * SDM;
-#pragma unroll
-          for (int jj = 0; jj < SDM; jj++) {
-            const float2 d = dp[jj];
-#pragma unroll
-            for (int i = 0; i < TDM; i++) {
-              const float2 w = tv[jj * TDM + i];
-              acc[q][i].x += w.x * d.x - w.y * d.y;
-              acc[q][i].y += w.x * d.y + w.y * d.x;
-            }
-          }
-        }
-      }
-    }
-  }
-  if (live) {
-#pragma unroll
-    for (int q = 0; q < KB; q++) {
-      if (rhs0 + q >= nrhs) break;
-#pragma unroll
-      for (int i = 0; i < TDM; i++)
-        effVal[(rhs0 + q) * valRhs + ((int64_t)ts * nEff + f) * TDM + i] =
-            make_float2(acc[q][i].x * nrmfc, acc[q][i].y * nrmfc);
-    }
-  }
-}
-
-// grid (target slots, right-hand sides)
-template <int NP>
-__global__ void __launch_bounds__(128)
-    k_m2l_inv32(const int32_t* __restrict__ nodes, const float2* __restrict__ effVal, int64_t valRhs, int nEff,
-                int tdm, const int32_t* __restrict__ ijk, int nDC, float* __restrict__ dchk, int64_t dchkRhs) {
-  using F = FftDims32<NP>;
-  constexpr int N = F::N, NH = F::NH, H = F::H;
-  __shared__ float2 Y2[NP * N * NH];
-  __shared__ float2 Y1[NP * NP * NH];
-  __shared__ float2 tw[N];
-  const int slot = blockIdx.x;
-  const int node = nodes[slot];
-  const int tid = threadIdx.x;
-  if (tid < N) {
-    double s, c;
-    sincospi(2.0 * tid / N, &s, &c);
-    tw[tid] = make_float2((float)c, (float)-s);
-  }
-  __syncthreads();
-  const float2* in = effVal + blockIdx.y * valRhs + (int64_t)slot * nEff * tdm;
-  float* dc = dchk + blockIdx.y * dchkRhs + (int64_t)node * nDC * tdm;
-  for (int m = 0; m < tdm; m++) {
-    for (int e = tid; e < NP * N * NH; e += blockDim.x) {
-      int kx = e % NH, ky = (e / NH) % N, zb = e / (NH * N);
-      float2 s = make_float2(0.f, 0.f);
-#pragma unroll 4
-      for (int kz = 0; kz < N; kz++) {
-        r8_cmacc(s, in[((int64_t)(kz * N + ky) * NH + kx) * tdm + m], tw[(kz * (zb + H)) % N]);
-      }
-      Y2[e] = s;
-    }
-    __syncthreads();
-    for (int e = tid; e < NP * NP * NH; e += blockDim.x) {
-      int kx = e % NH, yb = (e / NH) % NP, zb = e / (NH * NP);
-      float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int ky = 0; ky < N; ky++) {
-        r8_cmacc(s, Y2[(zb * N + ky) * NH + kx], tw[(ky * (yb + H)) % N]);
-      }
-      Y1[e] = s;
-    }
-    __syncthreads();
-    for (int i = tid; i < nDC; i += blockDim.x) {
-      int p = ijk[i];
-      int a = p & 255, b = (p >> 8) & 255, cc = p >> 16;
-      const float2* y1 = &Y1[(cc * NP + b) * NH];
-      const int x = a + H;
-      float s = 0.f;
-#pragma unroll
-      for (int kx = 0; kx < NH; kx++) {
-        float2 t = cmulc(y1[kx], tw[(kx * x) % N]);
-        s += (kx == 0 || 2 * kx == N) ? t.x : 2.f * t.x;  // the Nyquist term only for even N
-      }
-      dc[(int64_t)i * tdm + m] += s;
-    }
-    __syncthreads();
-  }
-}
-
-// Scalar equivalent kernels, blocks of 8 right-hand sides: one CTA per
-// (slot, block) transforms the 8 densities together.  Each pass is a set of
-// 1-D DFTs along one axis: a thread owns one line of one right-hand side,
-// reads its np (or N) inputs from shared memory once and produces all the
-// line's outputs, so shared-memory traffic is one read per input (the kernels
-// are bound by it otherwise).  Shared staging arrays are planes [8][...]
-// padded against bank conflicts; in global memory the spectra are written
-// (and read back by k_m2l_inv32r8) as [block][slot][frequency][8], the
-// forward's last pass ordered right-hand side fastest for contiguous writes.
+// Spectral transforms, every equivalent kernel: one CTA transforms 8 planes, a
+// plane being one component of one right-hand side of one slot.  The spectra
+// are laid out [block of RW right-hand sides][slot][component][frequency][RW]
+// (RW = 1, 2, 4 or 8), so plane p of a block is right-hand side p % RW of
+// component p / RW % dof of slot p / RW / dof: 8 right-hand sides of a scalar
+// slot, 2 components of 4 right-hand sides, or 8 components and slots of one.
+// Each pass is a set of 1-D DFTs along one axis: a thread owns one line of one
+// plane, reads its np (or N) inputs from shared memory once and produces all
+// the line's outputs, so shared-memory traffic is one read per input (the
+// kernels are bound by it otherwise).  Shared staging arrays are planes
+// [8][...] padded against bank conflicts; the pass that writes (the forward's
+// last) or reads (the inverse's first) the spectra runs right-hand sides, then
+// kx fastest: runs of 8 RW NH contiguous bytes.
 // The grid is FftDims32 (N = 2np - 1 points per axis); the twiddles of every
 // pass come from one table twb[k][b] = exp(-2 pi i k (b + np/2) / N).  Dynamic
 // shared memory r8_fwd_smem<NP>() / r8_inv_smem<NP>().
@@ -1065,19 +847,20 @@ constexpr size_t r8_inv_smem() {  // Y1 + Y2 (padded planes) + twiddles + roots
   return sizeof(float2) * (8 * r8_pad(NP * NP * F::NH) + 8 * r8_pad(NP * F::N * F::NH) + F::N * NP + F::N);
 }
 
-__device__ __forceinline__ void r8_load(const float2* p, float2 (&v)[8]) {
-  const float4* q = reinterpret_cast<const float4*>(p);
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const float4 t = q[i];
-    v[2 * i] = make_float2(t.x, t.y);
-    v[2 * i + 1] = make_float2(t.z, t.w);
-  }
+// LG: log2 of RW where it is known (3), so the strides are constants; -1 takes
+// the argument
+template <int LG>
+__device__ __forceinline__ int r8_lg(int lgRW) {
+  return LG >= 0 ? LG : lgRW;
 }
-__device__ __forceinline__ void r8_store(float2* p, const float2 (&v)[8]) {
-  float4* q = reinterpret_cast<float4*>(p);
-#pragma unroll
-  for (int i = 0; i < 4; i++) q[i] = make_float4(v[2 * i].x, v[2 * i].y, v[2 * i + 1].x, v[2 * i + 1].y);
+// the (plane, kx, ky) of item i of the pass over the spectra: right-hand side
+// fastest, then kx, then the other planes, then ky
+template <int NH>
+__device__ __forceinline__ void r8_item(int i, int lgRW, int& plane, int& kx, int& ky) {
+  const int rr = i & ((1 << lgRW) - 1), q = i >> lgRW, hi = q / NH, lgHi = 3 - lgRW;
+  kx = q - hi * NH;
+  plane = ((hi & ((1 << lgHi) - 1)) << lgRW) | rr;
+  ky = hi >> lgHi;
 }
 template <int NP>
 __device__ __forceinline__ void r8_twiddles(float2* twb, float2* roots) {
@@ -1092,10 +875,9 @@ __device__ __forceinline__ void r8_twiddles(float2* twb, float2* roots) {
 // The line transforms with the twiddles in registers: twb[k][b] is the root
 // w^m, m = k (b + H) mod N, so with both loops unrolled each product names
 // its root at compile time and the N roots are held per thread as packed
-// pairs.  Forward products s += a w (r8_cmac) take (w.x, w.y) and (w.y, w.x);
-// inverse products s += a conj(w) (r8_cmacc) take (w.x, w.x) and (w.y, w.y).
-// Each is two packed FP32x2 FMAs with the same per-component order as the
-// scalar helpers, so the results are the same.
+// pairs.  Forward products s += a w take (w.x, w.y) and (w.y, w.x); inverse
+// products s += a conj(w) take (w.x, w.x) and (w.y, w.y).  Each is two packed
+// FP32x2 FMAs.
 template <int N, int H>
 struct R8Idx {
   static constexpr int at(int k, int b) { return (k * (b + H)) % N; }
@@ -1111,11 +893,12 @@ __device__ __forceinline__ void r8_cmacc2(unsigned long long& s, unsigned long l
   pq_fma2(s, aswp, wyy);  // (s.x + a.y w.y, s.y - a.x w.y)
 }
 
-template <int NP>
+template <int NP, int LG>
 __global__ void __launch_bounds__(256)
-    k_m2l_fwd32r8(const int32_t* __restrict__ nodes, const int32_t* __restrict__ depth, int rootLevel, float deg,
-                  const float* __restrict__ uden, int64_t udenRhs, const int32_t* __restrict__ ijk, int nUE,
-                  float2* __restrict__ effDen, int64_t blkStride, int nEff, int kc) {
+    k_m2l_fwd32r8(int nPlanes, int lgRWarg, const int32_t* __restrict__ nodes, const int32_t* __restrict__ depth,
+                  int rootLevel, Scale4 deg, int sdm, const float* __restrict__ uden, int64_t udenRhs,
+                  const int32_t* __restrict__ ijk, int nUE, float2* __restrict__ effDen, int64_t blkStride, int nEff,
+                  int kc) {
   using F = FftDims32<NP>;
   constexpr int N = F::N, NH = F::NH;
   constexpr int S1 = r8_pad(NP * NP * NH), S2 = r8_pad(NP * N * NH), S3 = NP * NP * NP;
@@ -1125,21 +908,30 @@ __global__ void __launch_bounds__(256)
   float2* twb = X2 + S2 * 8;                             // [N][NP]
   float2* roots = twb + N * NP;                          // [N]
   float* cube = reinterpret_cast<float*>(roots + N);     // [8][NP][NP][NP]
-  const int slot = blockIdx.x;
-  const int v = nodes[slot];
-  const int r0 = blockIdx.y * 8;
+  __shared__ const float* pIn[8];  // the planes' densities (null past the last plane or right-hand side)
+  __shared__ float pScl[8];
+  const int lgRW = r8_lg<LG>(lgRWarg);
+  const int p0 = blockIdx.x * 8, RW = 1 << lgRW;
   const int tid = threadIdx.x;
   using IX = R8Idx<N, F::H>;
   r8_twiddles<NP>(twb, roots);
-  const float scl = (float)exp2((double)(depth[v] + rootLevel) * deg);
+  if (tid < 8) {
+    const int p = p0 + tid, sm = p >> lgRW, m = sm % sdm, rhs = blockIdx.y * RW + (p & (RW - 1));
+    pIn[tid] = nullptr;
+    if (p < nPlanes && rhs < kc) {
+      const int v = nodes[sm / sdm];
+      pIn[tid] = uden + (int64_t)rhs * udenRhs + (int64_t)v * nUE * sdm + m;
+      pScl[tid] = (float)exp2((double)(depth[v] + rootLevel) * (m == 0 ? deg.v[0] : m == 1 ? deg.v[1] : m == 2 ? deg.v[2] : deg.v[3]));
+    }
+  }
   for (int i = tid; i < S3 * 8; i += blockDim.x) cube[i] = 0.f;
   __syncthreads();
   for (int i = tid; i < nUE * 8; i += blockDim.x) {  // surface point fastest: coalesced reads of each plane
     const int j = i % nUE, r = i / nUE;
-    if (r0 + r >= kc) continue;
+    const float* in = pIn[r];
+    if (!in) continue;
     const int p = ijk[j];
-    cube[r * S3 + ((p >> 16) * NP + ((p >> 8) & 255)) * NP + (p & 255)] =
-        uden[(int64_t)(r0 + r) * udenRhs + (int64_t)v * nUE + j] * scl;
+    cube[r * S3 + ((p >> 16) * NP + ((p >> 8) & 255)) * NP + (p & 255)] = in[(int64_t)j * sdm] * pScl[r];
   }
   __syncthreads();
   unsigned long long wp[N], ws[N];  // the roots as (w.x, w.y) and (w.y, w.x)
@@ -1149,7 +941,7 @@ __global__ void __launch_bounds__(256)
     wp[m] = pq_pk(w.x, w.y);
     ws[m] = pq_pk(w.y, w.x);
   }
-  // x pass (real -> half spectrum): a thread owns one x line of one right-hand side
+  // x pass (real -> half spectrum): a thread owns one x line of one plane
   for (int i = tid; i < NP * NP * 8; i += blockDim.x) {
     const int row = i % (NP * NP), r = i / (NP * NP);  // row = zb * NP + yb
     unsigned long long cc[NP];
@@ -1167,8 +959,7 @@ __global__ void __launch_bounds__(256)
     }
   }
   __syncthreads();
-  // y pass: a thread owns one y line (kx, zb) of one right-hand side and all N
-  // ky outputs
+  // y pass: a thread owns one y line (kx, zb) of one plane and all N ky outputs
   for (int i = tid; i < NH * NP * 8; i += blockDim.x) {
     const int kx = i % NH, zb = (i / NH) % NP, r = i / (NH * NP);
     unsigned long long axx[NP], nayy[NP];
@@ -1187,11 +978,12 @@ __global__ void __launch_bounds__(256)
     }
   }
   __syncthreads();
-  // z pass: a thread owns one z line (kx, ky) of one right-hand side and all N kz
-  // outputs; right-hand side fastest so the global writes are contiguous
-  float2* out = effDen + blockIdx.y * blkStride + (int64_t)slot * nEff * 8;
+  // z pass: a thread owns one z line (kx, ky) of one plane and all N kz outputs
   for (int i = tid; i < NH * N * 8; i += blockDim.x) {
-    const int r = i & 7, kx = (i >> 3) % NH, ky = (i >> 3) / NH;
+    int r, kx, ky;
+    r8_item<NH>(i, lgRW, r, kx, ky);
+    if (p0 + r >= nPlanes) continue;
+    float2* out = effDen + blockIdx.y * blkStride + (int64_t)((p0 + r) >> lgRW) * nEff * RW + (r & (RW - 1));
     unsigned long long axx[NP], nayy[NP];
 #pragma unroll
     for (int zb = 0; zb < NP; zb++) {
@@ -1204,7 +996,7 @@ __global__ void __launch_bounds__(256)
       unsigned long long s = 0ull;
 #pragma unroll
       for (int zb = 0; zb < NP; zb++) r8_cmac2(s, axx[zb], nayy[zb], wp[IX::at(kz, zb)], ws[IX::at(kz, zb)]);
-      out[((int64_t)(kz * N + ky) * NH + kx) * 8 + r] = pq_unpk(s);
+      out[((kz * N + ky) * NH + kx) * RW] = pq_unpk(s);
     }
   }
 }
@@ -1213,10 +1005,11 @@ __global__ void __launch_bounds__(256)
 // 32 lanes read 256 contiguous bytes and every element is read once, so the
 // CTA needs no staging space (4 CTAs per SM at np = 6; staging the 64.5 KB
 // block in shared memory first allowed 2 and measured 1.3x slower).
-template <int NP>
+template <int NP, int LG>
 __global__ void __launch_bounds__(256)
-    k_m2l_inv32r8(const int32_t* __restrict__ nodes, const float2* __restrict__ effVal, int64_t blkStride, int nEff,
-                  const int32_t* __restrict__ ijk, int nDC, float* __restrict__ dchk, int64_t dchkRhs, int kc) {
+    k_m2l_inv32r8(int nPlanes, int lgRWarg, const int32_t* __restrict__ nodes, const float2* __restrict__ effVal,
+                  int64_t blkStride, int nEff, int tdm, const int32_t* __restrict__ ijk, int nDC,
+                  float* __restrict__ dchk, int64_t dchkRhs, int kc) {
   using F = FftDims32<NP>;
   constexpr int N = F::N, NH = F::NH;
   constexpr int S1 = r8_pad(NP * NP * NH), S2 = r8_pad(NP * N * NH);
@@ -1225,12 +1018,17 @@ __global__ void __launch_bounds__(256)
   float2* Y2 = Y1 + S1 * 8;                          // [8][NP][N][NH]
   float2* twb = Y2 + S2 * 8;                         // [N][NP]
   float2* roots = twb + N * NP;                      // [N]
-  const int slot = blockIdx.x;
-  const int node = nodes[slot];
-  const int r0 = blockIdx.y * 8;
+  __shared__ float* pOut[8];  // the planes' check potentials (null past the last plane or right-hand side)
+  const int lgRW = r8_lg<LG>(lgRWarg);
+  const int p0 = blockIdx.x * 8, RW = 1 << lgRW;
   const int tid = threadIdx.x;
   using IX = R8Idx<N, F::H>;
-  const float2* Xg = effVal + blockIdx.y * blkStride + (int64_t)slot * nEff * 8;
+  if (tid < 8) {
+    const int p = p0 + tid, sm = p >> lgRW, rhs = blockIdx.y * RW + (p & (RW - 1));
+    pOut[tid] = p < nPlanes && rhs < kc
+                    ? dchk + (int64_t)rhs * dchkRhs + (int64_t)nodes[sm / tdm] * nDC * tdm + sm % tdm
+                    : nullptr;
+  }
   r8_twiddles<NP>(twb, roots);
   __syncthreads();
   unsigned long long wxx[N], wyy[N];  // the roots as (w.x, w.x) and (w.y, w.y)
@@ -1240,13 +1038,15 @@ __global__ void __launch_bounds__(256)
     wxx[m] = pq_pk(w.x, w.x);
     wyy[m] = pq_pk(w.y, w.y);
   }
-  // z pass, band outputs only: a thread owns one z line (kx, ky) of one
-  // right-hand side, right-hand side fastest as in HBM
+  // z pass, band outputs only: a thread owns one z line (kx, ky) of one plane
   for (int i = tid; i < NH * N * 8; i += blockDim.x) {
-    const int r = i & 7, kx = (i >> 3) % NH, ky = (i >> 3) / NH;
+    int r, kx, ky;
+    r8_item<NH>(i, lgRW, r, kx, ky);
+    if (p0 + r >= nPlanes) continue;
+    const float2* Xg = effVal + blockIdx.y * blkStride + (int64_t)((p0 + r) >> lgRW) * nEff * RW + (r & (RW - 1));
     float2 c[N];
 #pragma unroll
-    for (int kz = 0; kz < N; kz++) c[kz] = Xg[((kz * N + ky) * NH + kx) * 8 + r];  // all loads of the line first
+    for (int kz = 0; kz < N; kz++) c[kz] = Xg[((kz * N + ky) * NH + kx) * RW];  // all loads of the line first
     unsigned long long s[NP];
 #pragma unroll
     for (int zb = 0; zb < NP; zb++) s[zb] = 0ull;
@@ -1260,7 +1060,7 @@ __global__ void __launch_bounds__(256)
     for (int zb = 0; zb < NP; zb++) Y2[r * S2 + (zb * N + ky) * NH + kx] = pq_unpk(s[zb]);
   }
   __syncthreads();
-  // y pass: a thread owns one y line (kx, zb) of one right-hand side
+  // y pass: a thread owns one y line (kx, zb) of one plane
   for (int i = tid; i < NH * NP * 8; i += blockDim.x) {
     const int kx = i % NH, zb = (i / NH) % NP, r = i / (NH * NP);
     unsigned long long s[NP];
@@ -1279,7 +1079,8 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   for (int i = tid; i < nDC * 8; i += blockDim.x) {  // x pass (c2r) at the surface points
     const int j = i % nDC, r = i / nDC;
-    if (r0 + r >= kc) continue;
+    float* dst = pOut[r];
+    if (!dst) continue;
     const int p = ijk[j];
     const int a = p & 255, b = (p >> 8) & 255, cc = p >> 16;
     const float2* y1 = &Y1[r * S1 + (cc * NP + b) * NH];
@@ -1289,7 +1090,7 @@ __global__ void __launch_bounds__(256)
       const float2 w = twb[kx * NP + a];
       s += ((kx == 0 || 2 * kx == N) ? 1.f : 2.f) * cmulc(y1[kx], w).x;
     }
-    dchk[(int64_t)(r0 + r) * dchkRhs + (int64_t)node * nDC + j] += s;
+    dst[(int64_t)j * tdm] += s;
   }
 }
 
@@ -1373,6 +1174,22 @@ static void m2t_items(const Plan& P, int numSMs, std::vector<int4>& items, std::
   std::vector<int4> sorted(items.size());
   for (size_t i = 0; i < order.size(); i++) sorted[i] = items[order[i]];
   items.swap(sorted);
+}
+
+// the vector kernels' FP32 translations for k_m2l_had_v32, in symmetric blocks
+// where the FP64 tables are symmetric (D.hvSym)
+template <int SDM, int TDM>
+static std::string hv_layout32(const Plan& P, DevState& D) {
+  if (!D.hvT32 || D.hvSymOf32 != D.hvSym) {
+    const int64_t n = D.hvSym ? hv_table_size<float2, SDM, TDM, true>(P.nEff32)
+                              : hv_table_size<float2, SDM, TDM, false>(P.nEff32);
+    FMMG_TRY(dalloc(D, D.hvT32, (size_t)n));
+  }
+  D.hvSymOf32 = D.hvSym;
+  if (D.hvSym) launch_hv_pack<float2, SDM, TDM, true>(D.stream, D.m2lT32, D.transIdDev, P.nEff32, D.hvT32);
+  else launch_hv_pack<float2, SDM, TDM, false>(D.stream, D.m2lT32, D.transIdDev, P.nEff32, D.hvT32);
+  FMMG_CK(cudaGetLastError());
+  return std::string();
 }
 
 static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
@@ -1494,6 +1311,8 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     std::vector<float2> t(P.m2lT32.size());
     for (size_t i = 0; i < t.size(); i++) t[i] = make_float2((float)P.m2lT32[i].real(), (float)P.m2lT32[i].imag());
     FMMG_CK(cudaMemcpy(D.m2lT32, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    if (P.sdm == 4) FMMG_TRY((hv_layout32<4, 3>(P, D)));
+    else if (P.sdm == 3) FMMG_TRY((hv_layout32<3, 3>(P, D)));
     if (D.m2lTw32) {  // combined translations of the 27-product Hadamard (had_pq.cuh), FP64 sums
       auto w = [](int code, int d) -> double {
         if (code == 0) return d == 0 ? 1.0 : 0.0;
@@ -1525,9 +1344,6 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
       }
       FMMG_CK(cudaMemcpy(D.m2lTw32, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice));
     }
-    int16_t tid[343];
-    for (int i = 0; i < 343; i++) tid[i] = (int16_t)P.transId[i / 49][(i / 7) % 7][i % 7];
-    FMMG_CK(cudaMemcpyToSymbol(c_transId32, tid, sizeof(tid)));
     D.mixedOpsStale = false;
   }
   return std::string();
@@ -1638,17 +1454,32 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
   cudaEventRecord(D.ev[EV_NEAR], st);
   const int nsrc = (int)P.vSrcNodes.size(), ntrg = (int)P.vTrgNodes.size(), npar = (int)P.vParents.size();
   const int64_t effDR = (int64_t)nsrc * P.nEff32 * P.sdm, effVR = (int64_t)ntrg * P.nEff32 * P.tdm;
-  const bool r8 = P.sdm == 1 && P.tdm == 1 && kc >= 2 && D.hadPQ;  // blocks of 8 interleaved right-hand sides
-  const int nblk = (kc + 7) / 8;
-  const int64_t blkDen = (int64_t)nsrc * P.nEff32 * 8, blkVal = (int64_t)ntrg * P.nEff32 * 8;
-  if ((mask & 4) && nsrc > 0 && r8) {
+  // Spectra in blocks of RW interleaved right-hand sides.  Scalar kernels: 8,
+  // or 1 for a single right-hand side and for the list form.  Vector kernels:
+  // the smallest power of two that holds them, 4 instead of 8 where that
+  // leaves fewer right-hand sides of padding.
+  const bool scalar = P.sdm == 1 && P.tdm == 1;
+  const bool r8 = scalar && kc >= 2 && D.hadPQ;
+  int lgRW = r8 ? 3 : 0;
+  if (!scalar) {
+    while (lgRW < 3 && (1 << lgRW) < kc) lgRW++;
+    if (lgRW == 3 && (kc + 3) / 4 * 4 < (kc + 7) / 8 * 8) lgRW = 2;
+  }
+  const int RW = 1 << lgRW, nblk = (kc + RW - 1) / RW;
+  const int64_t blkDen = effDR * RW, blkVal = effVR * RW;
+  const int denPlanes = nsrc * P.sdm * RW, valPlanes = ntrg * P.tdm * RW;
+  if ((mask & 4) && nsrc > 0) {
+    Scale4 deg;
+    deg.mod = P.sdm;
+    for (int k = 0; k < 4; k++) deg.v[k] = k < P.sdm ? P.deg[k] : 0.0;
 #define FMMG_FWD32R8(NP_)                                                                                      \
   do {                                                                                                         \
     constexpr size_t sm = r8_fwd_smem<NP_>();                                                                  \
-    cudaFuncSetAttribute(k_m2l_fwd32r8<NP_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);            \
-    k_m2l_fwd32r8<NP_><<<dim3(nsrc, nblk), 256, sm, st>>>(D.vSrcNodes, D.depth, rl, (float)P.deg[0], D.uden32, \
-                                                          nn * ue, D.surfIJK, P.nUE, D.effDen32, blkDen,       \
-                                                          P.nEff32, kc);                                         \
+    auto* kf = lgRW == 3 ? k_m2l_fwd32r8<NP_, 3> : k_m2l_fwd32r8<NP_, -1>;                                      \
+    cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);                            \
+    kf<<<dim3((denPlanes + 7) / 8, nblk), 256, sm, st>>>(                                                      \
+        denPlanes, lgRW, D.vSrcNodes, D.depth, rl, deg, P.sdm, D.uden32, nn * ue, D.surfIJK, P.nUE,            \
+        D.effDen32, blkDen, P.nEff32, kc);                                                                     \
   } while (0)
     switch (P.o.np) {
       case 3: FMMG_FWD32R8(3); break;
@@ -1660,42 +1491,21 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
     }
 #undef FMMG_FWD32R8
     ls->launches++;
-  } else if ((mask & 4) && nsrc > 0) {
-    Scale4 deg;
-    deg.mod = P.sdm;
-    for (int k = 0; k < 4; k++) deg.v[k] = P.deg[k];
-#define FMMG_FWD32(NP_)                                                                                         \
-  k_m2l_fwd32<NP_><<<dim3(nsrc, kc), 128, 0, st>>>(D.vSrcNodes, D.depth, rl, deg, P.sdm, D.uden32, nn * ue,    \
-                                                    D.surfIJK, P.nUE, D.effDen32, effDR, P.nEff32)
-    switch (P.o.np) {
-      case 3: FMMG_FWD32(3); break;
-      case 4: FMMG_FWD32(4); break;
-      case 5: FMMG_FWD32(5); break;
-      case 6: FMMG_FWD32(6); break;
-      case 7: FMMG_FWD32(7); break;
-      case 8: FMMG_FWD32(8); break;
-    }
-#undef FMMG_FWD32
-    ls->launches++;
   }
   cudaEventRecord(D.ev[EV_M2L_FWD], st);
   if ((mask & 4) && npar > 0 && ntrg > 0) {
-    dim3 grid(npar, (P.nEff32 + 31) / 32, kb);
     const float nrmfc = 1.0f / float(P.nReg32);
-    // vector kernels: 8 right-hand sides a thread when there are more than 4
-    // (each translation value loaded serves twice the multiply-adds; the pair
-    // kernels keep their 4)
-#define FMMG_HAD32(SD_, TD_)                                                                                   \
-  do {                                                                                                         \
-    if (kc > 4)                                                                                                \
-      k_m2l_had32<SD_, TD_, 8><<<dim3(npar, (P.nEff32 + 31) / 32, (kc + 7) / 8), 256, 0, st>>>(                \
-          D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen32, effDR, D.m2lT32, D.effVal32, effVR, P.nEff32, kc,   \
-          nrmfc);                                                                                              \
-    else                                                                                                       \
-      k_m2l_had32<SD_, TD_, KB><<<grid, 256, 0, st>>>(D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen32, effDR, \
-                                                       D.m2lT32, D.effVal32, effVR, P.nEff32, kc, nrmfc);      \
-  } while (0)
-    if (P.sdm == 1 && P.tdm == 1 && D.hadPQ) {
+#define FMMG_HADV(SD_, SYM_, R_, RL_)                                                                          \
+  launch_had_v32<SD_, 3, SYM_, R_, RL_>(st, D.numSMs, nblk, npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn,  \
+                                              D.effDen32, blkDen, D.hvT32, D.effVal32, blkVal, P.nEff32, nrmfc)
+#define FMMG_HADV_RW(SD_, SYM_)                 \
+  switch (RW) {                                 \
+    case 1: FMMG_HADV(SD_, SYM_, 1, 1); break;  \
+    case 2: FMMG_HADV(SD_, SYM_, 2, 1); break;  \
+    case 4: FMMG_HADV(SD_, SYM_, 2, 2); break;  \
+    default: FMMG_HADV(SD_, SYM_, 2, 4); break; \
+  }
+    if (scalar && D.hadPQ) {
       if (!r8) {  // planes of one right-hand side
         const size_t smem = pqx_smem_bytes<32>();
         cudaFuncSetAttribute(k_m2l_had_pqx2<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1739,7 +1549,7 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
             npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen32, PqLayout{blkDen, (int64_t)P.nEff32 * 8}, D.m2lT32,
             D.effVal32, PqLayout{blkVal, (int64_t)P.nEff32 * 8}, 8, 1, P.nEff32, kc, nrmfc, D.transIdDev);
       }
-    } else if (P.sdm == 1 && P.tdm == 1) {
+    } else if (scalar) {
       if (!D.vListsReady) throw std::logic_error("the expanded V lists are not on the device (dev_upload_vlists)");
       const size_t smem = had_smem_bytes<float2>();
       cudaFuncSetAttribute(k_m2l_had_list<float2, KB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1748,19 +1558,25 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
       k_m2l_had_list<float2, KB, false><<<g2, HS_THREADS, smem, st>>>(
           ntrg, D.vTrgPtr, (const int2*)D.vTrgEnt, D.effDen32, effDR, D.m2lT32, D.effVal32, effVR, P.nEff32, kc,
           nrmfc);
-    } else if (P.sdm == 4 && P.tdm == 3) FMMG_HAD32(4, 3);
-    else FMMG_HAD32(3, 3);
-#undef FMMG_HAD32
+    } else if (P.sdm == 4 && P.tdm == 3) {
+      if (D.hvSymOf32) FMMG_HADV_RW(4, true) else FMMG_HADV_RW(4, false)
+    } else {
+      if (D.hvSymOf32) FMMG_HADV_RW(3, true) else FMMG_HADV_RW(3, false)
+    }
+#undef FMMG_HADV_RW
+#undef FMMG_HADV
     ls->launches++;
   }
   cudaEventRecord(D.ev[EV_M2L_HAD], st);
-  if ((mask & 4) && npar > 0 && ntrg > 0 && r8) {
+  if ((mask & 4) && npar > 0 && ntrg > 0) {
 #define FMMG_INV32R8(NP_)                                                                                      \
   do {                                                                                                         \
     constexpr size_t sm = r8_inv_smem<NP_>();                                                                  \
-    cudaFuncSetAttribute(k_m2l_inv32r8<NP_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);            \
-    k_m2l_inv32r8<NP_><<<dim3(ntrg, nblk), 256, sm, st>>>(D.vTrgNodes, D.effVal32, blkVal, P.nEff32, D.surfIJK,  \
-                                                          P.nDC, D.dchk32, nn * dc, kc);                       \
+    auto* ki = lgRW == 3 ? k_m2l_inv32r8<NP_, 3> : k_m2l_inv32r8<NP_, -1>;                                      \
+    cudaFuncSetAttribute(ki, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);                            \
+    ki<<<dim3((valPlanes + 7) / 8, nblk), 256, sm, st>>>(                                                      \
+        valPlanes, lgRW, D.vTrgNodes, D.effVal32, blkVal, P.nEff32, P.tdm, D.surfIJK, P.nDC, D.dchk32,         \
+        nn * dc, kc);                                                                                          \
   } while (0)
     switch (P.o.np) {
       case 3: FMMG_INV32R8(3); break;
@@ -1771,20 +1587,6 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
       case 8: FMMG_INV32R8(8); break;
     }
 #undef FMMG_INV32R8
-    ls->launches++;
-  } else if ((mask & 4) && npar > 0 && ntrg > 0) {
-#define FMMG_INV32(NP_)                                                                                   \
-  k_m2l_inv32<NP_><<<dim3(ntrg, kc), 128, 0, st>>>(D.vTrgNodes, D.effVal32, effVR, P.nEff32, P.tdm, D.surfIJK, \
-                                                    P.nDC, D.dchk32, nn * dc)
-    switch (P.o.np) {
-      case 3: FMMG_INV32(3); break;
-      case 4: FMMG_INV32(4); break;
-      case 5: FMMG_INV32(5); break;
-      case 6: FMMG_INV32(6); break;
-      case 7: FMMG_INV32(7); break;
-      case 8: FMMG_INV32(8); break;
-    }
-#undef FMMG_INV32
     ls->launches++;
   }
   cudaEventRecord(D.ev[EV_M2L_INV], st);

@@ -5,8 +5,8 @@
 //                     M2M + C2E as batched row GEMMs (k_gemm_rows)
 //   U-list  :773-785  k_p2p_near_w (true kernel, sources of adjacent leaves)
 //   V-list  :1015-1051 k_m2l_fwd (r2c of each upward density on the (2np)^3
-//                     grid), k_m2l_had (per-frequency products grouped by
-//                     parent pairs), k_m2l_inv (c2r + gather onto DC)
+//                     grid), k_m2l_had_pq / k_m2l_had_v64 (per-frequency
+//                     products grouped by parent pairs), k_m2l_inv (c2r + gather onto DC)
 //   W-list  :1139-1175 S2T entries folded into k_p2p_near_w, M2T in k_e2t
 //   X-list  :1241-1257 S2T entries folded into k_p2p_near_w, S2L in k_src2surf
 //   downward:1368-1438 per level L2L + C2E row GEMMs, L2T in k_e2t
@@ -33,12 +33,12 @@
 #include "gemm_rows.cuh"
 #include "had_pq.cuh"
 #include "had_smem.cuh"
+#include "had_vec.cuh"
 #include "kernels.hpp"
 
 namespace fmmg {
 
 
-__constant__ int16_t c_transId[343];  // (rx+3)*49+(ry+3)*7+(rz+3) -> 0..315 or -1
 
 // ------------------------------------------------------------------ helpers
 __global__ void k_gather_den(int64_t n, int sd, const int64_t* __restrict__ perm, const double* __restrict__ in,
@@ -422,72 +422,9 @@ __global__ void __launch_bounds__(128)
         s.x += t.x;
         s.y += t.y;
       }
-      out[(int64_t)e * sdm + m] = s;
+      out[(int64_t)m * nEff + e] = s;
     }
     __syncthreads();
-  }
-}
-
-// k_m2l_had: effVal(c) = (1/(2np)^3) sum_{v in V(c)} T_{idx(c,v)} .* effDen(v)
-// (cptwvv, matmgnt3d_mpi.cpp:414-429).  One CTA per (target parent P,
-// 32-frequency chunk); warp w owns child c = w of P.  The V-list of c is the
-// set of children v of P's same-depth non-leaf neighbours Q that do not touch
-// c; idx = v - c in child widths.
-template <int SDM, int TDM>
-__global__ void __launch_bounds__(256)
-    k_m2l_had(const int32_t* __restrict__ rowOut, const int64_t* __restrict__ vPtr, const int8_t* __restrict__ vOff,
-              const int32_t* __restrict__ nIn, const double2* __restrict__ effDen, const double2* __restrict__ T,
-              double2* __restrict__ effVal, int nEff, double nrmfc) {
-  // the parent's neighbour entries (input child slots resolved at setup,
-  // offset code), 32 at a time in shared memory for the CTA
-  __shared__ int sSl[32 * 8];
-  __shared__ int sOf[32];
-  const int b = blockIdx.x;
-  const int c = threadIdx.x >> 5;
-  const int f = blockIdx.y * 32 + (threadIdx.x & 31);
-  const int ts = rowOut[8 * b + c];
-  const int cx = c >> 2, cy = (c >> 1) & 1, cz = c & 1;
-  double2 acc[TDM];
-#pragma unroll
-  for (int i = 0; i < TDM; i++) acc[i] = make_double2(0, 0);
-  const bool live = ts >= 0 && f < nEff;  // every thread stays for the CTA's barriers
-  const int64_t e1 = vPtr[b + 1];
-  for (int64_t e0 = vPtr[b]; e0 < e1; e0 += 32) {
-    const int ne = (int)min((int64_t)32, e1 - e0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < ne * 8; i += blockDim.x) sSl[i] = nIn[8 * e0 + i];
-    if (threadIdx.x < ne) sOf[threadIdx.x] = vOff[e0 + threadIdx.x];
-    __syncthreads();
-    if (!live) continue;
-    for (int j = 0; j < ne; j++) {
-      const int off = sOf[j];
-      const int dx = off / 9 - 1, dy = (off / 3) % 3 - 1, dz = off % 3 - 1;
-#pragma unroll 1
-      for (int c2 = 0; c2 < 8; c2++) {
-        const int s = sSl[j * 8 + c2];
-        if (s < 0) continue;
-        const int rx = 2 * dx + (c2 >> 2) - cx, ry = 2 * dy + ((c2 >> 1) & 1) - cy, rz = 2 * dz + (c2 & 1) - cz;
-        if (max(abs(rx), max(abs(ry), abs(rz))) <= 1) continue;
-        const int id = c_transId[(rx + 3) * 49 + (ry + 3) * 7 + (rz + 3)];
-        double2 d[SDM];
-#pragma unroll
-        for (int jj = 0; jj < SDM; jj++) d[jj] = effDen[((int64_t)s * nEff + f) * SDM + jj];
-        const double2* Tf = T + ((int64_t)id * nEff + f) * (SDM * TDM);
-#pragma unroll
-        for (int jj = 0; jj < SDM; jj++)
-#pragma unroll
-          for (int i = 0; i < TDM; i++) {
-            double2 tv = Tf[jj * TDM + i];
-            acc[i].x += tv.x * d[jj].x - tv.y * d[jj].y;
-            acc[i].y += tv.x * d[jj].y + tv.y * d[jj].x;
-          }
-      }
-    }
-  }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < TDM; i++)
-      effVal[((int64_t)ts * nEff + f) * TDM + i] = make_double2(acc[i].x * nrmfc, acc[i].y * nrmfc);
   }
 }
 
@@ -521,7 +458,7 @@ __global__ void __launch_bounds__(128)
       double2 s = make_double2(0, 0);
 #pragma unroll 4
       for (int kz = 0; kz < N; kz++) {
-        double2 t = cmulc(in[((int64_t)(kz * N + ky) * NH + kx) * tdm + m], tw[(kz * (zb + H)) % N]);
+        double2 t = cmulc(in[(int64_t)m * nEff + (int64_t)(kz * N + ky) * NH + kx], tw[(kz * (zb + H)) % N]);
         s.x += t.x;
         s.y += t.y;
       }
@@ -658,6 +595,8 @@ static void dev_clear(DevState& D) {
   for (DevState::OpT* op : {&D.tL2L, &D.tUpF1, &D.tUpF2, &D.tDnF1, &D.tDnF2, &D.tM2MUp}) *op = DevState::OpT();
   for (TcOp* op : {&D.cL2L, &D.cUpF1, &D.cUpF2, &D.cDnF1, &D.cDnF2, &D.cM2MUp}) *op = TcOp();  // memory freed above
   D.transIdDev = nullptr;
+  D.hvT = nullptr;
+  D.hvT32 = nullptr;
   D.m2lT32 = nullptr;
   D.m2lTw32 = nullptr;
   D.denK = D.valK = nullptr;
@@ -689,6 +628,32 @@ static void dev_clear(DevState& D) {
   D.m2tPart = nullptr;
 }
 
+// the vector kernels' translations for k_m2l_had_v64, symmetric blocks where
+// the tables are (to 64 rounding errors of a translation's largest value)
+template <int SDM, int TDM>
+static std::string hv_layout(const Plan& P, DevState& D) {
+  int* dFlag = nullptr;
+  int flag = 0;
+  PlanBufs tmp;
+  tmp.device = D.device;
+  FMMG_CK(tmp.get(dFlag, 1));
+  FMMG_CK(cudaMemset(dFlag, 0, sizeof(int)));
+  k_hv_asym<double2, SDM, TDM><<<316, 256>>>(D.m2lT, P.nEff, 64 * 2.2e-16, dFlag);
+  FMMG_CK(cudaMemcpy(&flag, dFlag, sizeof(int), cudaMemcpyDeviceToHost));
+  D.hvSym = flag == 0;
+  if (!D.hvT || D.hvSymOf64 != D.hvSym) {
+    const int64_t n = D.hvSym ? hv_table_size<double2, SDM, TDM, true>(P.nEff)
+                              : hv_table_size<double2, SDM, TDM, false>(P.nEff);
+    FMMG_TRY(dput<double2>(D, D.hvT, nullptr, (size_t)n));
+  }
+  D.hvSymOf64 = D.hvSym;
+  if (D.hvSym) launch_hv_pack<double2, SDM, TDM, true>(0, D.m2lT, D.transIdDev, P.nEff, D.hvT);
+  else launch_hv_pack<double2, SDM, TDM, false>(0, D.m2lT, D.transIdDev, P.nEff, D.hvT);
+  FMMG_CK(cudaGetLastError());
+  FMMG_CK(cudaDeviceSynchronize());
+  return std::string();
+}
+
 std::string dev_upload_operators(const Plan& P, DevState& D) {
   FMMG_CK(cudaSetDevice(D.device));
   auto put = [&](double*& dst, const std::vector<double>& v) -> std::string {
@@ -707,8 +672,9 @@ std::string dev_upload_operators(const Plan& P, DevState& D) {
   }
   int16_t tid[343];
   for (int i = 0; i < 343; i++) tid[i] = (int16_t)P.transId[i / 49][(i / 7) % 7][i % 7];
-  FMMG_CK(cudaMemcpyToSymbol(c_transId, tid, sizeof(tid)));
   if (!D.transIdDev) FMMG_TRY(dput(D, D.transIdDev, tid, 343));
+  if (P.sdm == 4) FMMG_TRY((hv_layout<4, 3>(P, D)));
+  else if (P.sdm == 3) FMMG_TRY((hv_layout<3, 3>(P, D)));
   D.mixedOpsStale = true;
   D.adjOpsStale = true;
   return std::string();
@@ -978,7 +944,6 @@ static void launch_m2l_np(const Plan& P, DevState& D, LaunchStats* ls) {
   }
   cudaEventRecord(D.ev[EV_M2L_FWD], D.stream);
   if (npar > 0 && ntrg > 0) {
-    dim3 grid(npar, (P.nEff + 31) / 32);
     const double nrmfc = 1.0 / double(P.nReg);
     if (P.sdm == 1 && P.tdm == 1 && D.hadPQ) {
       const size_t smem = pq_smem_bytes<double2>(32);
@@ -996,12 +961,17 @@ static void launch_m2l_np(const Plan& P, DevState& D, LaunchStats* ls) {
       k_m2l_had_list<double2, 1, false><<<g2, HS_THREADS, smem, D.stream>>>(
           ntrg, D.vTrgPtr, (const int2*)D.vTrgEnt, D.effDen, 0, D.m2lT, D.effVal, 0, P.nEff, 1, nrmfc);
     }
-    else if (P.sdm == 4 && P.tdm == 3)
-      k_m2l_had<4, 3><<<grid, 256, 0, D.stream>>>(D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen, D.m2lT, D.effVal,
-                                                  P.nEff, nrmfc);
-    else
-      k_m2l_had<3, 3><<<grid, 256, 0, D.stream>>>(D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen, D.m2lT, D.effVal,
-                                                  P.nEff, nrmfc);
+    else {
+#define FMMG_HADV64(SD_, SYM_)                                                                                  \
+  launch_had_v64<SD_, 3, SYM_>(D.stream, D.numSMs, npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen, D.hvT,   \
+                               D.effVal, P.nEff, nrmfc)
+      if (P.sdm == 4) {
+        if (D.hvSymOf64) FMMG_HADV64(4, true); else FMMG_HADV64(4, false);
+      } else {
+        if (D.hvSymOf64) FMMG_HADV64(3, true); else FMMG_HADV64(3, false);
+      }
+#undef FMMG_HADV64
+    }
     cudaEventRecord(D.ev[EV_M2L_HAD], D.stream);
     Scale4 none;
     none.mod = 0;
