@@ -649,8 +649,9 @@ static void run_adjoint(const Plan& P, DevState& D, int& launches) {
                                                                       D.nrm, D.trg, w, g, mu, ve);
     launches++;
   }
-  // upward, transposed: C2E^T then M2M^T per level, root side first
-  for (int d = 1; d <= P.maxDepth; d++) {
+  // upward, transposed: C2E^T then M2M^T per level, root side first (nothing
+  // reaches the densities of depth 1, see run_stages)
+  for (int d = 2; d <= P.maxDepth; d++) {
     const int32_t* rows;
     int n = rows_at(D.offUpC2E, d, rows);
     if (n > 0) {

@@ -190,7 +190,7 @@ std::string dev_evaluate_mixed(const Plan& P, DevState& D, const double* dDenCal
 struct Scale4;
 void gemm_rows(DevState& D, int nrows, const int32_t* rows, const int32_t* chd, int xChild, int yChild,
                const double* X, int64_t ldx, const double* W, double* Y, int64_t ldy, int K, int N, Scale4 xs,
-               Scale4 ys, double beta, LaunchStats* ls);
+               Scale4 ys, double beta, LaunchStats* ls, const int32_t* rowDepth = nullptr, int rootLevel = 0);
 void spectral_fwd(const Plan& P, DevState& D, int n, const int32_t* nodes, Scale4 deg, int dof, const double* x,
                   double2* spec);
 void spectral_inv(const Plan& P, DevState& D, int n, const int32_t* nodes, int dof, const double2* spec, double* y,

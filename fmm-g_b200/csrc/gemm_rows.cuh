@@ -1,4 +1,5 @@
-// gemm_rows.cuh -- batched row GEMM of the translation stages, FP64 and FP32.
+// gemm_rows.cuh -- batched row GEMM of the translation stages on the CUDA cores,
+// FP32 (gemm_f64.cuh is the FP64 form, gemm_tc.cuh the tensor-core FP32 one).
 //
 // For every listed node (and every right-hand side),
 //   Y[row] = beta * Y[row] + ys .* (W (xs .* X[row])),
@@ -9,7 +10,7 @@
 // their transposes in the adjoint.
 //
 // Tiling: 128 (rows x right-hand sides) x 64 (outputs) per CTA, K in steps of
-// BK (16 for FP32, 8 for FP64: four 16-byte vectors per tile row), 256
+// BK = 16 (four 16-byte vectors per tile row), 256
 // threads each owning an 8 x 4 register tile.  The next K step is
 // fetched into registers while the current one is multiplied from shared
 // memory (two buffers, one barrier per step).

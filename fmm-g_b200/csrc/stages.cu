@@ -2,7 +2,7 @@
 //
 // Stage map (reference fmm3d_mpi/fmm3d_eval_mpi.cpp):
 //   upward  :557-595  S2M (k_src2surf on each leaf's UC surface), then per level
-//                     M2M + C2E as batched row GEMMs (k_gemm_rows)
+//                     M2M + C2E as batched row GEMMs (k_gemm_f64)
 //   U-list  :773-785  k_p2p_near_w (true kernel, sources of adjacent leaves)
 //   V-list  :1015-1051 k_m2l_fwd (r2c of each upward density on the (2np)^3
 //                     grid), k_m2l_had_pq / k_m2l_had_v64 (per-frequency
@@ -30,6 +30,7 @@
 #include "engine.hpp"
 #include "plan_pool.cuh"
 #include "dense_kernel.cuh"
+#include "gemm_f64.cuh"
 #include "gemm_rows.cuh"
 #include "had_pq.cuh"
 #include "had_smem.cuh"
@@ -871,9 +872,11 @@ std::string dev_upload(const Plan& P, DevState& D, const double* src, const doub
 }
 
 // ------------------------------------------------------------------ launcher
+// rowDepth: the rows are of several levels, and ys holds the degrees: their Y
+// scale is 2^(-(level) degree) by each row's depth (k_gemm_f64)
 void gemm_rows(DevState& D, int nrows, const int32_t* rows, const int32_t* chd, int xChild, int yChild,
                const double* X, int64_t ldx, const double* W, double* Y, int64_t ldy, int K, int N, Scale4 xs,
-               Scale4 ys, double beta, LaunchStats* ls) {
+               Scale4 ys, double beta, LaunchStats* ls, const int32_t* rowDepth, int rootLevel) {
   if (nrows <= 0) return;
   GrScale<double> gx, gy;
   gx.mod = xs.mod;
@@ -882,11 +885,11 @@ void gemm_rows(DevState& D, int nrows, const int32_t* rows, const int32_t* chd, 
     gx.v[k] = xs.v[k];
     gy.v[k] = ys.v[k];
   }
-  // FP64 keeps each output's K sum in sequential order (no split-K scratch):
-  // the 1e-10 parity with the oracle's sequential sums depends on it at np = 7
-  const int n = launch_gemm_rows<double, 8>(D.stream, D.numSMs, nullptr, 0, nrows, 1, rows, chd, xChild, yChild, X,
-                                            ldx, 0, W, Y, ldy, 0, K, N, gx, gy, beta);
-  if (ls) ls->launches += n;
+  // row lengths are even (a surface has 6 m^2 + 2 points) and arrays come from
+  // cudaMalloc, so 16-byte pieces of a row are aligned
+  launch_gemm_f64(D.stream, D.numSMs, nrows, rows, chd, xChild, yChild, X, ldx, W, Y, ldy, K, N, gx, gy, beta,
+                  rowDepth, rootLevel);
+  if (ls) ls->launches++;
 }
 
 template <int KT>
@@ -1078,12 +1081,19 @@ static void run_stages(const Plan& P, DevState& D, int mask, LaunchStats* ls, bo
   if (mask & 1)  // upward: S2M
     launch_s2surf<KT>(P, D, (int)P.s2mLeaves.size(), D.s2mLeaves, nullptr, nullptr, D.sam[1], P.nUC, D.uchk, uc, ls);
   cudaEventRecord(D.ev[EV_S2M], st);
-  if (mask & 1) {  // upward: M2M + C2E per level
-    for (int d = P.maxDepth; d >= 1; d--) {
-      int64_t a = D.offUpM2M[d], b = D.offUpM2M[d + 1];
+  if (mask & 1) {  // upward: C2E of all leaves at once, then M2M + C2E of the parents per level
+    // down to depth 2: nothing reads the densities of depth 1, whose boxes all
+    // touch (no V list there) and whose leaves' W nodes lie deeper
+    Scale4 deg;
+    deg.mod = P.sdm;
+    for (int k = 0; k < 4; k++) deg.v[k] = k < P.sdm ? P.deg[k] : 0.0;
+    const int64_t l0 = D.offUpLeaf[std::min(2, P.maxDepth + 1)], l1 = D.offUpLeaf[P.maxDepth + 1];
+    gemm_rows(D, (int)(l1 - l0), D.levelRows + l0, D.chd, 0, 0, D.uchk, uc, D.uc2ue, D.uden, ue, uc, ue, unit_scale(),
+              deg, 0.0, ls, D.depth, rl);
+    for (int d = P.maxDepth - 1; d >= 2; d--) {
+      const int64_t a = D.offUpM2M[d], b = D.offUpM2M[d + 1];
       gemm_rows(D, (int)(b - a), D.levelRows + a, D.chd, 1, 0, D.uden, ue, D.m2m, D.uchk, uc, 8 * ue, uc,
                 level_scale(P, d + 1 + rl, +1.0), unit_scale(), 0.0, ls);
-      a = D.offUpC2E[d]; b = D.offUpC2E[d + 1];
       gemm_rows(D, (int)(b - a), D.levelRows + a, D.chd, 0, 0, D.uchk, uc, D.uc2ue, D.uden, ue, uc, ue, unit_scale(),
                 level_scale(P, d + rl, -1.0), 0.0, ls);
     }
