@@ -44,6 +44,7 @@ struct DevState {
   int32_t* surfIJK = nullptr;  // np-surface point -> packed (i, j, k)
   // work lists
   int32_t *evtrLeaves = nullptr;
+  int64_t maxLeafTrg = 0;  // targets of the fullest evaluator leaf
   int64_t *nearPtr = nullptr; int32_t *nearIdx = nullptr;     // merged near list
   int64_t *nearUPtr = nullptr; int32_t *nearUIdx = nullptr;   // stage-split forms
   int64_t *nearWPtr = nullptr; int32_t *nearWIdx = nullptr;
@@ -159,6 +160,15 @@ struct DevState {
   };
   std::vector<Block> spare;
 };
+
+// FP32 near field: the leaves above which a warp a leaf fills the GPU (48 warps an
+// SM); and the blocks of tb targets that the fullest leaf takes (grid.y; a
+// leaf of more than 64 blocks loops)
+inline int near_warps(int numSMs) { return 48 * numSMs; }
+inline unsigned near_blocks(const DevState& D, int tb) {
+  const int64_t b = (D.maxLeafTrg + tb - 1) / tb;
+  return (unsigned)(b < 1 ? 1 : (b > 64 ? 64 : b));
+}
 
 // counts of the last stage launch list (for reporting)
 struct LaunchStats {

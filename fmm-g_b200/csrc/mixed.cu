@@ -33,16 +33,8 @@
 
 namespace fmmg {
 
-constexpr int MX_THREADS = 128;
 constexpr int MX_THREADS_FAR = 192;  // M2T: 2^6 x 3 also allows target groups of 24, 48, 96
 constexpr int MX_TILE = 128;
-// staged sources (or surface points) per round: 256 when a source carries at
-// most 8 density values and no normal (the static shared memory stays under
-// 48 KB), else 128
-template <int DEN, bool NRM>
-constexpr int mx_tile() {
-  return (DEN <= 8 && !NRM) ? 256 : 128;
-}
 constexpr int MX_MAXE = 256;
 
 // fill eBeg/ePre for entries [ec, ec+ne) and return the total source count
@@ -136,122 +128,205 @@ __device__ __forceinline__ void mx_den(const float* __restrict__ s, float (&d)[N
   }
 }
 
-// near field: U-list, direct W and X entries; grid (evaluator leaves, RHS blocks).
+// near field: U-list, direct W and X entries; grid (evaluator leaves, blocks of
+// tb targets, RHS blocks).  The warps and lanes are arranged as in
+// k_p2p_near_w (stages.cu): NR = 2 targets a lane, TG = ceil(targets / 2) lanes a
+// group, S = 32 / TG groups that split the sources, WS = 1 or 4 warps a leaf;
+// leaves in order[] (decreasing targets x near sources).
 // The offsets are formed from hi/lo FP32 pairs of the box-centred
 // coordinates, (x_hi - y_hi) + (x_lo - y_lo): the hi difference of close
 // points is exact, so near-coincident pairs keep their separation.  For the
 // double-layer kernels (source normal, NRM) n.(x - y) is formed in FP64 from
-// those pairs and the normal's hi/lo pair: on densely sampled surfaces
+// the FP64 box-centred coordinates and normals: on densely sampled surfaces
 // near-coincident pairs dominate the sum and n.(x - y) cancels to curvature
 // size, O(r^2), while any FP32 rounding of the offset or the normal leaves an
 // O(eps r) error in it (relative error eps / (kappa r), 1e-3 at r = 1e-6).
-template <int KT, int KB>
-__global__ void __launch_bounds__(MX_THREADS)
-    k_p2p_near32(const int32_t* __restrict__ rows, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+// A CTA a leaf with CTA-wide barriers left the longest leaf's CTA running
+// alone, and as the lower-priority stream's work it held the SMs that the
+// chain of row GEMMs beside it was waiting for: Laplace double layer, 50,021
+// sources and 30,011 targets apart, k = 3: 1.06 -> 0.30 ms.
+constexpr int NX_WARPS = 4, NX_CH = 32, NX_MAXE = 128, NX_R = 2;
+template <int KT, int KB, int WS>
+__global__ void __launch_bounds__(32 * NX_WARPS)
+    k_p2p_near32(int nLeaves, int tb, const int32_t* __restrict__ order, const int32_t* __restrict__ rows,
+                 const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                  const int64_t* __restrict__ srcBeg, const int64_t* __restrict__ srcCnt,
                  const int64_t* __restrict__ trgBeg, const int64_t* __restrict__ trgCnt,
                  const double* __restrict__ src, const double* __restrict__ nrm, const float* __restrict__ den32,
                  int64_t den32Blk, const double* __restrict__ trg, const double* __restrict__ ctr,
                  double* __restrict__ val, int64_t valStride, int nrhs, float mu, float ve) {
-  constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD, NRM = KTraits<KT>::NRM;
-  constexpr int MX_TILE = mx_tile<SD * KB, NRM != 0>();
-  __shared__ float4 sPos[MX_TILE];
-  __shared__ float4 sPosLo[MX_TILE];
-  __shared__ float4 sNrm[NRM ? MX_TILE : 1];
-  __shared__ double sPosD[NRM ? 3 * MX_TILE : 1];  // FP64 box-centred source positions and normals (NRM)
-  __shared__ double sNrmD[NRM ? 3 * MX_TILE : 1];
-  __shared__ __align__(16) float sDen[MX_TILE * SD * KB];
-  __shared__ int64_t eBeg[MX_MAXE];
-  __shared__ int32_t ePre[MX_MAXE + 1];
-  __shared__ double sRed[MX_THREADS * TD * KB];
-  const int row = blockIdx.x;
-  const int rhs0 = blockIdx.y * KB;
+  constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD, NRM = KTraits<KT>::NRM, NA = TD * KB;
+  __shared__ float4 sPos[NX_WARPS][NX_CH];
+  __shared__ float4 sPosLo[NX_WARPS][NX_CH];
+  __shared__ float4 sNrm[NX_WARPS][NRM ? NX_CH : 1];
+  __shared__ double sPosD[NX_WARPS][NRM ? 3 * NX_CH : 1];  // FP64 box-centred source positions and normals (NRM)
+  __shared__ double sNrmD[NX_WARPS][NRM ? 3 * NX_CH : 1];
+  __shared__ __align__(16) float sDen[NX_WARPS][NX_CH * SD * KB];
+  __shared__ int64_t eBeg[NX_WARPS][NX_MAXE];
+  __shared__ int32_t ePre[NX_WARPS][NX_MAXE + 1];
+  __shared__ double sRed[WS > 1 ? 32 * NX_R * NA : 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int li = blockIdx.x * (NX_WARPS / WS) + warp / WS, sub = warp % WS;
+  if (li >= nLeaves) return;  // WS == 1 only: no CTA-wide barrier below then
+  const int row = order[li];
+  const int rhs0 = blockIdx.z * KB;
   const int g = rows[row];
-  const int64_t tb = trgBeg[g], tn = trgCnt[g];
+  const int64_t tBeg = trgBeg[g], tn = trgCnt[g];
   const int64_t e0 = ptr[row], e1 = ptr[row + 1];
   const double cx = ctr[3 * g], cy = ctr[3 * g + 1], cz = ctr[3 * g + 2];
-  const int tid = threadIdx.x;
-  const int TG = mx_group<MX_THREADS>(tn);
-  const int S = MX_THREADS / TG;
-  const int tl = tid % TG, sp = tid / TG;
-  for (int64_t t0 = 0; t0 < tn; t0 += TG) {
-    const int64_t t = t0 + tl;
-    const bool act = t < tn;
-    float tx = 0, ty = 0, tz = 0, txl = 0, tyl = 0, tzl = 0;
-    double tdx = 0, tdy = 0, tdz = 0;  // FP64 box-centred target (NRM)
-    if (act) {
-      const double dx = trg[3 * (tb + t)] - cx, dy = trg[3 * (tb + t) + 1] - cy, dz = trg[3 * (tb + t) + 2] - cz;
-      tdx = dx;
-      tdy = dy;
-      tdz = dz;
-      tx = (float)dx;
-      ty = (float)dy;
-      tz = (float)dz;
-      txl = (float)(dx - tx);
-      tyl = (float)(dy - ty);
-      tzl = (float)(dz - tz);
-    }
-    double acc[TD * KB];
+  for (int64_t t0 = (int64_t)blockIdx.y * tb; t0 < tn; t0 += (int64_t)gridDim.y * tb) {
+    const int nt = (int)min((int64_t)tb, tn - t0);  // at most 64
+    const int TG = (nt + NX_R - 1) / NX_R, S = 32 / TG;
+    const int tl = lane % TG, sp = lane / TG;
+    float th[NX_R][3], tlo[NX_R][3];
+    double td[NX_R][NRM ? 3 : 1];  // FP64 box-centred targets (NRM)
+    double acc[NX_R][NA];
 #pragma unroll
-    for (int c = 0; c < TD * KB; c++) acc[c] = 0.0;
-    for (int64_t ec = e0; ec < e1; ec += MX_MAXE) {
-      const int ne = (int)min((int64_t)MX_MAXE, e1 - ec);
-      const int total = load_entries(idx, ec, ne, 0, srcBeg, srcCnt, eBeg, ePre);
-      for (int base = 0; base < total; base += MX_TILE) {
-        const int cnt = min(MX_TILE, total - base);
-        __syncthreads();
-        for (int i = tid; i < cnt; i += MX_THREADS) {
-          const int64_t s = entry_source(base + i, ne, eBeg, ePre);
+    for (int r = 0; r < NX_R; r++) {
+      const int64_t t = tBeg + t0 + min(tl + r * TG, nt - 1);  // past the last: repeated, not stored
+      const double d[3] = {trg[3 * t] - cx, trg[3 * t + 1] - cy, trg[3 * t + 2] - cz};
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        th[r][c] = (float)d[c];
+        tlo[r][c] = (float)(d[c] - th[r][c]);
+        if (NRM) td[r][c] = d[c];
+      }
+#pragma unroll
+      for (int c = 0; c < NA; c++) acc[r][c] = 0.0;
+    }
+    for (int64_t ec = e0; ec < e1; ec += NX_MAXE) {
+      const int ne = (int)min((int64_t)NX_MAXE, e1 - ec);
+      __syncwarp();
+      int running = 0;  // the warp's entry table: starts and prefix counts
+      for (int eb = 0; eb < ne; eb += 32) {
+        const int e = eb + lane;
+        int c = 0;
+        if (e < ne) {
+          const int s2 = idx[ec + e];
+          eBeg[warp][e] = srcBeg[s2];
+          c = (int)srcCnt[s2];
+        }
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += v;
+        }
+        if (e < ne) ePre[warp][e + 1] = running + incl;
+        running += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane == 0) ePre[warp][0] = 0;
+      __syncwarp();
+      const int total = running;
+      // FP32 partial sums over up to 128 sources of the warp, then FP64
+      float part[NX_R][NA];
+      for (int base = sub * NX_CH, round = 0; base < total; base += WS * NX_CH, round++) {
+        const int cnt = min(NX_CH, total - base);
+        __syncwarp();
+        if (lane < cnt) {
+          const int i = lane;
+          const int64_t s = entry_source(base + i, ne, eBeg[warp], ePre[warp]);
           const double dx = src[3 * s] - cx, dy = src[3 * s + 1] - cy, dz = src[3 * s + 2] - cz;
-          sPos[i] = make_float4((float)dx, (float)dy, (float)dz, 0.f);
-          sPosLo[i] = make_float4((float)(dx - (float)dx), (float)(dy - (float)dy), (float)(dz - (float)dz), 0.f);
+          sPos[warp][i] = make_float4((float)dx, (float)dy, (float)dz, 0.f);
+          sPosLo[warp][i] = make_float4((float)(dx - (float)dx), (float)(dy - (float)dy), (float)(dz - (float)dz), 0.f);
           if (NRM) {
             const double nx = nrm[3 * s], ny = nrm[3 * s + 1], nz = nrm[3 * s + 2];
-            sNrm[i] = make_float4((float)nx, (float)ny, (float)nz, 0.f);
-            sPosD[3 * i] = dx;
-            sPosD[3 * i + 1] = dy;
-            sPosD[3 * i + 2] = dz;
-            sNrmD[3 * i] = nx;
-            sNrmD[3 * i + 1] = ny;
-            sNrmD[3 * i + 2] = nz;
+            sNrm[warp][i] = make_float4((float)nx, (float)ny, (float)nz, 0.f);
+            sPosD[warp][3 * i] = dx;
+            sPosD[warp][3 * i + 1] = dy;
+            sPosD[warp][3 * i + 2] = dz;
+            sNrmD[warp][3 * i] = nx;
+            sNrmD[warp][3 * i + 1] = ny;
+            sNrmD[warp][3 * i + 2] = nz;
           }
           // the block's KB x SD densities: contiguous in the FP32 copy (rows of
           // 8 right-hand sides per source, zeros past the last one)
           const float* ds = den32 + (rhs0 >> 3) * den32Blk + s * 8 * SD + (rhs0 & 7) * SD;
 #pragma unroll
-          for (int r = 0; r < KB * SD; r++) sDen[i * KB * SD + r] = ds[r];
+          for (int r = 0; r < KB * SD; r++) sDen[warp][i * KB * SD + r] = ds[r];
         }
-        __syncthreads();
-        if (act) {
-          float part[TD * KB];
+        __syncwarp();
+        if ((round & 3) == 0) {
 #pragma unroll
-          for (int c = 0; c < TD * KB; c++) part[c] = 0.f;
+          for (int r = 0; r < NX_R; r++)
+#pragma unroll
+            for (int c = 0; c < NA; c++) part[r][c] = 0.f;
+        }
+        if (sp < S) {
           for (int i = sp; i < cnt; i += S) {
-            // offsets from hi/lo FP32 pairs of the box-centred coordinates:
-            // the hi difference of close points is exact, so a near-coincident
-            // pair keeps its separation to FP32 precision of the separation
-            const float4 q = sPos[i], ql = sPosLo[i];
-            const float ox = (tx - q.x) + (txl - ql.x), oy = (ty - q.y) + (tyl - ql.y), oz = (tz - q.z) + (tzl - ql.z);
+            const float4 q = sPos[warp][i], ql = sPosLo[warp][i];
             float nv[3] = {0.f, 0.f, 0.f};
-            float rn = 0.f;
             if (NRM) {
-              const float4 qn = sNrm[i];
+              const float4 qn = sNrm[warp][i];
               nv[0] = qn.x;
               nv[1] = qn.y;
               nv[2] = qn.z;
-              rn = (float)((tdx - sPosD[3 * i]) * sNrmD[3 * i] + (tdy - sPosD[3 * i + 1]) * sNrmD[3 * i + 1] +
-                           (tdz - sPosD[3 * i + 2]) * sNrmD[3 * i + 2]);
             }
             float d[KB * SD];
-            mx_den<KB * SD>(&sDen[i * KB * SD], d);
-            kaccum_multi<KT, KB, float, float>(ox, oy, oz, NRM ? nv : nullptr, d, part, mu, ve, NRM ? &rn : nullptr);
-          }
+            mx_den<KB * SD>(&sDen[warp][i * KB * SD], d);
 #pragma unroll
-          for (int c = 0; c < TD * KB; c++) acc[c] += (double)part[c];
+            for (int r = 0; r < NX_R; r++) {
+              const float ox = (th[r][0] - q.x) + (tlo[r][0] - ql.x), oy = (th[r][1] - q.y) + (tlo[r][1] - ql.y),
+                          oz = (th[r][2] - q.z) + (tlo[r][2] - ql.z);
+              float rn = 0.f;
+              if constexpr (NRM != 0)
+                rn = (float)((td[r][0] - sPosD[warp][3 * i]) * sNrmD[warp][3 * i] +
+                             (td[r][1] - sPosD[warp][3 * i + 1]) * sNrmD[warp][3 * i + 1] +
+                             (td[r][2] - sPosD[warp][3 * i + 2]) * sNrmD[warp][3 * i + 2]);
+              kaccum_multi<KT, KB, float, float>(ox, oy, oz, NRM ? nv : nullptr, d, part[r], mu, ve, NRM ? &rn : nullptr);
+            }
+          }
+        }
+        if ((round & 3) == 3 || base + WS * NX_CH >= total) {
+#pragma unroll
+          for (int r = 0; r < NX_R; r++)
+#pragma unroll
+            for (int c = 0; c < NA; c++) acc[r][c] += (double)part[r][c];
         }
       }
     }
-    reduce_store<TD, KB>(sRed, acc, tid, tl, sp, TG, S, act, val, tb + t, rhs0, nrhs, valStride);
+#pragma unroll
+    for (int r = 0; r < NX_R; r++)
+#pragma unroll
+      for (int c = 0; c < NA; c++) {
+        const double own = acc[r][c];
+        for (int k = 1; k < S; k++) acc[r][c] += __shfl_sync(0xffffffffu, own, (lane + k * TG) & 31);
+      }
+    auto store = [&]() {
+#pragma unroll
+      for (int r = 0; r < NX_R; r++) {
+        if (tl + r * TG >= nt) continue;
+#pragma unroll
+        for (int q = 0; q < KB; q++) {
+          if (rhs0 + q >= nrhs) break;
+#pragma unroll
+          for (int c = 0; c < TD; c++)
+            val[(int64_t)(rhs0 + q) * valStride + (tBeg + t0 + tl + r * TG) * TD + c] += acc[r][q * TD + c];
+        }
+      }
+    };
+    if constexpr (WS == 1) {
+      if (sp == 0) store();
+    } else {
+      // the warps' sums meet in the first one, in warp order
+      for (int w = 1; w < WS; w++) {
+        __syncthreads();
+        if (sub == w && sp == 0) {
+#pragma unroll
+          for (int r = 0; r < NX_R; r++)
+#pragma unroll
+            for (int c = 0; c < NA; c++) sRed[(tl * NX_R + r) * NA + c] = acc[r][c];
+        }
+        __syncthreads();
+        if (sub == 0 && sp == 0) {
+#pragma unroll
+          for (int r = 0; r < NX_R; r++)
+#pragma unroll
+            for (int c = 0; c < NA; c++) acc[r][c] += sRed[(tl * NX_R + r) * NA + c];
+        }
+      }
+      if (sub == 0 && sp == 0) store();
+    }
   }
 }
 
@@ -295,17 +370,21 @@ __device__ __forceinline__ unsigned long long nl_fma(unsigned long long a, unsig
 // shared memory; its lanes take two targets each and split each chunk's
 // sources in 32 / TG strides.  The offsets, r^2 and 1/(4 pi r) of a source
 // against both targets and the KB multiply-adds of its densities run as
-// packed FP32x2 operations (half the instructions of a one-target loop), with
-// the offsets from hi/lo pairs and the coincidence rule (r^2 < 1e-16 adds
+// packed FP32x2 operations (half the instructions of a one-target loop).  As in
+// k_p2p_near_w (stages.cu) TG = ceil(targets / 2) need not be a power of two
+// (17 targets take 27 lanes, 16 or 32 lanes a group left them half idle), and
+// with fewer leaves than the GPU holds warps (48 an SM) the CTA's WS = 4 warps
+// share one: 100,000 points 0.35 -> 0.16 ms.  With 62,000 leaves that takes 2.10
+// ms and a warp a leaf 1.53 (1.64 with 8, 16 or 32 lanes a group).  With the offsets from hi/lo pairs and the coincidence rule (r^2 < 1e-16 adds
 // nothing) of k_p2p_near32; per-chunk FP32 partial sums go into FP64
 // accumulators, which meet through warp shuffles at the end.  The leaves come
 // in order[] (rows by decreasing targets x near sources), so the four warps of
 // a CTA carry similar work and the longest leaves start first.  Six CTAs an SM
 // (80 registers) measured faster than four without spills (1.73 vs 2.00 ms).
 constexpr int NW_WARPS = 4, NW_CH = 64, NW_MAXE = 128;
-template <int KB>
+template <int KB, int WS>
 __global__ void __launch_bounds__(32 * NW_WARPS, 6)
-    k_p2p_near32_lap2w(int nLeaves, const int32_t* __restrict__ order, const int32_t* __restrict__ rows,
+    k_p2p_near32_lap2w(int nLeaves, int tb, const int32_t* __restrict__ order, const int32_t* __restrict__ rows,
                        const int64_t* __restrict__ ptr,
                        const int32_t* __restrict__ idx, const int64_t* __restrict__ srcBeg,
                        const int64_t* __restrict__ srcCnt, const int64_t* __restrict__ trgBeg,
@@ -317,28 +396,30 @@ __global__ void __launch_bounds__(32 * NW_WARPS, 6)
   __shared__ __align__(16) float sDen[NW_WARPS][NW_CH * KB];
   __shared__ int64_t eBeg[NW_WARPS][NW_MAXE];
   __shared__ int32_t ePre[NW_WARPS][NW_MAXE + 1];
+  __shared__ double sRed[WS > 1 ? 32 * 2 * KB : 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (blockIdx.x * NW_WARPS + warp >= nLeaves) return;
-  const int row = order[blockIdx.x * NW_WARPS + warp];
-  const int rhs0 = blockIdx.y * KB;
+  const int li = blockIdx.x * (NW_WARPS / WS) + warp / WS, sub = warp % WS;
+  if (li >= nLeaves) return;  // WS == 1 only: no CTA-wide barrier below then
+  const int row = order[li];
+  const int rhs0 = blockIdx.z * KB;
   const int g = rows[row];
-  const int64_t tb = trgBeg[g], tn = trgCnt[g];
+  const int64_t tBeg = trgBeg[g], tn = trgCnt[g];
   const int64_t e0 = ptr[row], e1 = ptr[row + 1];
   const double cx = ctr[3 * g], cy = ctr[3 * g + 1], cz = ctr[3 * g + 2];
-  const int64_t pairs = (tn + 1) / 2;
-  const int TG = pairs > 16 ? 32 : (pairs > 8 ? 16 : 8), S = 32 / TG;
-  const int tl = lane % TG, sp = lane / TG;
   const float c4pi = (float)(1.0 / (4.0 * 3.14159265358979323846));
-  for (int64_t t0 = 0; t0 < tn; t0 += 2 * TG) {
+  for (int64_t t0 = (int64_t)blockIdx.y * tb; t0 < tn; t0 += (int64_t)gridDim.y * tb) {
+    const int nt = (int)min((int64_t)tb, tn - t0);  // at most 64
+    const int TG = (nt + 1) / 2, S = 32 / TG;
+    const int tl = lane % TG, sp = lane / TG;
     const int64_t ta = t0 + tl, tbb = t0 + tl + TG;
-    const bool actA = ta < tn, actB = tbb < tn;
+    const bool actA = sp < S, actB = actA && tl + TG < nt;
     unsigned long long txh = 0, tyh = 0, tzh = 0, txl = 0, tyl = 0, tzl = 0;
     {
       float h[2][3] = {{0, 0, 0}, {0, 0, 0}}, l[2][3] = {{0, 0, 0}, {0, 0, 0}};
       for (int q = 0; q < 2; q++) {
         const int64_t t = q ? tbb : ta;
         if (!(q ? actB : actA)) continue;
-        const double d[3] = {trg[3 * (tb + t)] - cx, trg[3 * (tb + t) + 1] - cy, trg[3 * (tb + t) + 2] - cz};
+        const double d[3] = {trg[3 * (tBeg + t)] - cx, trg[3 * (tBeg + t) + 1] - cy, trg[3 * (tBeg + t) + 2] - cz};
         for (int c = 0; c < 3; c++) {
           h[q][c] = (float)d[c];
           l[q][c] = (float)(d[c] - h[q][c]);
@@ -378,7 +459,7 @@ __global__ void __launch_bounds__(32 * NW_WARPS, 6)
       if (lane == 0) ePre[warp][0] = 0;
       __syncwarp();
       const int total = running;
-      for (int base = 0; base < total; base += NW_CH) {
+      for (int base = sub * NW_CH; base < total; base += WS * NW_CH) {
         const int cnt = min(NW_CH, total - base);
         __syncwarp();
         for (int i = lane; i < cnt; i += 32) {
@@ -424,20 +505,40 @@ __global__ void __launch_bounds__(32 * NW_WARPS, 6)
         }
       }
     }
-    if (S > 1) {
 #pragma unroll
-      for (int r = 0; r < KB; r++)
-        for (int o = TG; o < 32; o <<= 1) {
-          acc[0][r] += __shfl_xor_sync(0xffffffffu, acc[0][r], o);
-          acc[1][r] += __shfl_xor_sync(0xffffffffu, acc[1][r], o);
-        }
+    for (int r = 0; r < KB; r++) {
+      const double a = acc[0][r], b = acc[1][r];
+      for (int k = 1; k < S; k++) {
+        acc[0][r] += __shfl_sync(0xffffffffu, a, (lane + k * TG) & 31);
+        acc[1][r] += __shfl_sync(0xffffffffu, b, (lane + k * TG) & 31);
+      }
     }
-    if (sp == 0) {
+    if constexpr (WS > 1) {  // the warps' sums meet in the first one, in warp order
+      for (int w = 1; w < WS; w++) {
+        __syncthreads();
+        if (sub == w && sp == 0) {
+#pragma unroll
+          for (int r = 0; r < KB; r++) {
+            sRed[(2 * tl) * KB + r] = acc[0][r];
+            sRed[(2 * tl + 1) * KB + r] = acc[1][r];
+          }
+        }
+        __syncthreads();
+        if (sub == 0 && sp == 0) {
+#pragma unroll
+          for (int r = 0; r < KB; r++) {
+            acc[0][r] += sRed[(2 * tl) * KB + r];
+            acc[1][r] += sRed[(2 * tl + 1) * KB + r];
+          }
+        }
+      }
+    }
+    if (sub == 0 && sp == 0) {
 #pragma unroll
       for (int r = 0; r < KB; r++) {
         if (rhs0 + r >= nrhs) break;
-        if (actA) val[(int64_t)(rhs0 + r) * valStride + tb + ta] += acc[0][r];
-        if (actB) val[(int64_t)(rhs0 + r) * valStride + tb + tbb] += acc[1][r];
+        val[(int64_t)(rhs0 + r) * valStride + tBeg + ta] += acc[0][r];
+        if (actB) val[(int64_t)(rhs0 + r) * valStride + tBeg + tbb] += acc[1][r];
       }
     }
   }
@@ -1425,14 +1526,20 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
   cudaEventRecord(D.ev[EV_UP_GEMM], st);
   auto near = [&](const int64_t* ptr, const int32_t* idx, cudaStream_t sn) {
     if (nl == 0) return;
-    if constexpr (KT == LAP_S_U)  // two targets a thread, packed FP32x2, a warp per leaf
-      k_p2p_near32_lap2w<KB><<<dim3((nl + NW_WARPS - 1) / NW_WARPS, kb), 32 * NW_WARPS, 0, sn>>>(
-          nl, D.nearOrder, D.evtrLeaves, ptr, idx, D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt, D.src, D.den32, den32Blk,
-          D.trg, D.ctr, D.valK, valStride, kc);
-    else
-      k_p2p_near32<KT, KB><<<dim3(nl, kb), MX_THREADS, 0, sn>>>(D.evtrLeaves, ptr, idx, D.srcBeg, D.srcCnt, D.trgBeg,
-                                                               D.trgCnt, D.src, D.nrm, D.den32, den32Blk, D.trg, D.ctr,
-                                                               D.valK, valStride, kc, mu, ve);
+    constexpr int TB = 64;  // two targets a lane
+    const bool few = nl < near_warps(D.numSMs);
+    const dim3 grid(few ? nl : (nl + NW_WARPS - 1) / NW_WARPS, near_blocks(D, few ? TB / 2 : TB), kb);
+    if constexpr (KT == LAP_S_U) {  // packed FP32x2
+      auto* k = few ? k_p2p_near32_lap2w<KB, NW_WARPS> : k_p2p_near32_lap2w<KB, 1>;
+      k<<<grid, 32 * NW_WARPS, 0, sn>>>(nl, few ? TB / 2 : TB, D.nearOrder, D.evtrLeaves, ptr, idx, D.srcBeg, D.srcCnt,
+                                        D.trgBeg, D.trgCnt, D.src, D.den32, den32Blk, D.trg, D.ctr, D.valK,
+                                        valStride, kc);
+    } else {
+      auto* k = few ? k_p2p_near32<KT, KB, NX_WARPS> : k_p2p_near32<KT, KB, 1>;
+      k<<<grid, 32 * NX_WARPS, 0, sn>>>(nl, few ? TB / 2 : TB, D.nearOrder, D.evtrLeaves, ptr, idx, D.srcBeg, D.srcCnt,
+                                        D.trgBeg, D.trgCnt, D.src, D.nrm, D.den32, den32Blk, D.trg, D.ctr, D.valK,
+                                        valStride, kc, mu, ve);
+    }
     ls->launches++;
   };
   auto nearAll = [&](cudaStream_t sn) {

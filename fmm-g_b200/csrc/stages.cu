@@ -70,48 +70,62 @@ constexpr int P2P_TILE = 128;
 constexpr int P2P_MAXE = 256;
 
 
-// k_p2p_near_w: the same sums, one warp per evaluator leaf (P2PW_WARPS
-// leaves a CTA) and no CTA-wide barrier: the warp builds its entry table
-// (source ranges and their prefix counts, a shuffle scan per 32 entries),
-// stages P2PW_CH sources at a time in its own slice of shared memory, and
-// splits them over S = 32 / TG lane groups of TG = 8, 16 or 32 targets; the
-// groups' FP64 partial sums meet through warp shuffles.  A leaf with few
-// targets no longer leaves most of a CTA idle behind block barriers.
+// k_p2p_near_w: the same sums, by warps without a CTA-wide barrier in their
+// loops.  A warp builds its entry table (source ranges and their prefix counts,
+// a shuffle scan per 32 entries) and stages P2PW_CH sources at a time in its
+// own slice of shared memory.  Its lanes are S groups of TG: a lane of a group
+// holds PR targets (4 for scalar kernels, 2 otherwise), TG = ceil(targets / PR)
+// and S = 32 / TG split the sources, so that 17 targets, the mean of the
+// 1M-point workload's leaves, occupy 30 lanes where one target a lane left 15
+// idle; the PR independent inverse square roots of a lane hide the latency of
+// the FP64 pipe.  The groups' partial sums meet through warp shuffles.
+// The 4 warps of a CTA share a leaf and take its chunks of sources in turn (one
+// warp a leaf left the GPU idle behind the longest leaves, and all of it with
+// few leaves), their sums meet in shared memory in warp order; blocks of tb
+// targets of a leaf run as separate CTAs (grid.y).
+// Against one warp a leaf and one target a lane: 65,536 points in 554 leaves 2.58
+// -> 0.37 ms, Stokes 60,007 points 1.28 -> 0.28, 1M points in 62,000 leaves 2.15 ->
+// 1.54 (1.93 with one warp a leaf).
 constexpr int P2PW_WARPS = 4, P2PW_CH = 64, P2PW_MAXE = 128;
 template <int KT>
+constexpr int p2pw_targets() {
+  return KTraits<KT>::SD * KTraits<KT>::TD == 1 ? 4 : 2;
+}
+template <int KT>
 __global__ void __launch_bounds__(32 * P2PW_WARPS)
-    k_p2p_near_w(int nLeaves, const int32_t* __restrict__ rows, const int64_t* __restrict__ ptr,
+    k_p2p_near_w(int tb, const int32_t* __restrict__ rows, const int64_t* __restrict__ ptr,
                  const int32_t* __restrict__ idx, const int64_t* __restrict__ srcBeg,
                  const int64_t* __restrict__ srcCnt, const int64_t* __restrict__ trgBeg,
                  const int64_t* __restrict__ trgCnt, const double* __restrict__ src, const double* __restrict__ nrm,
                  const double* __restrict__ den, const double* __restrict__ trg, double* __restrict__ val, double mu,
                  double ve) {
-  constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD, NRM = KTraits<KT>::NRM;
+  constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD, NRM = KTraits<KT>::NRM, PR = p2pw_targets<KT>();
+  constexpr int WS = P2PW_WARPS;
   __shared__ double sPos[P2PW_WARPS][P2PW_CH * 3];
   __shared__ double sNrm[P2PW_WARPS][NRM ? P2PW_CH * 3 : 1];
   __shared__ double sDen[P2PW_WARPS][P2PW_CH * SD];
   __shared__ int64_t eBeg[P2PW_WARPS][P2PW_MAXE];
   __shared__ int32_t ePre[P2PW_WARPS][P2PW_MAXE + 1];
+  __shared__ double sRed[WS][32 * PR * TD];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * P2PW_WARPS + warp;
-  if (row >= nLeaves) return;  // no CTA-wide barrier below
+  const int row = blockIdx.x;
   const int g = rows[row];
-  const int64_t tb = trgBeg[g], tn = trgCnt[g];
+  const int64_t tBeg = trgBeg[g], tn = trgCnt[g];
   const int64_t e0 = ptr[row], e1 = ptr[row + 1];
-  const int TG = tn > 16 ? 32 : (tn > 8 ? 16 : 8), S = 32 / TG;
-  const int tl = lane % TG, sp = lane / TG;
-  for (int64_t t0 = 0; t0 < tn; t0 += TG) {
-    const int64_t t = t0 + tl;
-    const bool act = t < tn;
-    double tx = 0, ty = 0, tz = 0;
-    if (act) {
-      tx = trg[3 * (tb + t)];
-      ty = trg[3 * (tb + t) + 1];
-      tz = trg[3 * (tb + t) + 2];
-    }
-    double acc[TD];
+  for (int64_t t0 = (int64_t)blockIdx.y * tb; t0 < tn; t0 += (int64_t)gridDim.y * tb) {
+    const int nt = (int)min((int64_t)tb, tn - t0);  // at most 32 PR
+    const int TG = (nt + PR - 1) / PR, S = 32 / TG;
+    const int tl = lane % TG, sp = lane / TG;
+    double tx[PR], ty[PR], tz[PR], acc[PR][TD];
 #pragma unroll
-    for (int c = 0; c < TD; c++) acc[c] = 0.0;
+    for (int r = 0; r < PR; r++) {
+      const int64_t t = tBeg + t0 + min(tl + r * TG, nt - 1);  // past the last: repeated, not stored
+      tx[r] = trg[3 * t];
+      ty[r] = trg[3 * t + 1];
+      tz[r] = trg[3 * t + 2];
+#pragma unroll
+      for (int c = 0; c < TD; c++) acc[r][c] = 0.0;
+    }
     for (int64_t ec = e0; ec < e1; ec += P2PW_MAXE) {
       const int ne = (int)min((int64_t)P2PW_MAXE, e1 - ec);
       __syncwarp();
@@ -136,7 +150,7 @@ __global__ void __launch_bounds__(32 * P2PW_WARPS)
       if (lane == 0) ePre[warp][0] = 0;
       __syncwarp();
       const int total = running;
-      for (int base = 0; base < total; base += P2PW_CH) {
+      for (int base = warp * P2PW_CH; base < total; base += WS * P2PW_CH) {
         const int cnt = min(P2PW_CH, total - base);
         __syncwarp();
         for (int i = lane; i < cnt; i += 32) {
@@ -159,20 +173,39 @@ __global__ void __launch_bounds__(32 * P2PW_WARPS)
           for (int c = 0; c < SD; c++) sDen[warp][SD * i + c] = den[s2 * SD + c];
         }
         __syncwarp();
-        if (act) {
-          for (int i = sp; i < cnt; i += S)
-            kaccum<KT, double, double>(tx - sPos[warp][3 * i], ty - sPos[warp][3 * i + 1], tz - sPos[warp][3 * i + 2],
-                                       NRM ? &sNrm[warp][3 * i] : nullptr, &sDen[warp][SD * i], acc, mu, ve);
+        if (sp < S) {
+          for (int i = sp; i < cnt; i += S) {
+            const double qx = sPos[warp][3 * i], qy = sPos[warp][3 * i + 1], qz = sPos[warp][3 * i + 2];
+#pragma unroll
+            for (int r = 0; r < PR; r++)
+              kaccum<KT, double, double>(tx[r] - qx, ty[r] - qy, tz[r] - qz, NRM ? &sNrm[warp][3 * i] : nullptr,
+                                         &sDen[warp][SD * i], acc[r], mu, ve);
+          }
         }
       }
     }
 #pragma unroll
-    for (int c = 0; c < TD; c++)
-      for (int o = TG; o < 32; o <<= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-    if (act && sp == 0) {
+    for (int r = 0; r < PR; r++)
 #pragma unroll
-      for (int c = 0; c < TD; c++) val[(tb + t) * TD + c] += acc[c];
+      for (int c = 0; c < TD; c++) {
+        const double own = acc[r][c];
+        for (int k = 1; k < S; k++) acc[r][c] += __shfl_sync(0xffffffffu, own, (lane + k * TG) & 31);
+      }
+    if (sp == 0) {
+#pragma unroll
+      for (int r = 0; r < PR; r++)
+        if (tl + r * TG < nt)
+#pragma unroll
+          for (int c = 0; c < TD; c++) sRed[warp][(tl + r * TG) * TD + c] = acc[r][c];
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nt * TD; i += blockDim.x) {
+      double s = 0.0;
+#pragma unroll
+      for (int w = 0; w < WS; w++) s += sRed[w][i];
+      val[(tBeg + t0) * TD + i] += s;
+    }
+    __syncthreads();
   }
 }
 
@@ -779,6 +812,8 @@ std::string dev_upload(const Plan& P, DevState& D, const double* src, const doub
             ijk.push_back(i | (j << 8) | (k << 16));
     FMMG_TRY(dput(D, D.surfIJK, ijk));
   }
+  D.maxLeafTrg = 0;
+  for (int32_t g : P.evtrLeaves) D.maxLeafTrg = std::max(D.maxLeafTrg, P.trgCnt[g]);
   lap(0);
   // work lists
   FMMG_TRY(dput(D, D.evtrLeaves, P.evtrLeaves));
@@ -897,8 +932,9 @@ static void launch_near(const Plan& P, DevState& D, const int64_t* ptr, const in
                         cudaStream_t sn) {
   int n = (int)P.evtrLeaves.size();
   if (n == 0) return;
-  k_p2p_near_w<KT><<<(n + P2PW_WARPS - 1) / P2PW_WARPS, 32 * P2PW_WARPS, 0, sn>>>(
-      n, D.evtrLeaves, ptr, idx, D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt, D.src, D.nrm, D.den, D.trg, D.val,
+  constexpr int TB = 16 * p2pw_targets<KT>();  // half the lanes' targets: the sources split in two at least
+  k_p2p_near_w<KT><<<dim3(n, near_blocks(D, TB)), 32 * P2PW_WARPS, 0, sn>>>(
+      TB, D.evtrLeaves, ptr, idx, D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt, D.src, D.nrm, D.den, D.trg, D.val,
       P.o.coefs[0], P.o.coefs[1]);
   if (ls) ls->launches++;
 }
