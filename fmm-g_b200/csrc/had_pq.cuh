@@ -25,6 +25,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "had_smem.cuh"
 
 namespace fmmg {
@@ -36,6 +38,16 @@ inline size_t pq_smem_bytes(int fw) {
   return (size_t)317 * fw * sizeof(C);
 }
 constexpr int PQ_PARENTS = 128;  // output parents per CTA
+
+// Output parents per CTA of the scalar Hadamard kernels: `most` (the tuned
+// figure), fewer where that many would leave fewer than `ctas` CTAs, down to one
+// for each scheduler of an SM (4): with 72 parents and 10 slices of frequencies 10
+// CTAs of 128 ran one after another on 10 SMs what 180 of 4 share out (FP64,
+// 4,000 points: 0.141 -> 0.057 ms).
+inline int had_rows_per_cta(int nRows, int slices, int ctas, int most) {
+  const int64_t r = ((int64_t)nRows * slices + ctas - 1) / ctas;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(most, std::max<int64_t>(4, r)));
+}
 
 template <typename C>
 __device__ __forceinline__ void pq_cfma(C& acc, const C t, const C d) {
@@ -636,9 +648,13 @@ static __global__ void __launch_bounds__(PQX_THREADS, 1)
 // products are 9 complex multiplies and 18 complex multiply-adds.  Per right-
 // hand side that is a few more FP32 operations than the 27-product kernel but
 // R times fewer translation reads.
-// Lanes: FB = 4 R frequencies x (8 / R) groups of R right-hand sides of a
-// block of 8; a warp owns one target parent; the CTA stages T'[27][27][FB].
-// Grid (rows / rows per CTA, nEff / FB, ceil(nrhs / 8)); dynamic shared
+// Lanes: FB = 32 / G frequencies x G groups of R right-hand sides of a block of
+// RW = G R; a warp owns one target parent; the CTA stages T'[27][27][FB].
+// Blocks of 8 take R = 4, G = 2 (or R = 2, G = 4), 2 to 4 right-hand sides G = 1:
+// in a block of 8 with 3 of them half of the lanes had none (Laplace double
+// layer, 50,021 points, k = 3: 0.295 -> 0.152 ms, its two
+// transforms 0.089 -> 0.062).
+// Grid (rows / rows per CTA, nEff / FB, ceil(nrhs / RW)); dynamic shared
 // memory 27 * 27 * FB * 8 bytes.
 __device__ __forceinline__ unsigned long long ho_cmul(float2 t, unsigned long long u) {
   unsigned long long r;
@@ -712,32 +728,32 @@ __device__ __forceinline__ void ho_ld256(const float* p, float4& a, float4& b) {
       : "l"(p));
 }
 
-template <int R>
+template <int R, int G>
 static __global__ void __launch_bounds__(PQX_THREADS, 1)
     k_m2l_had_o(int nRows, const int32_t* __restrict__ rowOut, const int64_t* __restrict__ nPtr,
                 const int8_t* __restrict__ nOff, const int32_t* __restrict__ nIn, const float2* __restrict__ effIn,
                 PqLayout inL, const float2* __restrict__ Tw, float2* __restrict__ effOut, PqLayout outL, int nEff,
                 int nrhs, float nrmfc) {
   static_assert(R == 2 || R == 4, "two or four right-hand sides a lane");
-  constexpr int G = 8 / R, FB = 32 / G;
+  constexpr int RW = G * R, FB = 32 / G;
   extern __shared__ __align__(16) unsigned char ho_smem[];
   float2* Ts = reinterpret_cast<float2*>(ho_smem);  // [27 offsets][27 combinations][FB frequencies]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int fl = lane % FB, rg = lane / FB;
   const int f0 = blockIdx.y * FB;
   const int f = f0 + fl;
-  const int rhs0 = blockIdx.z * 8 + rg * R;  // this lane's right-hand sides rhs0 .. rhs0 + R - 1
+  const int rhs0 = blockIdx.z * RW + rg * R;  // this lane's right-hand sides rhs0 .. rhs0 + R - 1
   for (int i = threadIdx.x; i < W8_OFFS * 27 * FB; i += blockDim.x) {
     const int oj = i / FB, ff = f0 + (i % FB);
     Ts[i] = ff < nEff ? Tw[(int64_t)oj * nEff + ff] : make_float2(0.f, 0.f);
   }
   __syncthreads();
   const bool act = f < nEff && rhs0 < nrhs;
-  // the block holds 8 right-hand-side slots, so rhs0 + R - 1 is in the buffer
-  const int64_t lanePos = act ? (int64_t)f * 8 + rg * R : 0;
+  // the block holds RW right-hand-side slots, so rhs0 + R - 1 is in the buffer
+  const int64_t lanePos = act ? (int64_t)f * RW + rg * R : 0;
   const float4* inF = reinterpret_cast<const float4*>(effIn + (act ? blockIdx.z * inL.blk : 0) + lanePos);
   float2* outF = effOut + blockIdx.z * outL.blk + lanePos;
-  const int64_t inSlot4 = inL.slot / 2;  // float4 units (slot strides are multiples of 8 float2)
+  const int64_t inSlot4 = inL.slot / 2;  // float4 units (slot strides are multiples of RW float2)
   // the warp's parent's neighbour entries (input child slots, offset code),
   // up to 32 at a time, so each neighbour starts on shared-memory reads
   __shared__ int4 sIn[PQX_THREADS / 32][32][2];

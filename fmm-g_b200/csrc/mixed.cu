@@ -1561,14 +1561,16 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
   cudaEventRecord(D.ev[EV_NEAR], st);
   const int nsrc = (int)P.vSrcNodes.size(), ntrg = (int)P.vTrgNodes.size(), npar = (int)P.vParents.size();
   const int64_t effDR = (int64_t)nsrc * P.nEff32 * P.sdm, effVR = (int64_t)ntrg * P.nEff32 * P.tdm;
-  // Spectra in blocks of RW interleaved right-hand sides.  Scalar kernels: 8,
-  // or 1 for a single right-hand side and for the list form.  Vector kernels:
-  // the smallest power of two that holds them, 4 instead of 8 where that
-  // leaves fewer right-hand sides of padding.
+  // Spectra in blocks of RW interleaved right-hand sides: the smallest power of
+  // two that holds them, 4 instead of 8 where that leaves fewer right-hand
+  // sides of padding; for scalar kernels 1 in the list form and 8 in the forms
+  // of the Hadamard kernel that tuning alone selects.
   const bool scalar = P.sdm == 1 && P.tdm == 1;
   const bool r8 = scalar && kc >= 2 && D.hadPQ;
+  const bool hadO = D.hadW && D.m2lTw32 && D.tune.hadRhsPerThread >= 3;
   int lgRW = r8 ? 3 : 0;
-  if (!scalar) {
+  if (!scalar || (r8 && D.hadW && D.m2lTw32 && D.tune.hadRhsPerThread == 4)) {
+    lgRW = 0;
     while (lgRW < 3 && (1 << lgRW) < kc) lgRW++;
     if (lgRW == 3 && (kc + 3) / 4 * 4 < (kc + 7) / 8 * 8) lgRW = 2;
   }
@@ -1616,24 +1618,27 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
       if (!r8) {  // planes of one right-hand side
         const size_t smem = pqx_smem_bytes<32>();
         cudaFuncSetAttribute(k_m2l_had_pqx2<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        dim3 g1((npar + D.tune.hadRows - 1) / D.tune.hadRows, (P.nEff32 + 31) / 32, kc);
+        const int sl = (P.nEff32 + 31) / 32, hr = had_rows_per_cta(npar, sl * kc, 6 * D.numSMs, D.tune.hadRows);
+        dim3 g1((npar + hr - 1) / hr, sl, kc);
         k_m2l_had_pqx2<32, false><<<g1, PQX_THREADS, smem, st>>>(
             npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen32, PqLayout{effDR, P.nEff32}, D.m2lT32, D.effVal32,
             PqLayout{effVR, P.nEff32}, 1, 0, P.nEff32, kc, nrmfc, D.transIdDev);
-      } else if (D.hadW && D.m2lTw32 && D.tune.hadRhsPerThread >= 3) {  // output-child accumulators
-#define FMMG_HADO(R_)                                                                                         \
+      } else if (hadO) {  // output-child accumulators
+#define FMMG_HADO(R_, G_)                                                                                     \
   do {                                                                                                        \
-    constexpr int FB = 4 * (R_);                                                                              \
+    constexpr int FB = 32 / (G_);                                                                             \
     const size_t smem = (size_t)W8_OFFS * 27 * FB * sizeof(float2);                                           \
-    cudaFuncSetAttribute(k_m2l_had_o<R_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);            \
-    dim3 go((npar + D.tune.hadRows - 1) / D.tune.hadRows, (P.nEff32 + FB - 1) / FB, nblk);                    \
-    k_m2l_had_o<R_><<<go, PQX_THREADS, smem, st>>>(npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen32,     \
-                                                   PqLayout{blkDen, (int64_t)P.nEff32 * 8}, D.m2lTw32,        \
-                                                   D.effVal32, PqLayout{blkVal, (int64_t)P.nEff32 * 8},       \
-                                                   P.nEff32, kc, nrmfc);                                      \
+    cudaFuncSetAttribute(k_m2l_had_o<R_, G_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
+    const int sl = (P.nEff32 + FB - 1) / FB;                                                                  \
+    const int hr = had_rows_per_cta(npar, sl * nblk, 3 * D.numSMs, D.tune.hadRows);                           \
+    k_m2l_had_o<R_, G_><<<dim3((npar + hr - 1) / hr, sl, nblk), PQX_THREADS, smem, st>>>(                     \
+        npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen32, PqLayout{blkDen, (int64_t)P.nEff32 * RW},      \
+        D.m2lTw32, D.effVal32, PqLayout{blkVal, (int64_t)P.nEff32 * RW}, P.nEff32, kc, nrmfc);                \
   } while (0)
-        if (D.tune.hadRhsPerThread == 4) FMMG_HADO(4);
-        else FMMG_HADO(2);
+        if (D.tune.hadRhsPerThread == 3) FMMG_HADO(2, 4);
+        else if (RW == 8) FMMG_HADO(4, 2);
+        else if (RW == 4) FMMG_HADO(4, 1);
+        else FMMG_HADO(2, 1);
 #undef FMMG_HADO
       } else if (D.hadW && D.m2lTw32 && D.tune.hadRhsPerThread == 2) {  // 27-product form, 2 RHS a thread
         const size_t smem = (size_t)W8_OFFS * 27 * W8X2_F * sizeof(float2);
