@@ -540,6 +540,7 @@ static std::string adj_prepare(const Plan& P, DevState& D) {
     D.adjListsReady = true;
   }
   if (D.adjOpsStale) {
+    OpBlocks scope(D);
     const int ue = P.nUE * P.sdm, uc = P.nUC * P.tdm, de = P.nDE * P.sdm, dc = P.nDC * P.tdm;
     std::vector<double> t;
     t = transposed(P.uc2ue, ue, uc);

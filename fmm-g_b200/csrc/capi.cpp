@@ -228,8 +228,9 @@ fmmg_status fmmg_setup(fmmg_handle* h, int64_t ns, const double* src, const doub
     if (h->setupDone) {
       drop_graph(h);
       // the blocks of this setup serve the next one (dev_alloc), and what is
-      // left over is freed at its end
-      fmmg::dev_release_for_reuse(h->dev);
+      // left over is freed at its end; the operator tables stay on the device
+      // unless the caller replaced some
+      fmmg::dev_release_for_reuse(h->dev, !h->tablesReplaced && !h->opsDirty);
       h->dDenIO = h->dValIO = nullptr;
       h->dDenK = h->dValK = nullptr;
       h->dAdjW = h->dAdjG = h->dAdjGrad = h->dAdjDen = nullptr;

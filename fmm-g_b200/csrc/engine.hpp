@@ -150,10 +150,18 @@ struct DevState {
   // lists, operator tables, work arrays and the rest
   double uploadMs[4] = {0, 0, 0, 0};
   int lastLaunches = 0;  // kernels launched by the last single-RHS evaluate  // interval k = ev[k] .. ev[k+1]
-  // every device block of the handle (sizes in allocBytes); after a re-setup
-  // the previous setup's blocks wait in spare for dev_alloc to reuse them
+  // every device block of the handle (sizes in allocBytes) but the operator
+  // tables'; after a re-setup the previous setup's blocks wait in spare for
+  // dev_alloc to reuse them
   std::vector<void*> allocs;
   std::vector<size_t> allocBytes;
+  // the operator tables' blocks (allocated under an OpBlocks scope): they do not
+  // depend on the points, so a re-setup keeps them while the tables are the
+  // built ones
+  std::vector<void*> opAllocs;
+  std::vector<size_t> opAllocBytes;
+  bool allocOps = false;
+  bool opsHeld = false;  // the FP64 tables are on the device
   struct Block {
     void* p;
     size_t bytes;
@@ -169,6 +177,14 @@ inline unsigned near_blocks(const DevState& D, int tb) {
   const int64_t b = (D.maxLeafTrg + tb - 1) / tb;
   return (unsigned)(b < 1 ? 1 : (b > 64 ? 64 : b));
 }
+
+struct OpBlocks {  // dev_alloc calls in its scope are operator tables
+  DevState& D;
+  explicit OpBlocks(DevState& d) : D(d) { D.allocOps = true; }
+  ~OpBlocks() { D.allocOps = false; }
+  OpBlocks(const OpBlocks&) = delete;
+  OpBlocks& operator=(const OpBlocks&) = delete;
+};
 
 // counts of the last stage launch list (for reporting)
 struct LaunchStats {
@@ -186,8 +202,10 @@ cudaError_t dev_alloc(DevState& D, void** p, size_t bytes);
 void dev_free(DevState& D);
 // re-setup: after the handle's streams drain, every block moves to D.spare
 // for the next setup's dev_alloc calls and the pointers are cleared as by
-// dev_free; dev_trim then frees the blocks nothing reused
-void dev_release_for_reuse(DevState& D);
+// dev_free; dev_trim then frees the blocks nothing reused.  keepOps: the
+// operator tables' blocks and pointers stay as they are (with the tables
+// replaced by the caller, the built ones have to be uploaded again)
+void dev_release_for_reuse(DevState& D, bool keepOps);
 void dev_trim(DevState& D);
 // run one right-hand side; den/val are device arrays in caller order
 std::string dev_evaluate(const Plan& P, DevState& D, const double* dDenCaller, double* dValCaller,

@@ -1351,6 +1351,7 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     FMMG_TRY(dalloc(D, D.valK, (size_t)kc * std::max<int64_t>(P.nt, 1) * P.td));
     FMMG_TRY(dalloc(D, D.m2tPart, (size_t)kc * std::max<int64_t>(D.m2tPartTargets, 1) * P.tdm));
     if (!D.l2l32) {
+      OpBlocks scope(D);
       FMMG_TRY(dalloc(D, D.l2l32, P.l2l.size()));
       FMMG_TRY(dalloc(D, D.m2lT32, P.m2lT32.size()));
       if (P.sdm == 1 && P.tdm == 1) FMMG_TRY(dalloc(D, D.m2lTw32, (size_t)27 * 27 * P.nEff32));
@@ -1364,6 +1365,7 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     D.mixedK = kc;
   }
   if (D.mixedOpsStale) {
+    OpBlocks scope(D);
     auto put = [&](float* dst, const std::vector<double>& v) -> std::string {
       std::vector<float> f(v.begin(), v.end());
       FMMG_CK(cudaMemcpy(dst, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));

@@ -575,8 +575,8 @@ cudaError_t dev_alloc(DevState& D, void** p, size_t bytes) {
       return e;
     }
   }
-  D.allocs.push_back(q);
-  D.allocBytes.push_back(bytes);
+  (D.allocOps ? D.opAllocs : D.allocs).push_back(q);
+  (D.allocOps ? D.opAllocBytes : D.allocBytes).push_back(bytes);
   *p = q;
   return cudaSuccess;
 }
@@ -587,8 +587,9 @@ void dev_trim(DevState& D) {
 }
 
 static void dev_clear(DevState& D);
+static void dev_clear_ops(DevState& D);
 
-void dev_release_for_reuse(DevState& D) {
+void dev_release_for_reuse(DevState& D, bool keepOps) {
   // the blocks may still be read by queued work of the handle
   if (D.stream) cudaStreamSynchronize(D.stream);
   if (D.side) cudaStreamSynchronize(D.side);
@@ -596,14 +597,44 @@ void dev_release_for_reuse(DevState& D) {
   D.allocs.clear();
   D.allocBytes.clear();
   dev_clear(D);
+  if (keepOps) return;
+  for (size_t i = 0; i < D.opAllocs.size(); i++)
+    D.spare.push_back(DevState::Block{D.opAllocs[i], D.opAllocBytes[i]});
+  D.opAllocs.clear();
+  D.opAllocBytes.clear();
+  dev_clear_ops(D);
 }
 
 void dev_free(DevState& D) {
   for (void* p : D.allocs) cudaFree(p);
+  for (void* p : D.opAllocs) cudaFree(p);
   D.allocs.clear();
   D.allocBytes.clear();
+  D.opAllocs.clear();
+  D.opAllocBytes.clear();
   dev_trim(D);
   dev_clear(D);
+  dev_clear_ops(D);
+}
+
+// the operator tables' pointers and flags back to "nothing uploaded"
+static void dev_clear_ops(DevState& D) {
+  D.uc2ue = D.m2m = D.dc2de = D.l2l = nullptr;
+  D.m2lT = nullptr;
+  D.l2l32 = nullptr;
+  D.upF1 = D.upF2 = D.dnF1 = D.dnF2 = nullptr;
+  D.m2mUp32 = nullptr;
+  for (DevState::OpT* op : {&D.tL2L, &D.tUpF1, &D.tUpF2, &D.tDnF1, &D.tDnF2, &D.tM2MUp}) *op = DevState::OpT();
+  for (TcOp* op : {&D.cL2L, &D.cUpF1, &D.cUpF2, &D.cDnF1, &D.cDnF2, &D.cM2MUp}) *op = TcOp();  // memory freed above
+  D.transIdDev = nullptr;
+  D.hvT = nullptr;
+  D.hvT32 = nullptr;
+  D.m2lT32 = nullptr;
+  D.m2lTw32 = nullptr;
+  D.uc2ueT = D.m2mT = D.dc2deT = D.l2lT = nullptr;
+  D.adjOpsStale = true;
+  D.mixedOpsStale = true;
+  D.opsHeld = false;
 }
 
 // every pointer and flag of D back to "nothing uploaded" (the memory itself
@@ -617,22 +648,11 @@ static void dev_clear(DevState& D) {
     D.evFork = D.evUp = D.evSide = nullptr;
   }
   D.evReady = false;
-  D.uc2ue = D.m2m = D.dc2de = D.l2l = nullptr;
-  D.m2lT = nullptr;
   D.chkPos = D.chkOut = nullptr;
   D.chkCap = 0;
   D.uchk32 = D.uden32 = D.dchk32 = D.dden32 = nullptr;
   D.effDen32 = D.effVal32 = nullptr;
-  D.l2l32 = nullptr;
-  D.upF1 = D.upF2 = D.dnF1 = D.dnF2 = D.upT32 = D.dnT32 = nullptr;
-  D.m2mUp32 = nullptr;
-  for (DevState::OpT* op : {&D.tL2L, &D.tUpF1, &D.tUpF2, &D.tDnF1, &D.tDnF2, &D.tM2MUp}) *op = DevState::OpT();
-  for (TcOp* op : {&D.cL2L, &D.cUpF1, &D.cUpF2, &D.cDnF1, &D.cDnF2, &D.cM2MUp}) *op = TcOp();  // memory freed above
-  D.transIdDev = nullptr;
-  D.hvT = nullptr;
-  D.hvT32 = nullptr;
-  D.m2lT32 = nullptr;
-  D.m2lTw32 = nullptr;
+  D.upT32 = D.dnT32 = nullptr;
   D.denK = D.valK = nullptr;
   D.den32 = nullptr;
   D.adjNearRows = D.adjNearIdx = D.adjFarRows = D.adjFarIdx = D.adjS2lRows = D.adjS2lIdx = nullptr;
@@ -644,14 +664,12 @@ static void dev_clear(DevState& D) {
   D.devErr = nullptr;
   D.vNbrTPtr = nullptr;
   D.vNbrOffT = nullptr;
-  D.uc2ueT = D.m2mT = D.dc2deT = D.l2lT = D.gradT = nullptr;
+  D.gradT = nullptr;
   D.adjListsReady = false;
   D.vListsReady = false;
   D.vTrgPtr = D.vSrcPtr = nullptr;
   D.vTrgEnt = D.vSrcEnt = nullptr;
-  D.adjOpsStale = true;
   D.mixedReady = false;
-  D.mixedOpsStale = true;
   D.mixedK = 0;
   D.mixedPassFor = D.mixedPassK = 0;
   D.m2tItems = nullptr;
@@ -690,6 +708,7 @@ static std::string hv_layout(const Plan& P, DevState& D) {
 
 std::string dev_upload_operators(const Plan& P, DevState& D) {
   FMMG_CK(cudaSetDevice(D.device));
+  OpBlocks scope(D);
   auto put = [&](double*& dst, const std::vector<double>& v) -> std::string {
     if (!dst) return dput(D, dst, v);
     FMMG_CK(cudaMemcpy(dst, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -711,6 +730,7 @@ std::string dev_upload_operators(const Plan& P, DevState& D) {
   else if (P.sdm == 3) FMMG_TRY((hv_layout<3, 3>(P, D)));
   D.mixedOpsStale = true;
   D.adjOpsStale = true;
+  D.opsHeld = true;
   return std::string();
 }
 
@@ -870,7 +890,10 @@ std::string dev_upload(const Plan& P, DevState& D, const double* src, const doub
   FMMG_TRY(dput(D, D.vRowOut, P.vRowOut));
   FMMG_TRY(dput(D, D.vNbrIn, P.vNbrIn));
   lap(1);
-  FMMG_TRY(dev_upload_operators(P, D));
+  // kept from the previous setup while the tables are the built ones: uploading
+  // them again took 15 of a setup's 20 ms at 30,000 Stokes points (the mixed
+  // form's, laid out on the host again, 50 ms more)
+  if (!D.opsHeld) FMMG_TRY(dev_upload_operators(P, D));
   lap(2);
   // work arrays
   const int64_t ue = (int64_t)P.nUE * P.sdm, uc = (int64_t)P.nUC * P.tdm;
