@@ -537,6 +537,7 @@ static std::string adj_prepare(const Plan& P, DevState& D) {
     FMMG_TRY(aj_put(D, D.vNbrOffT, P.vNbrOffT.data(), P.vNbrOffT.size()));
     FMMG_TRY(aj_put(D, D.vRowOutT, P.vRowOutT.data(), P.vRowOutT.size()));
     FMMG_TRY(aj_put(D, D.vNbrInT, P.vNbrInT.data(), P.vNbrInT.size()));
+    FMMG_CK(cudaStreamSynchronize(0));  // see dev_upload
     D.adjListsReady = true;
   }
   if (D.adjOpsStale) {
@@ -551,6 +552,7 @@ static std::string adj_prepare(const Plan& P, DevState& D) {
     FMMG_TRY(aj_put(D, D.dc2deT, t.data(), t.size()));
     t = transposed(P.l2l, 8 * dc, de);
     FMMG_TRY(aj_put(D, D.l2lT, t.data(), t.size()));
+    FMMG_CK(cudaStreamSynchronize(0));  // see dev_upload
     D.adjOpsStale = false;
   }
   return std::string();

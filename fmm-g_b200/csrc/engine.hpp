@@ -81,7 +81,7 @@ struct DevState {
   // mixed-precision work arrays and FP32 operator copies (allocated on first use)
   float *uchk32 = nullptr, *uden32 = nullptr, *dchk32 = nullptr, *dden32 = nullptr;
   float2 *effDen32 = nullptr, *effVal32 = nullptr;
-  float* l2l32 = nullptr;
+  float* dnFold32 = nullptr;  // C2E down x L2L folded, FP32 [8 de][de] (dn_fold)
   float *upF1 = nullptr, *upF2 = nullptr, *dnF1 = nullptr, *dnF2 = nullptr;  // factored pinvs
   float *upT32 = nullptr, *dnT32 = nullptr;  // [k][nn][kUp|kDn] intermediate of the factored C2E
   float2* m2lT32 = nullptr;
@@ -115,7 +115,7 @@ struct DevState {
   // (1, 2: 27-product accumulators, 1 or 2 right-hand sides a thread; 3, 4:
   // output-child accumulators, 2 or 4 right-hand sides a thread)
   // tcMask: which FP32 GEMM classes the tensor-core path takes (bit 0 leaf
-  // C2E F1, 1 leaf C2E F2, 2 folded C2E x M2M, 3 L2L, 4 downward C2E F1,
+  // C2E F1, 1 leaf C2E F2, 2 folded C2E x M2M, 3 folded C2E x L2L, 4 downward C2E F1,
   // 5 downward C2E F2); tcProducts: 3 (hi*hi + hi*lo + lo*hi) or 4 (+ lo*lo)
   struct Tune {
     int hadRows = 128, pqParents = 128, gemmSplitMul = 2, hadRhsPerThread = 4, tcMask = 63, tcProducts = 3;
@@ -124,7 +124,7 @@ struct DevState {
   // CUDA-core kernel, 2 the 128 x 64 CUDA-core kernel
   int gemmPath = 1;
   // the same operators split and laid out for the tensor-core kernel
-  TcOp cL2L, cUpF1, cUpF2, cDnF1, cDnF2, cM2MUp;
+  TcOp cDnFold, cUpF1, cUpF2, cDnF1, cDnF2, cM2MUp;
   // FP32 operators transposed and zero padded for the wide-tile GEMM,
   // Wt[k][n]: K to a multiple of 16, N to a multiple of 160 (ld)
   struct OpT {
@@ -132,7 +132,7 @@ struct DevState {
     int ld = 0;
     size_t cap = 0;  // allocated floats
   };
-  OpT tL2L, tUpF1, tUpF2, tDnF1, tDnF2, tM2MUp;
+  OpT tDnFold, tUpF1, tUpF2, tDnF1, tDnF2, tM2MUp;
   // C2E up x M2M folded (Plan fold_c2e_m2m), FP32 [ue][8 ue]: the FP32 pass
   // takes a parent's upward density from its children's in one product
   float* m2mUp32 = nullptr;

@@ -41,6 +41,18 @@ __device__ __forceinline__ T gr_sel(const GrScale<T>& s, int i) {
   return m == 0 ? s.v[0] : (m == 1 ? s.v[1] : (m == 2 ? s.v[2] : s.v[3]));
 }
 
+// Rows of several levels in one launch: with rowDepth, ys holds the degrees and
+// a row's scale is 2^(-(its node's depth + rootLevel) degree)
+template <typename T>
+__device__ __forceinline__ GrScale<T> gr_row_scale(const GrScale<T>& ys, const int32_t* rowDepth, int level) {
+  GrScale<T> r = ys;
+  if (rowDepth) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) r.v[c] = (T)scalbn(1.0, -(int)(level * ys.v[c]));
+  }
+  return r;
+}
+
 template <typename T>
 struct GrVec;
 template <>
@@ -61,7 +73,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
     k_gemm_rows_t(int nrows, int nrhs, const int32_t* __restrict__ rows, const int32_t* __restrict__ chd, int xChild,
                   int yChild, const T* __restrict__ X, int64_t ldx, int64_t xRhs, const T* __restrict__ W,
                   T* __restrict__ Y, int64_t ldy, int64_t yRhs, int K, int N, GrScale<T> xs, GrScale<T> ys, T beta,
-                  int kChunk, T* __restrict__ part) {
+                  int kChunk, T* __restrict__ part, const int32_t* __restrict__ rowDepth, int rootLevel) {
   typedef typename GrVec<T>::V V;
   constexpr int VW = sizeof(V) / sizeof(T);  // 4 floats or 2 doubles
   static_assert(BK / VW == 4, "four vectors per tile row");
@@ -70,6 +82,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
   __shared__ __align__(16) T Bs[2][BK][PB];
   __shared__ const T* xrow[GR_BM];
   __shared__ T* yrow[GR_BM];
+  __shared__ int ylev[GR_BM];
   const int tid = threadIdx.x;
   const int r0 = blockIdx.x * GR_BM, n0 = blockIdx.y * GR_BN;
   if (tid < GR_BM) {
@@ -79,6 +92,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
       const int node = rows[r - q * nrows];
       xrow[tid] = X + q * xRhs + (int64_t)(xChild ? chd[node] : node) * ldx;
       yrow[tid] = Y + q * yRhs + (int64_t)(yChild ? chd[node] : node) * ldy;
+      ylev[tid] = rowDepth ? rowDepth[node] + rootLevel : 0;
     } else {
       xrow[tid] = nullptr;
       yrow[tid] = nullptr;
@@ -191,11 +205,12 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
   for (int i = 0; i < 8; i++) {
     T* yr = yrow[tm * 8 + i];
     if (!yr) continue;
+    const GrScale<T> yv = gr_row_scale(ys, rowDepth, ylev[tm * 8 + i]);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const int n = n0 + tn * 4 + j;
       if (n < N) {
-        const T v = acc[i][j] * gr_sel(ys, n);
+        const T v = acc[i][j] * gr_sel(yv, n);
         yr[n] = beta == T(0) ? v : beta * yr[n] + v;
       }
     }
@@ -207,7 +222,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     k_gemm_reduce_t(int nrows, int nrhs, const int32_t* __restrict__ rows, const int32_t* __restrict__ chd,
                     int yChild, T* __restrict__ Y, int64_t ldy, int64_t yRhs, int N, int splits,
-                    const T* __restrict__ part, GrScale<T> ys, T beta) {
+                    const T* __restrict__ part, GrScale<T> ys, T beta, const int32_t* __restrict__ rowDepth,
+                    int rootLevel) {
   const int64_t M = (int64_t)nrows * nrhs;
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= M * N) return;
@@ -218,7 +234,7 @@ __global__ void __launch_bounds__(256)
   const int q = (int)(r / nrows);
   const int node = rows[r - (int64_t)q * nrows];
   T* yr = Y + q * yRhs + (int64_t)(yChild ? chd[node] : node) * ldy;
-  const T v = s * gr_sel(ys, n);
+  const T v = s * gr_sel(gr_row_scale(ys, rowDepth, rowDepth ? rowDepth[node] + rootLevel : 0), n);
   yr[n] = beta == T(0) ? v : beta * yr[n] + v;
 }
 
@@ -250,11 +266,13 @@ static __global__ void __launch_bounds__(GW_THREADS, 2)
     k_gemm_rows_w(int nrows, int nrhs, const int32_t* __restrict__ rows, const int32_t* __restrict__ chd, int xChild,
                   int yChild, const float* __restrict__ X, int64_t ldx, int64_t xRhs, const float* __restrict__ Wt,
                   int ldw, float* __restrict__ Y, int64_t ldy, int64_t yRhs, int K, int N, GrScale<float> xs,
-                  GrScale<float> ys, float beta, int kChunk, float* __restrict__ part, int yVec) {
+                  GrScale<float> ys, float beta, int kChunk, float* __restrict__ part, int yVec,
+                  const int32_t* __restrict__ rowDepth, int rootLevel) {
   __shared__ __align__(16) float As[2][GW_BK][GW_PA];
   __shared__ __align__(16) float Bs[2][GW_BK][GW_PB];
   __shared__ const float* xrow[GW_BM];
   __shared__ float* yrow[GW_BM];
+  __shared__ int ylev[GW_BM];
   const int tid = threadIdx.x;
   const int r0 = blockIdx.x * GW_BM, n0 = blockIdx.y * GW_BN;
   if (tid < GW_BM) {
@@ -264,6 +282,7 @@ static __global__ void __launch_bounds__(GW_THREADS, 2)
       const int node = rows[r - q * nrows];
       xrow[tid] = X + q * xRhs + (int64_t)(xChild ? chd[node] : node) * ldx;
       yrow[tid] = Y + q * yRhs + (int64_t)(yChild ? chd[node] : node) * ldy;
+      ylev[tid] = rowDepth ? rowDepth[node] + rootLevel : 0;
     } else {
       xrow[tid] = nullptr;
       yrow[tid] = nullptr;
@@ -362,13 +381,14 @@ static __global__ void __launch_bounds__(GW_THREADS, 2)
     }
     return;
   }
-  float ysc[10];
-#pragma unroll
-  for (int j = 0; j < 10; j++) ysc[j] = gr_sel(ys, n0 + gw_col(tn, j)) * xsc;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     float* yr = yrow[tm * 8 + i];
     if (!yr) continue;
+    const GrScale<float> yv = gr_row_scale(ys, rowDepth, ylev[tm * 8 + i]);
+    float ysc[10];
+#pragma unroll
+    for (int j = 0; j < 10; j++) ysc[j] = gr_sel(yv, n0 + gw_col(tn, j)) * xsc;
 #pragma unroll
     for (int g = 0; g < 2; g++) {  // the two 4-column groups
       const int n = n0 + g * 64 + tn * 4;
@@ -407,7 +427,8 @@ static __global__ void __launch_bounds__(GW_THREADS, 2)
 inline int launch_gemm_rows_w(cudaStream_t st, int splitCtas, float* scratch, size_t scratchElems, int nrows, int nrhs,
                               const int32_t* rows, const int32_t* chd, int xChild, int yChild, const float* X,
                               int64_t ldx, int64_t xRhs, const float* Wt, int ldw, float* Y, int64_t ldy,
-                              int64_t yRhs, int K, int N, GrScale<float> xs, GrScale<float> ys, float beta) {
+                              int64_t yRhs, int K, int N, GrScale<float> xs, GrScale<float> ys, float beta,
+                              const int32_t* rowDepth, int rootLevel) {
   if (nrows <= 0 || nrhs <= 0) return 0;
   const int64_t M = (int64_t)nrows * nrhs;
   const int tiles = (int)((M + GW_BM - 1) / GW_BM) * ((N + GW_BN - 1) / GW_BN);
@@ -423,11 +444,11 @@ inline int launch_gemm_rows_w(cudaStream_t st, int splitCtas, float* scratch, si
   dim3 grid((unsigned)((M + GW_BM - 1) / GW_BM), (N + GW_BN - 1) / GW_BN, splits);
   float* pt = splits > 1 ? scratch : nullptr;
   k_gemm_rows_w<<<grid, GW_THREADS, 0, st>>>(nrows, nrhs, rows, chd, xChild, yChild, X, ldx, xRhs, Wt, ldw, Y, ldy,
-                                             yRhs, K, N, xs, ys, beta, kChunk, pt, yVec);
+                                             yRhs, K, N, xs, ys, beta, kChunk, pt, yVec, rowDepth, rootLevel);
   if (splits == 1) return 1;
   const int64_t tot = M * N;
   k_gemm_reduce_t<float><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(nrows, nrhs, rows, chd, yChild, Y, ldy, yRhs,
-                                                                         N, splits, scratch, ys, beta);
+                                                                         N, splits, scratch, ys, beta, rowDepth, rootLevel);
   return 2;
 }
 
@@ -440,7 +461,7 @@ template <typename T, int BK>
 inline int launch_gemm_rows(cudaStream_t st, int splitCtas, T* scratch, size_t scratchElems, int nrows, int nrhs,
                             const int32_t* rows, const int32_t* chd, int xChild, int yChild, const T* X, int64_t ldx,
                             int64_t xRhs, const T* W, T* Y, int64_t ldy, int64_t yRhs, int K, int N, GrScale<T> xs,
-                            GrScale<T> ys, T beta) {
+                            GrScale<T> ys, T beta, const int32_t* rowDepth, int rootLevel) {
   if (nrows <= 0 || nrhs <= 0) return 0;
   const int64_t M = (int64_t)nrows * nrhs;
   const int tiles = (int)((M + GR_BM - 1) / GR_BM) * ((N + GR_BN - 1) / GR_BN);
@@ -459,14 +480,16 @@ inline int launch_gemm_rows(cudaStream_t st, int splitCtas, T* scratch, size_t s
   T* pt = splits > 1 ? scratch : nullptr;
   if (vec)
     k_gemm_rows_t<T, BK, true><<<grid, GR_THREADS, 0, st>>>(nrows, nrhs, rows, chd, xChild, yChild, X, ldx, xRhs, W,
-                                                             Y, ldy, yRhs, K, N, xs, ys, beta, kChunk, pt);
+                                                             Y, ldy, yRhs, K, N, xs, ys, beta, kChunk, pt,
+                                                             rowDepth, rootLevel);
   else
     k_gemm_rows_t<T, BK, false><<<grid, GR_THREADS, 0, st>>>(nrows, nrhs, rows, chd, xChild, yChild, X, ldx, xRhs, W,
-                                                              Y, ldy, yRhs, K, N, xs, ys, beta, kChunk, pt);
+                                                              Y, ldy, yRhs, K, N, xs, ys, beta, kChunk, pt,
+                                                              rowDepth, rootLevel);
   if (splits == 1) return 1;
   const int64_t tot = M * N;
   k_gemm_reduce_t<T><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(nrows, nrhs, rows, chd, yChild, Y, ldy, yRhs, N,
-                                                                     splits, scratch, ys, beta);
+                                                                     splits, scratch, ys, beta, rowDepth, rootLevel);
   return 2;
 }
 

@@ -138,13 +138,14 @@ __global__ void __launch_bounds__(T3_THREADS, 1)
                const int32_t* __restrict__ chd, int xChild, int yChild, const float* __restrict__ X, int64_t ldx,
                int64_t xRhs, float* __restrict__ Y, int64_t ldy, int64_t yRhs, int K, int N, GrScale<float> xs,
                GrScale<float> ys, float beta, int kChunk, float* __restrict__ part, int nProd,
-               int* __restrict__ errFlag) {
+               int* __restrict__ errFlag, const int32_t* __restrict__ rowDepth, int rootLevel) {
   using C = T3Cfg<BN>;
   static_assert(T3_NACC * BN <= 512 && BN % 32 == 0, "the block accumulators fit 512 TMEM columns");
   static_assert(T3_DWARPS == 8, "two drain warps per TMEM lane group, half the columns each");
   extern __shared__ unsigned char t3_smem_raw[];
   __shared__ const float* xrow[T3_BM];
   __shared__ float* yrow[T3_BM];
+  __shared__ int ylev[T3_BM];
   __shared__ __align__(8) uint64_t fullA[T3_STAGES], fullB[T3_STAGES], empty[T3_STAGES], accFull[T3_NACC],
       accEmpty[T3_NACC];
   __shared__ uint32_t tmemSlot;
@@ -162,6 +163,7 @@ __global__ void __launch_bounds__(T3_THREADS, 1)
       const int node = rows[r - (int64_t)q * nrows];
       xrow[tid] = X + q * xRhs + (int64_t)(xChild ? chd[node] : node) * ldx;
       yrow[tid] = Y + q * yRhs + (int64_t)(yChild ? chd[node] : node) * ldy;
+      ylev[tid] = rowDepth ? rowDepth[node] + rootLevel : 0;
     } else {
       xrow[tid] = nullptr;
       yrow[tid] = nullptr;
@@ -374,6 +376,7 @@ __global__ void __launch_bounds__(T3_THREADS, 1)
     const int half = (warp - T3_DWARP0) / 4;
     float* yr = yrow[m];
     const bool vecY = ((uintptr_t)yr % 16 == 0);
+    const GrScale<float> yv = gr_row_scale(ys, yr ? rowDepth : nullptr, yr ? ylev[m] : 0);
 #pragma unroll
     for (int cb = 0; cb < BN / 32; cb++) {
       const int nb = n0 + half * (BN / 2) + cb * 16;
@@ -387,7 +390,7 @@ __global__ void __launch_bounds__(T3_THREADS, 1)
       } else if (yr) {
         float a[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++) a[j] = R[cb * 16 + j] * gr_sel(ys, nb + j);
+        for (int j = 0; j < 16; j++) a[j] = R[cb * 16 + j] * gr_sel(yv, nb + j);
         if (vecY && nb + 16 <= N) {
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
@@ -448,30 +451,6 @@ __global__ void __launch_bounds__(TC_THREADS) k_wait_selftest(int arrive, long l
 
 constexpr int T3_BN = 160;  // covers the 152-wide surfaces of np = 6 in one tile
 
-// round to nearest TF32 (ties away from zero), as cvt.rna.tf32.f32
-inline float host_rna_tf32(float x) {
-  uint32_t u;
-  std::memcpy(&u, &x, 4);
-  if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0x1000u) & 0xffffe000u;
-  float r;
-  std::memcpy(&r, &u, 4);
-  return r;
-}
-
-// The hi / lo parts of W (from FP64) in the padded stacked layout.
-inline std::vector<float> tc_split_operator(const std::vector<double>& W, int n, int k, int nPad, int kPad) {
-  std::vector<float> t((size_t)2 * nPad * kPad, 0.f);
-  for (int i = 0; i < n; i++)
-    for (int j = 0; j < k; j++) {
-      const double w = W[(size_t)i * k + j];
-      const float hi = host_rna_tf32((float)w);
-      const float lo = host_rna_tf32((float)(w - (double)hi));
-      t[(size_t)i * kPad + j] = hi;
-      t[(size_t)(nPad + i) * kPad + j] = lo;
-    }
-  return t;
-}
-
 // The TMA tensor map of a TcOp: box 32 K values x T3_BN rows, 128-byte swizzle.
 inline std::string tc_encode_map(TcOp& op) {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
@@ -493,23 +472,64 @@ inline std::string tc_encode_map(TcOp& op) {
   return std::string();
 }
 
-// Uploads W (n x k, FP64 row-major) as a TcOp; `alloc(float*&, size_t)`
-// returns device memory that lives as long as the handle.
-template <typename Alloc>
-inline std::string tc_prepare_operator(TcOp& op, const std::vector<double>& W, int n, int k, Alloc alloc) {
+// One operator W (n x k, FP64 row-major, on the device) in the three forms of
+// the FP32 row GEMMs: plain (n x k), wt (transposed, zero padded to kp x ld) and
+// tc (hi rows then lo rows of nPad x kPad, both parts rounded to nearest TF32).
+static __global__ void k_pack_operator(const double* __restrict__ W, int n, int k, float* __restrict__ plain,
+                                       float* __restrict__ wt, int kp, int ld, float* __restrict__ tc, int nPad,
+                                       int kPad) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < (int64_t)n * k) plain[i] = (float)W[i];
+  if (i < (int64_t)kp * ld) {
+    const int r = (int)(i / ld), c = (int)(i % ld);
+    wt[i] = r < k && c < n ? (float)W[(int64_t)c * k + r] : 0.f;
+  }
+  if (i < (int64_t)nPad * kPad) {
+    const int r = (int)(i / kPad), c = (int)(i % kPad);
+    float hi = 0.f, lo = 0.f;
+    if (r < n && c < k) {
+      const double w = W[(int64_t)r * k + c];
+      const float f = (float)w;
+      hi = isfinite(f) ? tc_rna(f) : f;
+      const float d = (float)(w - (double)hi);
+      lo = isfinite(d) ? tc_rna(d) : d;
+    }
+    tc[i] = hi;
+    tc[(int64_t)nPad * kPad + i] = lo;
+  }
+}
+
+// Lays W (n x k, on the device) out as a TcOp and as the CUDA-core kernels'
+// plain and wt forms; `alloc(float*&, size_t)` returns device memory that lives
+// as long as the handle's tables.  On the device: the host's three passes over
+// the operators took half of the first mixed call of a Navier np = 8 handle (312 -> 150 ms).
+template <typename OpT, typename Alloc>
+inline std::string prepare_operator(cudaStream_t st, TcOp& op, OpT& wt, float* plain, const double* dW, int n, int k,
+                                    Alloc alloc) {
   op.ready = false;
   op.n = n;
   op.k = k;
   op.nPad = (n + T3_BN - 1) / T3_BN * T3_BN;
   op.kPad = (k + T3_BK - 1) / T3_BK * T3_BK;
-  const std::vector<float> t = tc_split_operator(W, n, k, op.nPad, op.kPad);
-  if (!op.p || t.size() > op.cap) {
-    std::string e = alloc(op.p, t.size());
+  const size_t size = (size_t)2 * op.nPad * op.kPad;
+  if (!op.p || size > op.cap) {
+    std::string e = alloc(op.p, size);
     if (!e.empty()) return e;
-    op.cap = t.size();
+    op.cap = size;
   }
-  cudaError_t ce = cudaMemcpy(op.p, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice);
-  if (ce != cudaSuccess) return std::string("operator upload: ") + cudaGetErrorString(ce);
+  const int kp = (k + GW_BK - 1) / GW_BK * GW_BK;
+  wt.ld = (n + GW_BN - 1) / GW_BN * GW_BN;
+  if (!wt.p || (size_t)kp * wt.ld > wt.cap) {
+    std::string e = alloc(wt.p, (size_t)kp * wt.ld);
+    if (!e.empty()) return e;
+    wt.cap = (size_t)kp * wt.ld;
+  }
+  const int64_t m = std::max<int64_t>(std::max<int64_t>((int64_t)n * k, (int64_t)kp * wt.ld),
+                                      (int64_t)op.nPad * op.kPad);
+  k_pack_operator<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(dW, n, k, plain, wt.p, kp, wt.ld, op.p, op.nPad,
+                                                               op.kPad);
+  cudaError_t ce = cudaGetLastError();
+  if (ce != cudaSuccess) return std::string("operator layout: ") + cudaGetErrorString(ce);
   std::string e = tc_encode_map(op);
   op.ready = e.empty();
   return e;
@@ -529,7 +549,8 @@ inline bool tc_usable(const TcOp* op, const float* X, int64_t ldx, int64_t xRhs,
 inline int launch_gemm_tc3(cudaStream_t st, int splitCtas, float* scratch, size_t scratchElems, const TcOp& op,
                            int nProd, int* errFlag, int nrows, int nrhs, const int32_t* rows, const int32_t* chd,
                            int xChild, int yChild, const float* X, int64_t ldx, int64_t xRhs, float* Y, int64_t ldy,
-                           int64_t yRhs, int K, int N, GrScale<float> xs, GrScale<float> ys, float beta) {
+                           int64_t yRhs, int K, int N, GrScale<float> xs, GrScale<float> ys, float beta,
+                           const int32_t* rowDepth, int rootLevel) {
   if (nrows <= 0 || nrhs <= 0) return 0;
   const int64_t M = (int64_t)nrows * nrhs;
   const int tiles = (int)((M + T3_BM - 1) / T3_BM) * ((N + T3_BN - 1) / T3_BN);
@@ -550,11 +571,13 @@ inline int launch_gemm_tc3(cudaStream_t st, int splitCtas, float* scratch, size_
   float* pt = splits > 1 ? scratch : nullptr;
   k_gemm_tc3<T3_BN><<<grid, T3_THREADS, T3Cfg<T3_BN>::SMEM, st>>>(op.map, op.nPad, nrows, nrhs, rows, chd, xChild,
                                                                    yChild, X, ldx, xRhs, Y, ldy, yRhs, K, N, xs, ys,
-                                                                   beta, kChunk, pt, nProd, errFlag);
+                                                                   beta, kChunk, pt, nProd, errFlag, rowDepth,
+                                                                   rootLevel);
   if (splits == 1) return 1;
   const int64_t tot = M * N;
   k_gemm_reduce_t<float><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(nrows, nrhs, rows, chd, yChild, Y, ldy, yRhs,
-                                                                         N, splits, scratch, ys, beta);
+                                                                         N, splits, scratch, ys, beta, rowDepth,
+                                                                         rootLevel);
   return 2;
 }
 
@@ -566,17 +589,18 @@ inline int launch_gemm_rows_f32(cudaStream_t st, int splitCtas, float* scratch, 
                                 int nProd, int* errFlag, int nrows, int nrhs, const int32_t* rows, const int32_t* chd,
                                 int xChild, int yChild, const float* X, int64_t ldx, int64_t xRhs, const float* W,
                                 const float* Wt, int ldw, float* Y, int64_t ldy, int64_t yRhs, int K, int N,
-                                GrScale<float> xs, GrScale<float> ys, float beta) {
+                                GrScale<float> xs, GrScale<float> ys, float beta, const int32_t* rowDepth,
+                                int rootLevel) {
   if (nrows <= 0 || nrhs <= 0) return 0;
   if (errFlag && tc_usable(tc, X, ldx, xRhs, K, N))
     return launch_gemm_tc3(st, splitCtas, scratch, scratchElems, *tc, nProd, errFlag, nrows, nrhs, rows, chd, xChild,
-                           yChild, X, ldx, xRhs, Y, ldy, yRhs, K, N, xs, ys, beta);
+                           yChild, X, ldx, xRhs, Y, ldy, yRhs, K, N, xs, ys, beta, rowDepth, rootLevel);
   const bool xvec = ((uintptr_t)X % 16 == 0) && ldx % 4 == 0 && xRhs % 4 == 0 && K % 4 == 0;
   if (Wt && xvec && ((uintptr_t)Wt % 16 == 0) && ldw % GW_BN == 0)
     return launch_gemm_rows_w(st, splitCtas, scratch, scratchElems, nrows, nrhs, rows, chd, xChild, yChild, X, ldx,
-                              xRhs, Wt, ldw, Y, ldy, yRhs, K, N, xs, ys, beta);
+                              xRhs, Wt, ldw, Y, ldy, yRhs, K, N, xs, ys, beta, rowDepth, rootLevel);
   return launch_gemm_rows<float, 16>(st, splitCtas, scratch, scratchElems, nrows, nrhs, rows, chd, xChild, yChild, X,
-                                     ldx, xRhs, W, Y, ldy, yRhs, K, N, xs, ys, beta);
+                                     ldx, xRhs, W, Y, ldy, yRhs, K, N, xs, ys, beta, rowDepth, rootLevel);
 }
 
 }  // namespace fmmg

@@ -30,6 +30,7 @@
 #include "had_smem.cuh"
 #include "had_vec.cuh"
 #include "kernels.hpp"
+#include "plan_pool.cuh"
 
 namespace fmmg {
 
@@ -1220,15 +1221,40 @@ static std::vector<double> pad_cols(const std::vector<double>& F, int m, int k) 
   return r;
 }
 
-// W row-major n x k -> Wt[k][n] in FP32, K padded to a multiple of GW_BK and N
-// to a multiple of GW_BN (ld) with zeros: the wide-tile GEMM reads whole tiles
-static std::vector<float> transpose_pad(const std::vector<double>& W, int n, int k, int& ld) {
-  const int kp = (k + GW_BK - 1) / GW_BK * GW_BK;
-  ld = (n + GW_BN - 1) / GW_BN * GW_BN;
-  std::vector<float> t((size_t)kp * ld, 0.f);
-  for (int i = 0; i < n; i++)
-    for (int j = 0; j < k; j++) t[(size_t)j * ld + i] = (float)W[(size_t)i * k + j];
-  return t;
+// t[o][j][c] = l2l[(o dc + c) de + j]: the transposes of L2L's 8 octant blocks
+static __global__ void k_l2l_blocks_t(int64_t n, int dc, int de, const double* __restrict__ l2l,
+                                      double* __restrict__ t) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int c = (int)(i % dc), j = (int)(i / dc % de);
+  const int64_t o = i / ((int64_t)dc * de);
+  t[i] = l2l[(o * dc + c) * de + j];
+}
+static __global__ void k_iota(int n, int32_t* p) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) p[i] = i;
+}
+
+// A child's downward density is the pseudo-inverse of its whole check
+// potential, V and X lists' part and the parent's (L2L) part; by linearity the
+// first is applied to all nodes at once and the second becomes one product per
+// level, G = C2E x L2L (8 de x de, formed here in FP64).  As for the upward
+// fold the product's norm is O(1) where the pseudo-inverse's is ~1e6, so it
+// loses nothing in FP32 (the L2L part no longer passes the inverse in FP32).
+static std::string dn_fold(const Plan& P, DevState& D, double* G, PlanBufs& tmp) {
+  const int de = P.nDE * P.sdm, dc = P.nDC * P.tdm;
+  double* lt = nullptr;
+  int32_t* iota = nullptr;
+  FMMG_CK(tmp.get(lt, (size_t)8 * de * dc));
+  FMMG_CK(tmp.get(iota, (size_t)de));
+  const int64_t n = (int64_t)8 * de * dc;
+  k_l2l_blocks_t<<<(unsigned)((n + 255) / 256), 256, 0, D.stream>>>(n, dc, de, D.l2l, lt);
+  k_iota<<<(de + 255) / 256, 256, 0, D.stream>>>(de, iota);
+  for (int o = 0; o < 8; o++)  // rows of the inverse times the block's columns
+    gemm_rows(D, de, iota, nullptr, 0, 0, D.dc2de, dc, lt + (size_t)o * de * dc, G + (size_t)o * de * de, de, dc, de,
+              unit_scale(), unit_scale(), 0.0, nullptr);
+  FMMG_CK(cudaGetLastError());
+  return std::string();
 }
 
 // Work arrays for a chunk of kc right-hand sides, and the FP32 operator copies.
@@ -1293,6 +1319,9 @@ static std::string hv_layout32(const Plan& P, DevState& D) {
   return std::string();
 }
 
+// Uploads go through the handle's stream: a cudaMemcpy from pageable memory
+// returns once the data is staged, and a stream created non-blocking does not
+// wait for the legacy stream's copy.
 static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
   const size_t ue = (size_t)P.nUE * P.sdm, uc = (size_t)P.nUC * P.tdm;
   const size_t de = (size_t)P.nDE * P.sdm, dc = (size_t)P.nDC * P.tdm;
@@ -1308,19 +1337,19 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     for (size_t r = 0; r < nl; r++) order[r] = (int32_t)r;
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return cost[a] > cost[b]; });
     FMMG_TRY(dalloc(D, D.nearOrder, nl));
-    FMMG_CK(cudaMemcpy(D.nearOrder, order.data(), nl * sizeof(int32_t), cudaMemcpyHostToDevice));
+    FMMG_CK(cudaMemcpyAsync(D.nearOrder, order.data(), nl * sizeof(int32_t), cudaMemcpyHostToDevice, D.stream));
   }
   if (!D.m2tItems && !P.farLeaves.empty()) {
     std::vector<int4> items;
     std::vector<int32_t> sl, sb, sc;
     m2t_items(P, D.numSMs, items, sl, sb, sc, D.m2tPartTargets);
     FMMG_TRY(dalloc(D, D.m2tItems, items.size()));
-    FMMG_CK(cudaMemcpy(D.m2tItems, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    FMMG_CK(cudaMemcpyAsync(D.m2tItems, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, D.stream));
     D.nM2tItems = (int)items.size();
     D.nM2tSplit = (int)sl.size();
     auto put = [&](int32_t*& dst, const std::vector<int32_t>& v) -> std::string {
       FMMG_TRY(dalloc(D, dst, v.size()));
-      FMMG_CK(cudaMemcpy(dst, v.data(), v.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+      FMMG_CK(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(int32_t), cudaMemcpyHostToDevice, D.stream));
       return std::string();
     };
     if (!sl.empty()) {
@@ -1341,6 +1370,9 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     FMMG_CK(cudaMemsetAsync(D.uden32, 0, sizeof(float) * kc * P.nn * ue, D.stream));
     FMMG_TRY(dalloc(D, D.dchk32, (size_t)kc * P.nn * dc));
     FMMG_TRY(dalloc(D, D.dden32, (size_t)kc * P.nn * de));
+    // the children without targets of a parent with some: its folded product
+    // adds to their rows, which nothing assigns or reads
+    FMMG_CK(cudaMemsetAsync(D.dden32, 0, sizeof(float) * kc * P.nn * de, D.stream));
     const size_t kc8 = (size_t)(kc + 7) / 8 * 8;  // the scalar k >= 2 layout stores blocks of 8
     FMMG_TRY(dalloc(D, D.effDen32, kc8 * P.vSrcNodes.size() * P.nEff32 * P.sdm));
     FMMG_TRY(dalloc(D, D.effVal32, kc8 * P.vTrgNodes.size() * P.nEff32 * P.tdm));
@@ -1350,9 +1382,9 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     FMMG_TRY(dalloc(D, D.den32, kc8 * P.ns * P.sd));
     FMMG_TRY(dalloc(D, D.valK, (size_t)kc * std::max<int64_t>(P.nt, 1) * P.td));
     FMMG_TRY(dalloc(D, D.m2tPart, (size_t)kc * std::max<int64_t>(D.m2tPartTargets, 1) * P.tdm));
-    if (!D.l2l32) {
+    if (!D.dnFold32) {
       OpBlocks scope(D);
-      FMMG_TRY(dalloc(D, D.l2l32, P.l2l.size()));
+      FMMG_TRY(dalloc(D, D.dnFold32, 8 * de * de));
       FMMG_TRY(dalloc(D, D.m2lT32, P.m2lT32.size()));
       if (P.sdm == 1 && P.tdm == 1) FMMG_TRY(dalloc(D, D.m2lTw32, (size_t)27 * 27 * P.nEff32));
       FMMG_TRY(dalloc(D, D.upF1, (size_t)kUpMax * uc));
@@ -1366,54 +1398,39 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
   }
   if (D.mixedOpsStale) {
     OpBlocks scope(D);
-    auto put = [&](float* dst, const std::vector<double>& v) -> std::string {
-      std::vector<float> f(v.begin(), v.end());
-      FMMG_CK(cudaMemcpy(dst, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
-      return std::string();
-    };
-    FMMG_TRY(put(D.l2l32, P.l2l));
-    // the factors padded to a rank that is a multiple of 4 (zero rows of F1,
-    // zero columns of F2), so the intermediate rows allow 16-byte tile fetches
-    FMMG_TRY(put(D.upF1, pad_rows(P.uc2ueF1, P.kUp, (int)uc)));
-    FMMG_TRY(put(D.upF2, pad_cols(P.uc2ueF2, (int)ue, P.kUp)));
-    FMMG_TRY(put(D.dnF1, pad_rows(P.dc2deF1, P.kDn, (int)dc)));
-    FMMG_TRY(put(D.dnF2, pad_cols(P.dc2deF2, (int)de, P.kDn)));
-    // the same operators transposed and padded for the wide-tile GEMM
-    auto putT = [&](DevState::OpT& op, const std::vector<double>& W, int n, int k) -> std::string {
-      int ld = 0;
-      const std::vector<float> t = transpose_pad(W, n, k, ld);
-      if (!op.p || t.size() > op.cap) {
-        FMMG_TRY(dalloc(D, op.p, t.size()));
-        op.cap = t.size();
-      }
-      op.ld = ld;
-      FMMG_CK(cudaMemcpy(op.p, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice));
-      return std::string();
+    // the operators from FP64 tables on the device; the factors padded to a
+    // rank that is a multiple of 4 (zero rows of F1, zero columns of F2), so the
+    // intermediate rows allow 16-byte tile fetches
+    auto alloc = [&](float*& p, size_t n) { return dalloc(D, p, n); };
+    PlanBufs tmp;
+    tmp.device = D.device;
+    auto prep = [&](TcOp& op, DevState::OpT& wt, float* plain, const std::vector<double>& W, int n,
+                    int k) -> std::string {
+      double* dW = nullptr;
+      FMMG_CK(tmp.get(dW, W.size()));
+      FMMG_CK(cudaMemcpyAsync(dW, W.data(), W.size() * sizeof(double), cudaMemcpyHostToDevice, D.stream));
+      return prepare_operator(D.stream, op, wt, plain, dW, n, k, alloc);
     };
     const int kUp4 = pad4(P.kUp), kDn4 = pad4(P.kDn);
-    FMMG_TRY(putT(D.tL2L, P.l2l, (int)(8 * dc), (int)de));
-    FMMG_TRY(putT(D.tUpF1, pad_rows(P.uc2ueF1, P.kUp, (int)uc), kUp4, (int)uc));
-    FMMG_TRY(putT(D.tUpF2, pad_cols(P.uc2ueF2, (int)ue, P.kUp), (int)ue, kUp4));
-    FMMG_TRY(putT(D.tDnF1, pad_rows(P.dc2deF1, P.kDn, (int)dc), kDn4, (int)dc));
-    FMMG_TRY(putT(D.tDnF2, pad_cols(P.dc2deF2, (int)de, P.kDn), (int)de, kDn4));
+    FMMG_TRY(prep(D.cUpF1, D.tUpF1, D.upF1, pad_rows(P.uc2ueF1, P.kUp, (int)uc), kUp4, (int)uc));
+    FMMG_TRY(prep(D.cUpF2, D.tUpF2, D.upF2, pad_cols(P.uc2ueF2, (int)ue, P.kUp), (int)ue, kUp4));
+    FMMG_TRY(prep(D.cDnF1, D.tDnF1, D.dnF1, pad_rows(P.dc2deF1, P.kDn, (int)dc), kDn4, (int)dc));
+    FMMG_TRY(prep(D.cDnF2, D.tDnF2, D.dnF2, pad_cols(P.dc2deF2, (int)de, P.kDn), (int)de, kDn4));
     // a parent's upward density straight from its children's: C2E up x M2M
     const std::vector<double>& fold = [&]() -> const std::vector<double>& {
       LinalgDeviceScope scope(D.device);  // formed on this GPU on first use (the host's sums, bit for bit)
       return P.folded_upward();
     }();
-    FMMG_TRY(put(D.m2mUp32, fold));
-    FMMG_TRY(putT(D.tM2MUp, fold, (int)ue, (int)(8 * ue)));
-    // the same six operators split into TF32 hi / lo parts for the tensor cores
-    auto tcAlloc = [&](float*& p, size_t n) { return dalloc(D, p, n); };
-    FMMG_TRY(tc_prepare_operator(D.cL2L, P.l2l, (int)(8 * dc), (int)de, tcAlloc));
-    FMMG_TRY(tc_prepare_operator(D.cUpF1, pad_rows(P.uc2ueF1, P.kUp, (int)uc), kUp4, (int)uc, tcAlloc));
-    FMMG_TRY(tc_prepare_operator(D.cUpF2, pad_cols(P.uc2ueF2, (int)ue, P.kUp), (int)ue, kUp4, tcAlloc));
-    FMMG_TRY(tc_prepare_operator(D.cDnF1, pad_rows(P.dc2deF1, P.kDn, (int)dc), kDn4, (int)dc, tcAlloc));
-    FMMG_TRY(tc_prepare_operator(D.cDnF2, pad_cols(P.dc2deF2, (int)de, P.kDn), (int)de, kDn4, tcAlloc));
-    FMMG_TRY(tc_prepare_operator(D.cM2MUp, fold, (int)ue, (int)(8 * ue), tcAlloc));
+    FMMG_TRY(prep(D.cM2MUp, D.tM2MUp, D.m2mUp32, fold, (int)ue, (int)(8 * ue)));
+    // the parent's part of a child's downward density: C2E down x L2L
+    double* G = nullptr;
+    FMMG_CK(tmp.get(G, 8 * de * de));
+    FMMG_TRY(dn_fold(P, D, G, tmp));
+    FMMG_TRY(prepare_operator(D.stream, D.cDnFold, D.tDnFold, D.dnFold32, G, (int)(8 * de), (int)de, alloc));
+    FMMG_CK(cudaStreamSynchronize(D.stream));  // tmp's blocks go back to the pool
     std::vector<float2> t(P.m2lT32.size());
     for (size_t i = 0; i < t.size(); i++) t[i] = make_float2((float)P.m2lT32[i].real(), (float)P.m2lT32[i].imag());
-    FMMG_CK(cudaMemcpy(D.m2lT32, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    FMMG_CK(cudaMemcpyAsync(D.m2lT32, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice, D.stream));
     if (P.sdm == 4) FMMG_TRY((hv_layout32<4, 3>(P, D)));
     else if (P.sdm == 3) FMMG_TRY((hv_layout32<3, 3>(P, D)));
     if (D.m2lTw32) {  // combined translations of the 27-product Hadamard (had_pq.cuh), FP64 sums
@@ -1445,7 +1462,7 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
           for (int f = 0; f < ne; f++) dst[f] = make_float2((float)acc[f].real(), (float)acc[f].imag());
         }
       }
-      FMMG_CK(cudaMemcpy(D.m2lTw32, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice));
+      FMMG_CK(cudaMemcpyAsync(D.m2lTw32, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, D.stream));
     }
     D.mixedOpsStale = false;
   }
@@ -1472,13 +1489,13 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
   // path is on and the class is in the tuning mask (the wide CUDA-core tiles
   // otherwise)
   auto useTc = [&](const TcOp& tc) {
-    const int cls = &tc == &D.cUpF1 ? 0 : &tc == &D.cUpF2 ? 1 : &tc == &D.cM2MUp ? 2 : &tc == &D.cL2L ? 3
+    const int cls = &tc == &D.cUpF1 ? 0 : &tc == &D.cUpF2 ? 1 : &tc == &D.cM2MUp ? 2 : &tc == &D.cDnFold ? 3
                     : &tc == &D.cDnF1 ? 4 : 5;
     return D.gemmPath == 1 && ((D.tune.tcMask >> cls) & 1);
   };
   auto gemm = [&](int nrows, const int32_t* rows, int xChild, int yChild, const float* X, int64_t ldx, int64_t xR,
                   const float* W, const DevState::OpT& wt, float* Y, int64_t ldy, int64_t yR, int K, int N, Scale4 xs,
-                  Scale4 ys, float beta, const TcOp& tc) {
+                  Scale4 ys, float beta, const TcOp& tc, const int32_t* rowDepth = nullptr) {
     if (nrows <= 0) return;
     GrScale<float> gx, gy;
     gx.mod = xs.mod;
@@ -1491,8 +1508,11 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
                                          D.gemmScratchBytes / sizeof(float), useTc(tc) ? &tc : nullptr,
                                          D.tune.tcProducts, D.devErr, nrows,
                                          kc, rows, D.chd, xChild, yChild, X, ldx, xR, W,
-                                         D.gemmPath == 2 ? nullptr : wt.p, wt.ld, Y, ldy, yR, K, N, gx, gy, beta);
+                                         D.gemmPath == 2 ? nullptr : wt.p, wt.ld, Y, ldy, yR, K, N, gx, gy, beta, rowDepth, rl);
   };
+  Scale4 degrees;  // the Y scale of rows of several levels
+  degrees.mod = P.sdm;
+  for (int k = 0; k < 4; k++) degrees.v[k] = k < P.sdm ? P.deg[k] : 0.0;
   const bool ovl = overlap && D.side;
   if (ovl) {  // fork: the densities are gathered and the target values cleared
     cudaEventRecord(D.evFork, st);
@@ -1507,20 +1527,20 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
   }
   cudaEventRecord(D.ev[EV_S2M], st);
   if (mask & 1) {
-    for (int d = P.maxDepth; d >= 1; d--) {
-      // leaves with sources: C2E as F2 (F1 uchk), so the large-norm pinv
-      // never multiplies in FP32
-      int64_t a = D.offUpLeaf[d], b = D.offUpLeaf[d + 1];
-      gemm((int)(b - a), D.levelRows + a, 0, 0, D.uchk32, uc, nn * uc, D.upF1, D.tUpF1, D.upT32, kUp4, nn * kUp4, uc,
-           kUp4, unit_scale(), unit_scale(), 0.f, D.cUpF1);
-      gemm((int)(b - a), D.levelRows + a, 0, 0, D.upT32, kUp4, nn * kUp4, D.upF2, D.tUpF2, D.uden32, ue, nn * ue, kUp4,
-           ue, unit_scale(), level_scale(P, d + rl, -1.0), 0.f, D.cUpF2);
-      // parents: C2E up x M2M folded on the host in FP64 (its norm is O(1)
-      // where the pinv's is ~1e6), one product from the children's upward
-      // densities (depth d + 1, done in the previous iteration) with no check
-      // surface in between
-      a = D.offUpM2M[d];
-      b = D.offUpM2M[d + 1];
+    // leaves with sources, of all levels at once: C2E as F2 (F1 uchk), so the
+    // large-norm pinv never multiplies in FP32
+    const int64_t l0 = D.offUpLeaf[std::min(2, P.maxDepth + 1)], l1 = D.offUpLeaf[P.maxDepth + 1];
+    gemm((int)(l1 - l0), D.levelRows + l0, 0, 0, D.uchk32, uc, nn * uc, D.upF1, D.tUpF1, D.upT32, kUp4, nn * kUp4, uc,
+         kUp4, unit_scale(), unit_scale(), 0.f, D.cUpF1);
+    gemm((int)(l1 - l0), D.levelRows + l0, 0, 0, D.upT32, kUp4, nn * kUp4, D.upF2, D.tUpF2, D.uden32, ue, nn * ue,
+         kUp4, ue, unit_scale(), degrees, 0.f, D.cUpF2, D.depth);
+    // parents, down to depth 2 (nothing reads the densities of depth 1, see
+    // run_stages): C2E up x M2M folded on the host in FP64 (its norm is O(1)
+    // where the pinv's is ~1e6), one product from the children's upward
+    // densities (depth d + 1, done in the previous iteration) with no check
+    // surface in between
+    for (int d = P.maxDepth - 1; d >= 2; d--) {
+      const int64_t a = D.offUpM2M[d], b = D.offUpM2M[d + 1];
       gemm((int)(b - a), D.levelRows + a, 1, 0, D.uden32, ue, nn * ue, D.m2mUp32, D.tM2MUp, D.uden32, ue, nn * ue,
            8 * ue, ue, level_scale(P, d + 1 + rl, +1.0), level_scale(P, d + rl, -1.0), 0.f, D.cM2MUp);
     }
@@ -1745,17 +1765,17 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
   }
   cudaEventRecord(D.ev[EV_S2L], st);
   if (mask & 32) {
-    for (int d = 2; d <= P.maxDepth; d++) {
-      if (d >= 3) {
-        int64_t a = D.offDnL2L[d - 1], b = D.offDnL2L[d];
-        gemm((int)(b - a), D.levelRows + a, 0, 1, D.dden32, de, nn * de, D.l2l32, D.tL2L, D.dchk32, dc, nn * dc, de, 8 * dc,
-             level_scale(P, d - 1 + rl, +1.0), unit_scale(), 1.f, D.cL2L);
-      }
-      int64_t a = D.offDnC2E[d], b = D.offDnC2E[d + 1];
-      gemm((int)(b - a), D.levelRows + a, 0, 0, D.dchk32, dc, nn * dc, D.dnF1, D.tDnF1, D.dnT32, kDn4, nn * kDn4, dc,
-           kDn4, unit_scale(), unit_scale(), 0.f, D.cDnF1);
-      gemm((int)(b - a), D.levelRows + a, 0, 0, D.dnT32, kDn4, nn * kDn4, D.dnF2, D.tDnF2, D.dden32, de, nn * de, kDn4,
-           de, unit_scale(), level_scale(P, d + rl, -1.0), 0.f, D.cDnF2);
+    // C2E of every node's own check potential, all levels at once, then the
+    // parents' densities down the levels through the folded product (dn_fold)
+    const int64_t n0 = D.offDnC2E[std::min(2, P.maxDepth + 1)], n1 = D.offDnC2E[P.maxDepth + 1];
+    gemm((int)(n1 - n0), D.levelRows + n0, 0, 0, D.dchk32, dc, nn * dc, D.dnF1, D.tDnF1, D.dnT32, kDn4, nn * kDn4, dc,
+         kDn4, unit_scale(), unit_scale(), 0.f, D.cDnF1);
+    gemm((int)(n1 - n0), D.levelRows + n0, 0, 0, D.dnT32, kDn4, nn * kDn4, D.dnF2, D.tDnF2, D.dden32, de, nn * de,
+         kDn4, de, unit_scale(), degrees, 0.f, D.cDnF2, D.depth);
+    for (int d = 3; d <= P.maxDepth; d++) {
+      const int64_t a = D.offDnL2L[d - 1], b = D.offDnL2L[d];
+      gemm((int)(b - a), D.levelRows + a, 0, 1, D.dden32, de, nn * de, D.dnFold32, D.tDnFold, D.dden32, de, nn * de,
+           de, 8 * de, level_scale(P, d - 1 + rl, +1.0), level_scale(P, d + rl, -1.0), 1.f, D.cDnFold);
     }
   }
   cudaEventRecord(D.ev[EV_DN_GEMM], st);

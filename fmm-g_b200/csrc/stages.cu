@@ -621,11 +621,11 @@ void dev_free(DevState& D) {
 static void dev_clear_ops(DevState& D) {
   D.uc2ue = D.m2m = D.dc2de = D.l2l = nullptr;
   D.m2lT = nullptr;
-  D.l2l32 = nullptr;
+  D.dnFold32 = nullptr;
   D.upF1 = D.upF2 = D.dnF1 = D.dnF2 = nullptr;
   D.m2mUp32 = nullptr;
-  for (DevState::OpT* op : {&D.tL2L, &D.tUpF1, &D.tUpF2, &D.tDnF1, &D.tDnF2, &D.tM2MUp}) *op = DevState::OpT();
-  for (TcOp* op : {&D.cL2L, &D.cUpF1, &D.cUpF2, &D.cDnF1, &D.cDnF2, &D.cM2MUp}) *op = TcOp();  // memory freed above
+  for (DevState::OpT* op : {&D.tDnFold, &D.tUpF1, &D.tUpF2, &D.tDnF1, &D.tDnF2, &D.tM2MUp}) *op = DevState::OpT();
+  for (TcOp* op : {&D.cDnFold, &D.cUpF1, &D.cUpF2, &D.cDnF1, &D.cDnF2, &D.cM2MUp}) *op = TcOp();  // memory freed above
   D.transIdDev = nullptr;
   D.hvT = nullptr;
   D.hvT32 = nullptr;
@@ -731,6 +731,7 @@ std::string dev_upload_operators(const Plan& P, DevState& D) {
   D.mixedOpsStale = true;
   D.adjOpsStale = true;
   D.opsHeld = true;
+  FMMG_CK(cudaStreamSynchronize(0));  // see dev_upload
   return std::string();
 }
 
@@ -742,6 +743,7 @@ std::string dev_upload_vlists(const Plan& P, DevState& D) {
   FMMG_TRY(dput(D, D.vTrgEnt, P.vTrgEnt));
   FMMG_TRY(dput(D, D.vSrcPtr, P.vSrcPtr));
   FMMG_TRY(dput(D, D.vSrcEnt, P.vSrcEnt));
+  FMMG_CK(cudaStreamSynchronize(0));  // see dev_upload
   D.vListsReady = true;
   return std::string();
 }
@@ -925,6 +927,9 @@ std::string dev_upload(const Plan& P, DevState& D, const double* src, const doub
     for (cudaEvent_t* e : {&D.evFork, &D.evUp, &D.evSide}) FMMG_CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     D.evReady = true;
   }
+  // a copy from pageable memory returns when it is staged; the handle's stream
+  // does not wait for the legacy stream's copies
+  FMMG_CK(cudaStreamSynchronize(0));
   lap(3);
   return std::string();
 }

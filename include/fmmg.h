@@ -271,7 +271,7 @@ fmmg_status fmmg_autotune(fmmg_handle* h, int k, int precision, const double* d_
  * or 2 right-hand sides a thread; 3, 4: 8 output-child accumulators, 2 or 4
  * right-hand sides a thread; default 4); with n >= 5, vals[4] = the FP32 GEMM
  * classes on the tensor cores when path 1 is on (bit 0 leaf C2E F1, 1 leaf
- * C2E F2, 2 folded C2E x M2M, 3 L2L, 4 downward C2E F1, 5 downward C2E F2;
+ * C2E F2, 2 folded C2E x M2M, 3 folded C2E x L2L, 4 downward C2E F1, 5 downward C2E F2;
  * default 63); with n >= 6, vals[5] = the products of the 3xTF32 split (3, or
  * 4 with lo*lo).  set != 0 installs them (FMMG_INVALID_ARG for values out of
  * range), else reads. */
