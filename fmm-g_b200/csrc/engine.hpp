@@ -86,7 +86,6 @@ struct DevState {
   float *upT32 = nullptr, *dnT32 = nullptr;  // [k][nn][kUp|kDn] intermediate of the factored C2E
   float2* m2lT32 = nullptr;
   float2* m2lTw32 = nullptr;  // combined translations of the 27-product Hadamard [27][27][nEff] (scalar kernels)
-  bool hadW = true;           // FP32 k >= 2 Hadamard in the 27-product form
   double *denK = nullptr, *valK = nullptr;  // permuted densities / values of a RHS chunk
   float* den32 = nullptr;  // the chunk's densities in FP32, [rhs / 8][n][8][sd] (what the pair kernels stage)
   bool mixedReady = false, mixedOpsStale = true;

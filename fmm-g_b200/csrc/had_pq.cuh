@@ -1,7 +1,7 @@
 // had_pq.cuh -- the M2L Hadamard step for scalar equivalent kernels, grouped
 // by parent pairs and register-blocked over the 8 x 8 child pairs.
 //
-//   effVal(c)[f] = (1/(2np)^3) sum_{v in V(c)} T_{v-c}[f] effDen(v)[f]
+//   effVal(c)[f] = (1/N^3) sum_{v in V(c)} T_{v-c}[f] effDen(v)[f]
 //   (cptwvv, fmm3d_mpi/matmgnt3d_mpi.cpp:414-429)
 //
 // V(c) for a child c of a parent P is the set of children c2 of P's
@@ -9,18 +9,8 @@
 // 1687-1698).  For a fixed neighbour offset o = Q - P the relative position of
 // the pair is r = 2o + (c2 - c), so the 64 pairs use at most 27 distinct
 // translations, and whether a pair interacts depends on (o, c2 - c) only.
-// One warp owns one output parent and 32 frequencies (lane = frequency): per
-// neighbour it loads the 8 child spectra of Q once into registers and applies
-// each distinct translation to every pair that uses it.  The 64 pairs are
-// unrolled by child offset e = c2 - c (27 groups); a [26 x 27] table in shared
-// memory gives the translation of (neighbour offset, e), or a zero row for
-// touching pairs, so one branch-free code path serves every neighbour offset.
-// The 316 translation spectra of the CTA's frequencies (plus the zero row) sit
-// in shared memory.
-//
-// ADJ selects the transposed operator: rows are the source parents Q with
-// their target parents P at offset o' = P - Q, outputs the source children,
-// and each pair uses conj(T) of the forward relative position -(2o' + c - c2).
+// One right-hand side, FP64 and FP32: k_m2l_had_d.  FP32 with several:
+// k_m2l_had_o and the other 27-product forms.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -30,14 +20,6 @@
 #include "had_smem.cuh"
 
 namespace fmmg {
-
-constexpr int PQ_THREADS = 512;
-// dynamic shared memory of the kernels below: 316 translations + the zero row, fw frequencies
-template <typename C>
-inline size_t pq_smem_bytes(int fw) {
-  return (size_t)317 * fw * sizeof(C);
-}
-constexpr int PQ_PARENTS = 128;  // output parents per CTA
 
 // Output parents per CTA of the scalar Hadamard kernels: `most` (the tuned
 // figure), fewer where that many would leave fewer than `ctas` CTAs, down to one
@@ -55,125 +37,6 @@ __device__ __forceinline__ void pq_cfma(C& acc, const C t, const C d) {
   acc.x = fma(-t.y, d.y, acc.x);
   acc.y = fma(t.x, d.y, acc.y);
   acc.y = fma(t.y, d.x, acc.y);
-}
-
-// child offset e = E (0..26): every pair (c out, c2 = c + e in) with the
-// translation of this (neighbour offset, e) -- zero for touching pairs; then E + 1.
-// One branch-free code path serves all 26 neighbour offsets.
-template <typename C, int KB, bool ADJ, int E, int FW = 32>
-__device__ __forceinline__ void pq_delta(C (&acc)[8][KB], const C (&in)[8][KB], const C* __restrict__ Ts,
-                                         const int16_t* __restrict__ sIdRow, int lane) {
-  if constexpr (E < 27) {
-    constexpr int ex = E / 9 - 1, ey = (E / 3) % 3 - 1, ez = E % 3 - 1;
-    C t = Ts[sIdRow[E] * FW + lane];
-    if (ADJ) t.y = -t.y;
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const int x2 = (c >> 2) + ex, y2 = ((c >> 1) & 1) + ey, z2 = (c & 1) + ez;
-      if (x2 < 0 || x2 > 1 || y2 < 0 || y2 > 1 || z2 < 0 || z2 > 1) continue;
-      const int c2 = x2 * 4 + y2 * 2 + z2;
-#pragma unroll
-      for (int q = 0; q < KB; q++) pq_cfma(acc[c][q], t, in[c2][q]);
-    }
-    pq_delta<C, KB, ADJ, E + 1, FW>(acc, in, Ts, sIdRow, lane);
-  }
-}
-
-template <bool ADJ>
-__device__ __forceinline__ void pq_id_table(int16_t* sId, const int16_t* __restrict__ transId) {
-  for (int i = threadIdx.x; i < 27 * 27; i += blockDim.x) {
-    const int o = i / 27, e = i % 27;
-    int rx = 2 * (o / 9 - 1) + (e / 9 - 1), ry = 2 * ((o / 3) % 3 - 1) + ((e / 3) % 3 - 1),
-        rz = 2 * (o % 3 - 1) + (e % 3 - 1);
-    if (ADJ) {
-      rx = -rx;
-      ry = -ry;
-      rz = -rz;
-    }
-    const int id = o == 13 ? -1 : transId[(rx + 3) * 49 + (ry + 3) * 7 + (rz + 3)];
-    sId[i] = (int16_t)(id < 0 ? 316 : id);  // row 316 of the staged slice is zero
-  }
-}
-
-// Rows are output parents.  rowOut[8*b + c] is the spectrum row of child c of
-// row b (or -1); per row the neighbour entries nPtr[b]..nPtr[b+1] carry the
-// offset code nOff (dx+1)*9+(dy+1)*3+(dz+1) of neighbour - row and the input
-// spectrum rows of the neighbour's 8 children nIn[8*e + c2] (or -1).  effIn /
-// effOut hold nrhs right-hand sides at strides inRhs / outRhs; transId maps
-// (rx+3)*49+(ry+3)*7+(rz+3) to a translation id or -1.  Grid (rows /
-// rows per CTA, nEff / 32, ceil(nrhs / KB)) (PQ_PARENTS rows per CTA by default); dynamic shared memory
-// pq_smem_bytes<C>(32).  The child slots of the next entry are fetched while
-// the current one is applied, so each neighbour costs one dependent load.
-template <typename C, int KB, bool ADJ>
-__global__ void __launch_bounds__(PQ_THREADS)
-    k_m2l_had_pq(int nRows, const int32_t* __restrict__ rowOut, const int64_t* __restrict__ nPtr,
-                 const int8_t* __restrict__ nOff, const int32_t* __restrict__ nIn, const C* __restrict__ effIn,
-                 int64_t inRhs, const C* __restrict__ T, C* __restrict__ effOut, int64_t outRhs, int nEff, int nrhs,
-                 typename CplxOps<C>::R nrmfc, const int16_t* __restrict__ transId) {
-  typedef typename CplxOps<C>::R R;
-  extern __shared__ unsigned char pq_smem[];
-  C* Ts = reinterpret_cast<C*>(pq_smem);  // [316][32]
-  __shared__ int16_t sId[27 * 27];        // [neighbour offset][child offset] -> translation id or -1
-  pq_id_table<ADJ>(sId, transId);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int f0 = blockIdx.y * 32;
-  const int f = f0 + lane;
-  const int rhs0 = blockIdx.z * KB;
-  for (int i = threadIdx.x; i < 317 * 32; i += blockDim.x) {
-    const int id = i >> 5, ff = f0 + (i & 31);
-    Ts[i] = (ff < nEff && id < 316) ? T[(int64_t)id * nEff + ff] : CplxOps<C>::zero();
-  }
-  __syncthreads();
-  if (f >= nEff) return;
-  const C* inF = effIn + (int64_t)rhs0 * inRhs + f;
-  const int per = (nRows + gridDim.x - 1) / gridDim.x;  // rows per CTA: the grid sets it (tunable)
-  const int bEnd = min(nRows, (int)(blockIdx.x + 1) * per);
-  for (int b = blockIdx.x * per + warp; b < bEnd; b += PQ_THREADS / 32) {
-    C acc[8][KB];
-#pragma unroll
-    for (int c = 0; c < 8; c++)
-#pragma unroll
-      for (int q = 0; q < KB; q++) acc[c][q] = CplxOps<C>::zero();
-    int64_t e = nPtr[b];
-    const int64_t e1 = nPtr[b + 1];
-    int4 sa = make_int4(-1, -1, -1, -1), sb = sa;
-    int off = 13;
-    if (e < e1) {
-      sa = reinterpret_cast<const int4*>(nIn)[2 * e];
-      sb = reinterpret_cast<const int4*>(nIn)[2 * e + 1];
-      off = nOff[e];
-    }
-    for (; e < e1; e++) {
-      const int sl[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
-      C in[8][KB];
-#pragma unroll
-      for (int c2 = 0; c2 < 8; c2++)
-#pragma unroll
-        for (int q = 0; q < KB; q++)
-          in[c2][q] = (sl[c2] >= 0 && rhs0 + q < nrhs) ? inF[(int64_t)q * inRhs + (int64_t)sl[c2] * nEff]
-                                                       : CplxOps<C>::zero();
-      const int offCur = off;
-      if (e + 1 < e1) {
-        sa = reinterpret_cast<const int4*>(nIn)[2 * (e + 1)];
-        sb = reinterpret_cast<const int4*>(nIn)[2 * (e + 1) + 1];
-        off = nOff[e + 1];
-      }
-      pq_delta<C, KB, ADJ, 0>(acc, in, Ts, &sId[offCur * 27], lane);
-    }
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const int t = rowOut[8 * b + c];
-      if (t < 0) continue;
-#pragma unroll
-      for (int q = 0; q < KB; q++)
-        if (rhs0 + q < nrhs) {
-          C o;
-          o.x = acc[c][q].x * (R)nrmfc;
-          o.y = acc[c][q].y * (R)nrmfc;
-          effOut[(int64_t)(rhs0 + q) * outRhs + (int64_t)t * nEff + f] = o;
-        }
-    }
-  }
 }
 
 // ---------------------------------------------------------------- FP32 form
@@ -195,139 +58,153 @@ __device__ __forceinline__ void pq_fma2(unsigned long long& acc, unsigned long l
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-// The translation of this group as the two packed operands (t.x, t.x) and
-// (t.y, t.y): for FW = 4 the CTA stages each translation pre-duplicated as
-// {t.x, t.x, t.y, t.y} (conjugated for ADJ), so one 16-byte shared load gives
-// both; for FW = 32 it stages plain complex values and packs in registers.
-template <bool ADJ, int FW>
-__device__ __forceinline__ void pq_tpair(const void* __restrict__ Ts, int row, int fl, unsigned long long& tx,
-                                         unsigned long long& ty) {
-  if constexpr (FW == 4) {
-    const ulonglong2 t = reinterpret_cast<const ulonglong2*>(Ts)[row * FW + fl];
-    tx = t.x;
-    ty = t.y;
-  } else {
-    const float2 t = reinterpret_cast<const float2*>(Ts)[row * FW + fl];
-    tx = pq_pk(t.x, t.x);
-    ty = ADJ ? pq_pk(-t.y, -t.y) : pq_pk(t.y, t.y);
-  }
-}
-
-template <bool ADJ, int E, int FW>
-__device__ __forceinline__ void pq_delta_x2(unsigned long long (&acc)[8], const unsigned long long (&inD)[8],
-                                            const unsigned long long (&inR)[8], const void* __restrict__ Ts,
-                                            const int16_t* __restrict__ sIdRow, int fl) {
-  if constexpr (E < 27) {
-    constexpr int ex = E / 9 - 1, ey = (E / 3) % 3 - 1, ez = E % 3 - 1;
-    unsigned long long tx, ty;
-    pq_tpair<ADJ, FW>(Ts, sIdRow[E], fl, tx, ty);
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const int x2 = (c >> 2) + ex, y2 = ((c >> 1) & 1) + ey, z2 = (c & 1) + ez;
-      if (x2 < 0 || x2 > 1 || y2 < 0 || y2 > 1 || z2 < 0 || z2 > 1) continue;
-      const int c2 = x2 * 4 + y2 * 2 + z2;
-      pq_fma2(acc[c], tx, inD[c2]);
-      pq_fma2(acc[c], ty, inR[c2]);
-    }
-    pq_delta_x2<ADJ, E + 1, FW>(acc, inD, inR, Ts, sIdRow, fl);
-  }
-}
-
-// FW frequencies x (32 / FW) right-hand sides per warp (lane = rhs * FW +
-// frequency), one right-hand side per thread: FW = 32 for a single
-// right-hand side, FW = 4 for blocks of 8, where every translation value read
-// from shared memory serves 8 lanes and the CTA stages only 4 frequencies of
-// the 316 translations (10 KB), so residency is set by registers.  Grid (rows
-// per CTA, nEff / FW, ceil(nrhs / (32 / FW))) (PQX_ROWS rows per CTA by default); blockIdx.z selects the
-// right-hand-side block of the layout below; dynamic shared memory
-// pqx_smem_bytes<FW>() (row 316 is the zero row of touching pairs).
 constexpr int PQX_THREADS = 256;
-constexpr int PQX_ROWS = 64;
-template <int FW>
-inline size_t pqx_smem_bytes() {
-  return (size_t)317 * FW * (FW == 4 ? 16 : 8);
-}
-
-// Spectrum layout: value (right-hand side r, slot s, frequency f) of effIn
-// sits at (r / RW) * in.blk + s * in.slot + f * fStride + (r % RW) * rStride
-// (effOut likewise): planes of one right-hand side (RW = 1, fStride = 1), or
-// blocks of 8 interleaved right-hand sides (RW = 8, fStride = 8, rStride = 1).
+// Spectrum layout of the forms with several right-hand sides: blocks of RW
+// interleaved ones, value (right-hand side r, slot s, frequency f) at
+// (r / RW) * blk + s * slot + f * RW + r % RW.
 struct PqLayout {
   int64_t blk, slot;
 };
 
-template <int FW, bool ADJ>
-__global__ void __launch_bounds__(PQX_THREADS, 3)
-    k_m2l_had_pqx2(int nRows, const int32_t* __restrict__ rowOut, const int64_t* __restrict__ nPtr,
-                   const int8_t* __restrict__ nOff, const int32_t* __restrict__ nIn, const float2* __restrict__ effIn,
-                   PqLayout inL, const float2* __restrict__ T, float2* __restrict__ effOut, PqLayout outL,
-                   int fStride, int rStride, int nEff, int nrhs, float nrmfc, const int16_t* __restrict__ transId) {
-  constexpr int RW = 32 / FW;
-  extern __shared__ __align__(16) unsigned char pqx_smem[];
-  __shared__ int16_t sId[27 * 27];
-  pq_id_table<ADJ>(sId, transId);
+// acc += t * d: FP32 as one packed FMA for the t.x terms and two scalar ones
+__device__ __forceinline__ void hd_cmac(double2& a, double2 t, double2 x) { pq_cfma(a, t, x); }
+__device__ __forceinline__ void hd_cmac(float2& a, float2 t, float2 x) {
+  unsigned long long p = pq_pk(a.x, a.y);
+  pq_fma2(p, pq_pk(t.x, t.x), pq_pk(x.x, x.y));
+  a = pq_unpk(p);
+  a.x = fmaf(-t.y, x.y, a.x);
+  a.y = fmaf(t.y, x.x, a.y);
+}
+
+// One right-hand side.  A warp owns one output parent and 32 frequencies (lane
+// = frequency).  The CTA stages the translations of its frequencies at every
+// relative position -3..3 per axis (zeros for the touching ones), so the 27
+// positions of a neighbour are constants from one base address and their reads
+// are independent; each translation serves every pair of its child offset, the
+// 64 pairs of a neighbour unrolled by child offset.  The spectra of the next
+// neighbour's 8 children load while this one's are multiplied.  That matters:
+// with an index table between the offset and the translation and the spectra
+// loaded where they are used, the FP64 pipe, the shared-memory path (108 cycles
+// of reads a neighbour for 128 of multiply-adds) and L2 were all under half
+// busy.  FP64: 1M points 3.88 -> 3.42 ms, 131,072 points 0.50 -> 0.38 ms; FP32
+// k = 1, 100,000 points 0.235 -> 0.164 ms.
+//
+// Rows are output parents.  rowOut[8*b + c] is the spectrum row of child c of
+// row b (or -1); per row the neighbour entries nPtr[b]..nPtr[b+1] carry the
+// offset code nOff (dx+1)*9+(dy+1)*3+(dz+1) of neighbour - row and the input
+// spectrum rows of the neighbour's 8 children nIn[8*e + c2] (or -1).  ADJ selects
+// the transposed operator: rows are the source parents with their target
+// parents as neighbours, and each pair uses conj(T) of the opposite position.
+// Grid (rows / per, nEff / 32, right-hand sides inRhs / outRhs apart); dynamic
+// shared memory hd_smem_bytes.
+template <typename C>
+struct HdShape;
+template <>
+struct HdShape<double2> {
+  static constexpr int THREADS = 512, CTAS = 1;  // 128 registers, 175 KB
+};
+template <>
+struct HdShape<float2> {
+  static constexpr int THREADS = 384, CTAS = 2;  // 80 registers, 88 KB
+};
+template <typename C>
+constexpr size_t hd_smem_bytes() {
+  return (size_t)343 * 32 * sizeof(C);
+}
+
+template <typename C, bool ADJ>
+__global__ void __launch_bounds__(HdShape<C>::THREADS, HdShape<C>::CTAS)
+    k_m2l_had_d(int nRows, int per, const int32_t* __restrict__ rowOut, const int64_t* __restrict__ nPtr,
+                const int8_t* __restrict__ nOff, const int32_t* __restrict__ nIn, const C* __restrict__ effIn,
+                int64_t inRhs, const C* __restrict__ T, C* __restrict__ effOut, int64_t outRhs, int nEff,
+                typename CplxOps<C>::R nrmfc, const int16_t* __restrict__ transId) {
+  constexpr int THREADS = HdShape<C>::THREADS, SG = ADJ ? -1 : 1;
+  extern __shared__ __align__(16) unsigned char hd_smem[];
+  C* Ts = reinterpret_cast<C*>(hd_smem);  // [343][32]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int fl = lane % FW, rl = lane / FW;
-  const int f0 = blockIdx.y * FW;
-  const int f = f0 + fl;
-  const int rhs = blockIdx.z * RW + rl;
-  for (int i = threadIdx.x; i < 317 * FW; i += blockDim.x) {
-    const int id = i / FW, ff = f0 + i % FW;
-    const float2 t = (ff < nEff && id < 316) ? T[(int64_t)id * nEff + ff] : make_float2(0.f, 0.f);
-    if constexpr (FW == 4) {
-      const float ty = ADJ ? -t.y : t.y;
-      reinterpret_cast<float4*>(pqx_smem)[i] = make_float4(t.x, t.x, ty, ty);
-    } else {
-      reinterpret_cast<float2*>(pqx_smem)[i] = t;
-    }
+  const int f0 = blockIdx.y * 32, f = f0 + lane;
+  for (int i = threadIdx.x; i < 343 * 32; i += THREADS) {
+    const int id = transId[i >> 5], ff = f0 + (i & 31);
+    C t = id >= 0 && ff < nEff ? T[(int64_t)id * nEff + ff] : CplxOps<C>::zero();
+    if (ADJ) t.y = -t.y;
+    Ts[i] = t;
   }
   __syncthreads();
-  const void* Ts = pqx_smem;
-  const bool act = f < nEff && rhs < nrhs;
-  const int64_t lanePos = act ? (int64_t)f * fStride + (int64_t)rl * rStride : 0;
-  const float2* inF = effIn + (act ? blockIdx.z * inL.blk : 0) + lanePos;
-  float2* outF = effOut + blockIdx.z * outL.blk + lanePos;
-  const int per = (nRows + gridDim.x - 1) / gridDim.x;  // rows per CTA: the grid sets it (tunable)
+  if (f >= nEff) return;
+  const C* inF = effIn + blockIdx.z * inRhs + f;
   const int bEnd = min(nRows, (int)(blockIdx.x + 1) * per);
-  for (int b = blockIdx.x * per + warp; b < bEnd; b += PQX_THREADS / 32) {
-    unsigned long long acc[8];
+  for (int b = blockIdx.x * per + warp; b < bEnd; b += THREADS / 32) {
+    C acc[8], xn[8];
 #pragma unroll
-    for (int c = 0; c < 8; c++) acc[c] = 0ull;
-    int64_t e = nPtr[b];
-    const int64_t e1 = nPtr[b + 1];
-    int4 sa = make_int4(-1, -1, -1, -1), sb = sa;
-    int off = 13;
-    if (e < e1) {
-      sa = reinterpret_cast<const int4*>(nIn)[2 * e];
-      sb = reinterpret_cast<const int4*>(nIn)[2 * e + 1];
-      off = nOff[e];
-    }
-    for (; e < e1; e++) {
+    for (int c = 0; c < 8; c++) acc[c] = CplxOps<C>::zero();
+    const int64_t e0 = nPtr[b];
+    const int ne = (int)(nPtr[b + 1] - e0);
+    const int4* in4 = reinterpret_cast<const int4*>(nIn) + 2 * e0;
+    int4 sa, sb;   // child slots one neighbour ahead of the loads
+    int offN = 13;
+    auto slots = [&](int j) {
+      sa = sb = make_int4(-1, -1, -1, -1);
+      if (j < ne) {
+        sa = in4[2 * j];
+        sb = in4[2 * j + 1];
+      }
+    };
+    auto load = [&]() {
       const int sl[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
-      unsigned long long inD[8], inR[8];
 #pragma unroll
-      for (int c2 = 0; c2 < 8; c2++) {
-        const float2 d = (act && sl[c2] >= 0) ? inF[(int64_t)sl[c2] * inL.slot] : make_float2(0.f, 0.f);
-        inD[c2] = pq_pk(d.x, d.y);
-        inR[c2] = pq_pk(-d.y, d.x);
+      for (int c2 = 0; c2 < 8; c2++) xn[c2] = sl[c2] >= 0 ? inF[(int64_t)sl[c2] * nEff] : CplxOps<C>::zero();
+    };
+    slots(0);
+    load();
+    slots(1);
+    if (ne > 0) offN = nOff[e0];
+    for (int j = 0; j < ne; j++) {
+      C x[8];
+#pragma unroll
+      for (int c2 = 0; c2 < 8; c2++) x[c2] = xn[c2];
+      const int off = offN;
+      load();
+      slots(j + 2);
+      if (j + 1 < ne) offN = nOff[e0 + j + 1];
+      // position of (neighbour child 0) - (output child 0)
+      const int pos = ((SG * 2 * (off / 9 - 1) + 3) * 7 + SG * 2 * ((off / 3) % 3 - 1) + 3) * 7 +
+                      SG * 2 * (off % 3 - 1) + 3;
+      const C* Tb = Ts + pos * 32 + lane;
+#pragma unroll
+      for (int E = 0; E < 27; E++) {
+        const int ex = E / 9 - 1, ey = (E / 3) % 3 - 1, ez = E % 3 - 1;
+        const C t = Tb[SG * (49 * ex + 7 * ey + ez) * 32];
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+          const int x2 = (c >> 2) + ex, y2 = ((c >> 1) & 1) + ey, z2 = (c & 1) + ez;
+          if (x2 < 0 || x2 > 1 || y2 < 0 || y2 > 1 || z2 < 0 || z2 > 1) continue;
+          hd_cmac(acc[c], t, x[x2 * 4 + y2 * 2 + z2]);
+        }
       }
-      const int offCur = off;
-      if (e + 1 < e1) {
-        sa = reinterpret_cast<const int4*>(nIn)[2 * (e + 1)];
-        sb = reinterpret_cast<const int4*>(nIn)[2 * (e + 1) + 1];
-        off = nOff[e + 1];
-      }
-      pq_delta_x2<ADJ, 0, FW>(acc, inD, inR, Ts, &sId[offCur * 27], fl);
     }
-    if (!act) continue;
 #pragma unroll
     for (int c = 0; c < 8; c++) {
       const int t = rowOut[8 * b + c];
       if (t < 0) continue;
-      const float2 a = pq_unpk(acc[c]);
-      outF[(int64_t)t * outL.slot] = make_float2(a.x * nrmfc, a.y * nrmfc);
+      C o;
+      o.x = acc[c].x * nrmfc;
+      o.y = acc[c].y * nrmfc;
+      effOut[blockIdx.z * outRhs + (int64_t)t * nEff + f] = o;
     }
   }
+}
+
+template <typename C, bool ADJ>
+inline void launch_had_d(cudaStream_t st, int numSMs, int mostRows, int nRows, int nrhs, const int32_t* rowOut,
+                         const int64_t* nPtr, const int8_t* nOff, const int32_t* nIn, const C* effIn, int64_t inRhs,
+                         const C* T, C* effOut, int64_t outRhs, int nEff, double nrmfc, const int16_t* transId) {
+  auto* k = k_m2l_had_d<C, ADJ>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hd_smem_bytes<C>());
+  const int sl = (nEff + 31) / 32;
+  const int per = had_rows_per_cta(nRows, sl * nrhs, 2 * HdShape<C>::CTAS * numSMs, mostRows);
+  k<<<dim3((nRows + per - 1) / per, sl, nrhs), HdShape<C>::THREADS, hd_smem_bytes<C>(), st>>>(
+      nRows, per, rowOut, nPtr, nOff, nIn, effIn, inRhs, T, effOut, outRhs, nEff, (typename CplxOps<C>::R)nrmfc,
+      transId);
 }
 
 }  // namespace fmmg

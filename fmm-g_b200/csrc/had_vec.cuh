@@ -146,7 +146,7 @@ __device__ __forceinline__ void hv_cmac(float2& a, float2 t, float2 x) {
 
 // Grid (chunks of `per` target parents, ceil(nEff / FW), blocks of RW = R RL
 // right-hand sides); dynamic shared memory hv_smem_bytes.  Tp: the packed
-// table (k_hv_pack).  rowOut, nPtr, nOff, nIn as in k_m2l_had_pq.
+// table (k_hv_pack).  rowOut, nPtr, nOff, nIn as in k_m2l_had_d.
 // Lanes = RL groups of R right-hand sides (fastest, as the spectra are laid
 // out) x FW frequencies x PW consecutive target parents.  A lane group walks
 // its parent's neighbours child by child: per existing input child it loads

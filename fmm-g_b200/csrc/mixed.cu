@@ -1589,9 +1589,9 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
   // of the Hadamard kernel that tuning alone selects.
   const bool scalar = P.sdm == 1 && P.tdm == 1;
   const bool r8 = scalar && kc >= 2 && D.hadPQ;
-  const bool hadO = D.hadW && D.m2lTw32 && D.tune.hadRhsPerThread >= 3;
+  const bool hadO = D.tune.hadRhsPerThread >= 3;
   int lgRW = r8 ? 3 : 0;
-  if (!scalar || (r8 && D.hadW && D.m2lTw32 && D.tune.hadRhsPerThread == 4)) {
+  if (!scalar || (r8 && D.tune.hadRhsPerThread == 4)) {
     lgRW = 0;
     while (lgRW < 3 && (1 << lgRW) < kc) lgRW++;
     if (lgRW == 3 && (kc + 3) / 4 * 4 < (kc + 7) / 8 * 8) lgRW = 2;
@@ -1638,13 +1638,8 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
   }
     if (scalar && D.hadPQ) {
       if (!r8) {  // planes of one right-hand side
-        const size_t smem = pqx_smem_bytes<32>();
-        cudaFuncSetAttribute(k_m2l_had_pqx2<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        const int sl = (P.nEff32 + 31) / 32, hr = had_rows_per_cta(npar, sl * kc, 6 * D.numSMs, D.tune.hadRows);
-        dim3 g1((npar + hr - 1) / hr, sl, kc);
-        k_m2l_had_pqx2<32, false><<<g1, PQX_THREADS, smem, st>>>(
-            npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen32, PqLayout{effDR, P.nEff32}, D.m2lT32, D.effVal32,
-            PqLayout{effVR, P.nEff32}, 1, 0, P.nEff32, kc, nrmfc, D.transIdDev);
+        launch_had_d<float2, false>(st, D.numSMs, D.tune.hadRows, npar, kc, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn,
+                                    D.effDen32, effDR, D.m2lT32, D.effVal32, effVR, P.nEff32, nrmfc, D.transIdDev);
       } else if (hadO) {  // output-child accumulators
 #define FMMG_HADO(R_, G_)                                                                                     \
   do {                                                                                                        \
@@ -1662,26 +1657,20 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
         else if (RW == 4) FMMG_HADO(4, 1);
         else FMMG_HADO(2, 1);
 #undef FMMG_HADO
-      } else if (D.hadW && D.m2lTw32 && D.tune.hadRhsPerThread == 2) {  // 27-product form, 2 RHS a thread
+      } else if (D.tune.hadRhsPerThread == 2) {  // 27-product form, 2 RHS a thread
         const size_t smem = (size_t)W8_OFFS * 27 * W8X2_F * sizeof(float2);
         cudaFuncSetAttribute(k_m2l_had_w8x2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         dim3 g8((npar + D.tune.hadRows - 1) / D.tune.hadRows, (P.nEff32 + W8X2_F - 1) / W8X2_F, nblk);
         k_m2l_had_w8x2<<<g8, PQX_THREADS, smem, st>>>(npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen32,
                                                        PqLayout{blkDen, (int64_t)P.nEff32 * 8}, D.m2lTw32, D.effVal32,
                                                        PqLayout{blkVal, (int64_t)P.nEff32 * 8}, P.nEff32, kc, nrmfc);
-      } else if (D.hadW && D.m2lTw32) {  // 27-product form
+      } else {  // 27-product form
         const size_t smem = (size_t)W8_OFFS * 27 * 4 * sizeof(float2);
         cudaFuncSetAttribute(k_m2l_had_w8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         dim3 g8((npar + D.tune.hadRows - 1) / D.tune.hadRows, (P.nEff32 + 3) / 4, nblk);
         k_m2l_had_w8<<<g8, PQX_THREADS, smem, st>>>(npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen32,
                                                      PqLayout{blkDen, (int64_t)P.nEff32 * 8}, D.m2lTw32, D.effVal32,
                                                      PqLayout{blkVal, (int64_t)P.nEff32 * 8}, P.nEff32, kc, nrmfc);
-      } else {
-        const size_t smem = pqx_smem_bytes<4>();
-        dim3 g8((npar + D.tune.hadRows - 1) / D.tune.hadRows, (P.nEff32 + 3) / 4, nblk);
-        k_m2l_had_pqx2<4, false><<<g8, PQX_THREADS, smem, st>>>(
-            npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen32, PqLayout{blkDen, (int64_t)P.nEff32 * 8}, D.m2lT32,
-            D.effVal32, PqLayout{blkVal, (int64_t)P.nEff32 * 8}, 8, 1, P.nEff32, kc, nrmfc, D.transIdDev);
       }
     } else if (scalar) {
       if (!D.vListsReady) throw std::logic_error("the expanded V lists are not on the device (dev_upload_vlists)");

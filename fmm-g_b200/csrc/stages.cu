@@ -5,7 +5,7 @@
 //                     M2M + C2E as batched row GEMMs (k_gemm_f64)
 //   U-list  :773-785  k_p2p_near_w (true kernel, sources of adjacent leaves)
 //   V-list  :1015-1051 k_m2l_fwd (r2c of each upward density on the (2np)^3
-//                     grid), k_m2l_had_pq / k_m2l_had_v64 (per-frequency
+//                     grid), k_m2l_had_d / k_m2l_had_v64 (per-frequency
 //                     products grouped by parent pairs), k_m2l_inv (c2r + gather onto DC)
 //   W-list  :1139-1175 S2T entries folded into k_p2p_near_w, M2T in k_e2t
 //   X-list  :1241-1257 S2T entries folded into k_p2p_near_w, S2L in k_src2surf
@@ -1013,13 +1013,8 @@ static void launch_m2l_np(const Plan& P, DevState& D, LaunchStats* ls) {
   if (npar > 0 && ntrg > 0) {
     const double nrmfc = 1.0 / double(P.nReg);
     if (P.sdm == 1 && P.tdm == 1 && D.hadPQ) {
-      const size_t smem = pq_smem_bytes<double2>(32);
-      cudaFuncSetAttribute(k_m2l_had_pq<double2, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      const int hr = had_rows_per_cta(npar, (P.nEff + 31) / 32, 2 * D.numSMs, D.tune.pqParents);
-      dim3 g2((npar + hr - 1) / hr, (P.nEff + 31) / 32, 1);
-      k_m2l_had_pq<double2, 1, false><<<g2, PQ_THREADS, smem, D.stream>>>(
-          npar, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn, D.effDen, 0, D.m2lT, D.effVal, 0, P.nEff, 1, nrmfc,
-          D.transIdDev);
+      launch_had_d<double2, false>(D.stream, D.numSMs, D.tune.pqParents, npar, 1, D.vRowOut, D.vPtr, D.vOff, D.vNbrIn,
+                                   D.effDen, 0, D.m2lT, D.effVal, 0, P.nEff, nrmfc, D.transIdDev);
     } else if (P.sdm == 1 && P.tdm == 1) {
       if (!D.vListsReady) throw std::logic_error("the expanded V lists are not on the device (dev_upload_vlists)");
       const size_t smem = had_smem_bytes<double2>();
@@ -1093,13 +1088,8 @@ void spectral_inv(const Plan& P, DevState& D, int n, const int32_t* nodes, int d
 void hadamard_pq64_adj(const Plan& P, DevState& D, const double2* in, double2* out) {
   const int nrow = (int)P.vParentsT.size();
   if (nrow <= 0) return;
-  const size_t smem = pq_smem_bytes<double2>(32);
-  cudaFuncSetAttribute(k_m2l_had_pq<double2, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const int hr = had_rows_per_cta(nrow, (P.nEff + 31) / 32, 2 * D.numSMs, D.tune.pqParents);
-  dim3 g2((nrow + hr - 1) / hr, (P.nEff + 31) / 32, 1);
-  k_m2l_had_pq<double2, 1, true><<<g2, PQ_THREADS, smem, D.stream>>>(
-      nrow, D.vRowOutT, D.vNbrTPtr, D.vNbrOffT, D.vNbrInT, in, 0, D.m2lT, out, 0, P.nEff, 1, 1.0 / double(P.nReg),
-      D.transIdDev);
+  launch_had_d<double2, true>(D.stream, D.numSMs, D.tune.pqParents, nrow, 1, D.vRowOutT, D.vNbrTPtr, D.vNbrOffT,
+                              D.vNbrInT, in, 0, D.m2lT, out, 0, P.nEff, 1.0 / double(P.nReg), D.transIdDev);
 }
 void hadamard_list64(const Plan& P, DevState& D, int nOut, const int64_t* ptr, const int32_t* ent, const double2* in,
                      double2* out, bool conj) {
