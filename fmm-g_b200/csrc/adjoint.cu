@@ -23,6 +23,7 @@
 #include "cuda_common.cuh"
 #include "engine.hpp"
 #include "kernels.hpp"
+#include "near_f64.cuh"
 
 namespace fmmg {
 
@@ -76,73 +77,14 @@ __device__ __forceinline__ void kaccum_t(double x, double y, double z, const dou
 // Points -> points, transposed (near-field P2P^T): for one source leaf (row),
 // g[s] += sum over the targets of the leaves listing it of K(x_t - y_s; n_s)^T w_t.
 template <int KT>
-__global__ void __launch_bounds__(AJ_THREADS)
-    k_pp_t(const int32_t* __restrict__ rows, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-           const int64_t* __restrict__ srcBeg, const int64_t* __restrict__ srcCnt,
-           const int64_t* __restrict__ trgBeg, const int64_t* __restrict__ trgCnt, const double* __restrict__ src,
-           const double* __restrict__ nrm, const double* __restrict__ trg, const double* __restrict__ w,
-           double* __restrict__ g, double mu, double ve) {
-  constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD, NRM = KTraits<KT>::NRM;
-  __shared__ double sPos[AJ_TILE * 3];
-  __shared__ double sW[AJ_TILE * TD];
-  __shared__ int64_t eBeg[AJ_MAXE];
-  __shared__ int32_t ePre[AJ_MAXE + 1];
-  __shared__ double sRed[AJ_THREADS * SD];
-  const int row = blockIdx.x;
-  const int a = rows[row];
-  const int64_t ob = srcBeg[a], on = srcCnt[a];
-  const int64_t e0 = ptr[row], e1 = ptr[row + 1];
-  const int tid = threadIdx.x;
-  const int TG = on <= 32 ? 32 : (on <= 64 ? 64 : 128);
-  const int S = AJ_THREADS / TG;
-  const int tl = tid % TG, sp = tid / TG;
-  for (int64_t o0 = 0; o0 < on; o0 += TG) {
-    const int64_t o = o0 + tl;
-    const bool act = o < on;
-    double px = 0, py = 0, pz = 0, n3[3] = {0, 0, 0};
-    if (act) {
-      px = src[3 * (ob + o)];
-      py = src[3 * (ob + o) + 1];
-      pz = src[3 * (ob + o) + 2];
-      if (NRM)
-        for (int d = 0; d < 3; d++) n3[d] = nrm[3 * (ob + o) + d];
-    }
-    double acc[SD];
-#pragma unroll
-    for (int c = 0; c < SD; c++) acc[c] = 0.0;
-    for (int64_t ec = e0; ec < e1; ec += AJ_MAXE) {
-      const int ne = (int)min((int64_t)AJ_MAXE, e1 - ec);
-      const int total = aj_load_entries(idx, ec, ne, 0, trgBeg, trgCnt, eBeg, ePre);
-      for (int base = 0; base < total; base += AJ_TILE) {
-        const int cnt = min(AJ_TILE, total - base);
-        __syncthreads();
-        for (int i = tid; i < cnt; i += AJ_THREADS) {
-          const int64_t t = aj_entry(base + i, ne, eBeg, ePre);
-          sPos[3 * i] = trg[3 * t];
-          sPos[3 * i + 1] = trg[3 * t + 1];
-          sPos[3 * i + 2] = trg[3 * t + 2];
-#pragma unroll
-          for (int c = 0; c < TD; c++) sW[TD * i + c] = w[t * TD + c];
-        }
-        __syncthreads();
-        if (act)
-          for (int i = sp; i < cnt; i += S)
-            kaccum_t<KT>(sPos[3 * i] - px, sPos[3 * i + 1] - py, sPos[3 * i + 2] - pz, n3, &sW[TD * i], acc, mu, ve);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < SD; c++) sRed[tid * SD + c] = acc[c];
-    __syncthreads();
-    if (sp == 0 && act)
-#pragma unroll
-      for (int c = 0; c < SD; c++) {
-        double s = 0;
-        for (int k = 0; k < S; k++) s += sRed[(tl + k * TG) * SD + c];
-        g[(ob + o) * SD + c] += s;
-      }
+struct NearP2PT {
+  static constexpr int SV = KTraits<KT>::TD, OC = KTraits<KT>::SD, PR = SV * OC == 1 ? 4 : 2;
+  static constexpr bool SN = false, ON = KTraits<KT>::NRM != 0, OWN_IS_TARGET = false;
+  static __device__ __forceinline__ void pair(double x, double y, double z, const double*, const double* on,
+                                              const double* v, double* acc, double mu, double ve) {
+    kaccum_t<KT>(x, y, z, on, v, acc, mu, ve);
   }
-}
+};
 
 // Points -> equivalent surface of a node, transposed equivalent kernel
 // (L2T^T onto the own DE surface with ptr == nullptr, M2T^T onto the UE surface
@@ -340,81 +282,18 @@ __device__ __forceinline__ bool kgrad(double x, double y, double z, const double
 // Near-field part of the target gradient: for one evaluator leaf,
 // grad[t] += w[t] * sum_s grad_x K(x_t - y_s; n_s) den[s] over its near list.
 template <int KT>
-__global__ void __launch_bounds__(AJ_THREADS)
-    k_grad_near(const int32_t* __restrict__ rows, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                const int64_t* __restrict__ srcBeg, const int64_t* __restrict__ srcCnt,
-                const int64_t* __restrict__ trgBeg, const int64_t* __restrict__ trgCnt,
-                const double* __restrict__ src, const double* __restrict__ nrm, const double* __restrict__ den,
-                const double* __restrict__ trg, const double* __restrict__ w, double* __restrict__ grad) {
-  constexpr int NRM = KTraits<KT>::NRM;
-  __shared__ double sPos[AJ_TILE * 3];
-  __shared__ double sNrm[NRM ? AJ_TILE * 3 : 1];
-  __shared__ double sDen[AJ_TILE];
-  __shared__ int64_t eBeg[AJ_MAXE];
-  __shared__ int32_t ePre[AJ_MAXE + 1];
-  __shared__ double sRed[AJ_THREADS * 3];
-  const int row = blockIdx.x;
-  const int g = rows[row];
-  const int64_t tb = trgBeg[g], tn = trgCnt[g];
-  const int64_t e0 = ptr[row], e1 = ptr[row + 1];
-  const int tid = threadIdx.x;
-  const int TG = tn <= 32 ? 32 : (tn <= 64 ? 64 : 128);
-  const int S = AJ_THREADS / TG;
-  const int tl = tid % TG, sp = tid / TG;
-  for (int64_t t0 = 0; t0 < tn; t0 += TG) {
-    const int64_t t = t0 + tl;
-    const bool act = t < tn;
-    double tx = 0, ty = 0, tz = 0;
-    if (act) {
-      tx = trg[3 * (tb + t)];
-      ty = trg[3 * (tb + t) + 1];
-      tz = trg[3 * (tb + t) + 2];
-    }
-    double acc[3] = {0, 0, 0};
-    for (int64_t ec = e0; ec < e1; ec += AJ_MAXE) {
-      const int ne = (int)min((int64_t)AJ_MAXE, e1 - ec);
-      const int total = aj_load_entries(idx, ec, ne, 0, srcBeg, srcCnt, eBeg, ePre);
-      for (int base = 0; base < total; base += AJ_TILE) {
-        const int cnt = min(AJ_TILE, total - base);
-        __syncthreads();
-        for (int i = tid; i < cnt; i += AJ_THREADS) {
-          const int64_t s = aj_entry(base + i, ne, eBeg, ePre);
-          sPos[3 * i] = src[3 * s];
-          sPos[3 * i + 1] = src[3 * s + 1];
-          sPos[3 * i + 2] = src[3 * s + 2];
-          if (NRM) {
-            sNrm[3 * i] = nrm[3 * s];
-            sNrm[3 * i + 1] = nrm[3 * s + 1];
-            sNrm[3 * i + 2] = nrm[3 * s + 2];
-          }
-          sDen[i] = den[s];
-        }
-        __syncthreads();
-        if (act)
-          for (int i = sp; i < cnt; i += S) {
-            double G[3];
-            if (kgrad<KT>(tx - sPos[3 * i], ty - sPos[3 * i + 1], tz - sPos[3 * i + 2], NRM ? &sNrm[3 * i] : nullptr,
-                          G)) {
-              acc[0] += G[0] * sDen[i];
-              acc[1] += G[1] * sDen[i];
-              acc[2] += G[2] * sDen[i];
-            }
-          }
-      }
-    }
-    __syncthreads();
-    for (int d = 0; d < 3; d++) sRed[tid * 3 + d] = acc[d];
-    __syncthreads();
-    if (sp == 0 && act) {
-      const double wt = w[tb + t];
-      for (int d = 0; d < 3; d++) {
-        double s = 0;
-        for (int k = 0; k < S; k++) s += sRed[(tl + k * TG) * 3 + d];
-        grad[(tb + t) * 3 + d] += wt * s;
-      }
-    }
+struct NearGrad {
+  static constexpr int SV = 1, OC = 3, PR = 3;
+  static constexpr bool SN = KTraits<KT>::NRM != 0, ON = false, OWN_IS_TARGET = true;
+  static __device__ __forceinline__ void pair(double x, double y, double z, const double* sn, const double*,
+                                              const double* v, double* acc, double, double) {
+    double G[3];
+    if (!kgrad<KT>(x, y, z, sn, G)) return;
+    acc[0] += G[0] * v[0];
+    acc[1] += G[1] * v[0];
+    acc[2] += G[2] * v[0];
   }
-}
+};
 
 // Far-field part of the target gradient through the equivalent densities
 // (Laplace single-layer equivalent kernel): the leaf's own DE surface (L2T)
@@ -647,9 +526,9 @@ static void run_adjoint(const Plan& P, DevState& D, int& launches) {
   }
   // near field, transposed: targets -> sources of the U, direct W and direct X leaves
   if (!P.adjNearRows.empty()) {
-    k_pp_t<KT><<<(unsigned)P.adjNearRows.size(), AJ_THREADS, 0, st>>>(D.adjNearRows, D.adjNearPtr, D.adjNearIdx,
-                                                                      D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt, D.src,
-                                                                      D.nrm, D.trg, w, g, mu, ve);
+    launch_near_f64<NearP2PT<KT>>(st, (int)P.adjNearRows.size(), D.maxLeafSrc, D.adjNearRows, D.adjNearPtr,
+                                  D.adjNearIdx, D.trgBeg, D.trgCnt, D.srcBeg, D.srcCnt, D.trg, nullptr, w, D.src, D.nrm,
+                                  nullptr, g, mu, ve);
     launches++;
   }
   // upward, transposed: C2E^T then M2M^T per level, root side first (nothing
@@ -682,9 +561,9 @@ template <int KT>
 static void run_target_grad(const Plan& P, DevState& D, int& launches) {
   cudaStream_t st = D.stream;
   if (!P.evtrLeaves.empty()) {
-    k_grad_near<KT><<<(unsigned)P.evtrLeaves.size(), AJ_THREADS, 0, st>>>(
-        D.evtrLeaves, D.nearPtr, D.nearIdx, D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt, D.src, D.nrm, D.den, D.trg,
-        D.val, D.gradT);
+    launch_near_f64<NearGrad<KT>>(st, (int)P.evtrLeaves.size(), D.maxLeafTrg, D.evtrLeaves, D.nearPtr, D.nearIdx,
+                                  D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt, D.src, D.nrm, D.den, D.trg, nullptr, D.val,
+                                  D.gradT, 0.0, 0.0);
     launches++;
   }
   if (!P.l2tLeaves.empty()) {

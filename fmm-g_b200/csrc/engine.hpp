@@ -44,7 +44,7 @@ struct DevState {
   int32_t* surfIJK = nullptr;  // np-surface point -> packed (i, j, k)
   // work lists
   int32_t *evtrLeaves = nullptr;
-  int64_t maxLeafTrg = 0;  // targets of the fullest evaluator leaf
+  int64_t maxLeafTrg = 0, maxLeafSrc = 0;  // targets of the fullest evaluator leaf, sources of the fullest leaf
   int64_t *nearPtr = nullptr; int32_t *nearIdx = nullptr;     // merged near list
   int64_t *nearUPtr = nullptr; int32_t *nearUIdx = nullptr;   // stage-split forms
   int64_t *nearWPtr = nullptr; int32_t *nearWIdx = nullptr;

@@ -131,7 +131,7 @@ __device__ __forceinline__ void mx_den(const float* __restrict__ s, float (&d)[N
 
 // near field: U-list, direct W and X entries; grid (evaluator leaves, blocks of
 // tb targets, RHS blocks).  The warps and lanes are arranged as in
-// k_p2p_near_w (stages.cu): NR = 2 targets a lane, TG = ceil(targets / 2) lanes a
+// k_near_f64 (near_f64.cuh): NR = 2 targets a lane, TG = ceil(targets / 2) lanes a
 // group, S = 32 / TG groups that split the sources, WS = 1 or 4 warps a leaf;
 // leaves in order[] (decreasing targets x near sources).
 // The offsets are formed from hi/lo FP32 pairs of the box-centred
@@ -372,7 +372,7 @@ __device__ __forceinline__ unsigned long long nl_fma(unsigned long long a, unsig
 // sources in 32 / TG strides.  The offsets, r^2 and 1/(4 pi r) of a source
 // against both targets and the KB multiply-adds of its densities run as
 // packed FP32x2 operations (half the instructions of a one-target loop).  As in
-// k_p2p_near_w (stages.cu) TG = ceil(targets / 2) need not be a power of two
+// k_near_f64 (near_f64.cuh) TG = ceil(targets / 2) need not be a power of two
 // (17 targets take 27 lanes, 16 or 32 lanes a group left them half idle), and
 // with fewer leaves than the GPU holds warps (48 an SM) the CTA's WS = 4 warps
 // share one: 100,000 points 0.35 -> 0.16 ms.  With 62,000 leaves that takes 2.10

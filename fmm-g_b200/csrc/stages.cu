@@ -3,13 +3,13 @@
 // Stage map (reference fmm3d_mpi/fmm3d_eval_mpi.cpp):
 //   upward  :557-595  S2M (k_src2surf on each leaf's UC surface), then per level
 //                     M2M + C2E as batched row GEMMs (k_gemm_f64)
-//   U-list  :773-785  k_p2p_near_w (true kernel, sources of adjacent leaves)
+//   U-list  :773-785  k_near_f64 (true kernel, sources of adjacent leaves)
 //   V-list  :1015-1051 k_m2l_fwd (r2c of each upward density on the (2np)^3
 //                     grid), k_m2l_had_d / k_m2l_had_v64 (per-frequency
 //                     products grouped by parent pairs), k_m2l_inv (c2r + gather onto DC)
-//   W-list  :1139-1175 S2T entries folded into k_p2p_near_w, M2T in k_e2t
-//   X-list  :1241-1257 S2T entries folded into k_p2p_near_w, S2L in k_src2surf
-//   downward:1368-1438 per level L2L + C2E row GEMMs, L2T in k_e2t
+//   W-list  :1139-1175 S2T entries folded into k_near_f64, M2T in k_e2t_w
+//   X-list  :1241-1257 S2T entries folded into k_near_f64, S2L in k_src2surf
+//   downward:1368-1438 per level L2L + C2E row GEMMs, L2T in k_e2t_w
 // Every output row (a leaf's targets, a box's check surface, a node's
 // spectrum) is owned by exactly one CTA, so no atomics are needed and the
 // stages are plain stream-ordered launches.
@@ -36,6 +36,7 @@
 #include "had_smem.cuh"
 #include "had_vec.cuh"
 #include "kernels.hpp"
+#include "near_f64.cuh"
 
 namespace fmmg {
 
@@ -59,128 +60,87 @@ __global__ void k_scatter_val(int64_t n, int td, const int64_t* __restrict__ per
 }
 
 // ------------------------------------------------------------------ near field
-// The CTA-per-box FP64 kernels below (k_e2t, k_src2surf) stage their sources
-// in tiles of P2P_TILE in shared memory; when a box has few targets the CTA
-// splits the tile between thread groups and reduces the partial sums at the
-// end.  The near field itself, for one evaluator leaf val[targets] +=
-// K(trg, src) den(src) over the source leaves of its near list (U-list,
-// direct W and X entries), is k_p2p_near_w: one warp per leaf.
-constexpr int P2P_THREADS = 128;
+// For one evaluator leaf val[targets] += K(trg, src) den(src) over the source
+// leaves of its near list (U-list, direct W and X entries): k_near_f64
+// (near_f64.cuh).  k_src2surf below stages its sources in tiles of P2P_TILE.
 constexpr int P2P_TILE = 128;
 constexpr int P2P_MAXE = 256;
 
 
-// k_p2p_near_w: the same sums, by warps without a CTA-wide barrier in their
-// loops.  A warp builds its entry table (source ranges and their prefix counts,
-// a shuffle scan per 32 entries) and stages P2PW_CH sources at a time in its
-// own slice of shared memory.  Its lanes are S groups of TG: a lane of a group
-// holds PR targets (4 for scalar kernels, 2 otherwise), TG = ceil(targets / PR)
-// and S = 32 / TG split the sources, so that 17 targets, the mean of the
-// 1M-point workload's leaves, occupy 30 lanes where one target a lane left 15
-// idle; the PR independent inverse square roots of a lane hide the latency of
-// the FP64 pipe.  The groups' partial sums meet through warp shuffles.
-// The 4 warps of a CTA share a leaf and take its chunks of sources in turn (one
-// warp a leaf left the GPU idle behind the longest leaves, and all of it with
-// few leaves), their sums meet in shared memory in warp order; blocks of tb
-// targets of a leaf run as separate CTAs (grid.y).
-// Against one warp a leaf and one target a lane: 65,536 points in 554 leaves 2.58
-// -> 0.37 ms, Stokes 60,007 points 1.28 -> 0.28, 1M points in 62,000 leaves 2.15 ->
-// 1.54 (1.93 with one warp a leaf).
-constexpr int P2PW_WARPS = 4, P2PW_CH = 64, P2PW_MAXE = 128;
-template <int KT>
-constexpr int p2pw_targets() {
-  return KTraits<KT>::SD * KTraits<KT>::TD == 1 ? 4 : 2;
+// k_e2t_w: target values from equivalent surfaces with the equivalent kernel:
+// L2T (own DE surface with the downward density, fmm3d_mpi.cpp:159-202;
+// farPtr == nullptr) and M2T (UE surfaces of the leaf's W nodes with their
+// upward densities, fmm3d_mpi.cpp:208-249).  WPR warps a leaf.  M2T: 8, or 16
+// with fewer than 16 leaves an SM, which take the W nodes in turn.  L2T: one, four
+// leaves a CTA, or with fewer than 48 leaves an SM four, which split the surface.
+// A leaf beside a refined region has hundreds of W nodes and most have one or
+// two: one barrier-bound CTA of 128 threads a leaf ran as long as the longest
+// (Stokes, 60,007 points: 0.64 ms for 6.4 M pairs).  Lanes as in k_near_f64: PR
+// targets each, TG = ceil(targets / PR) a group, S = 32 / TG groups that split the
+// surface points.  The unit surface is staged for the CTA, a node's densities in
+// the warp's slice of shared memory; with WPR = 8 the warps' sums meet there in
+// warp order.  1M points M2T 0.67 -> 0.38 ms (8 warps a leaf 0.34), L2T 0.46 -> 0.41;
+// Stokes 60,007 points M2T 0.64 -> 0.29 ms (8 warps 0.40).
+constexpr int E2T_L2T_WARPS = 4;
+template <int KM>
+constexpr int e2t_targets() {
+  return KTraits<KM>::SD == 1 ? 4 : 2;
 }
-template <int KT>
-__global__ void __launch_bounds__(32 * P2PW_WARPS)
-    k_p2p_near_w(int tb, const int32_t* __restrict__ rows, const int64_t* __restrict__ ptr,
-                 const int32_t* __restrict__ idx, const int64_t* __restrict__ srcBeg,
-                 const int64_t* __restrict__ srcCnt, const int64_t* __restrict__ trgBeg,
-                 const int64_t* __restrict__ trgCnt, const double* __restrict__ src, const double* __restrict__ nrm,
-                 const double* __restrict__ den, const double* __restrict__ trg, double* __restrict__ val, double mu,
-                 double ve) {
-  constexpr int SD = KTraits<KT>::SD, TD = KTraits<KT>::TD, NRM = KTraits<KT>::NRM, PR = p2pw_targets<KT>();
-  constexpr int WS = P2PW_WARPS;
-  __shared__ double sPos[P2PW_WARPS][P2PW_CH * 3];
-  __shared__ double sNrm[P2PW_WARPS][NRM ? P2PW_CH * 3 : 1];
-  __shared__ double sDen[P2PW_WARPS][P2PW_CH * SD];
-  __shared__ int64_t eBeg[P2PW_WARPS][P2PW_MAXE];
-  __shared__ int32_t ePre[P2PW_WARPS][P2PW_MAXE + 1];
-  __shared__ double sRed[WS][32 * PR * TD];
+template <int KM, int WARPS>
+static size_t e2t_smem(int nSurf) {  // unit surface, densities or (same place) the warps' sums
+  const int sums = 32 * e2t_targets<KM>() * KTraits<KM>::TD;
+  return sizeof(double) * (3 * (size_t)nSurf + (size_t)WARPS * std::max(nSurf * KTraits<KM>::SD, sums));
+}
+template <int KM, int WARPS, int WPR>
+__global__ void __launch_bounds__(32 * WARPS)
+    k_e2t_w(int nRows, const int32_t* __restrict__ rows, const int64_t* __restrict__ farPtr,
+            const int32_t* __restrict__ farIdx, const double* __restrict__ ctr, const double* __restrict__ rad,
+            const double* __restrict__ sam, int nSurf, const double* __restrict__ dens,
+            const int64_t* __restrict__ trgBeg, const int64_t* __restrict__ trgCnt, const double* __restrict__ trg,
+            double* __restrict__ val, double mu, double ve) {
+  constexpr int SD = KTraits<KM>::SD, TD = KTraits<KM>::TD, PR = e2t_targets<KM>();
+  static_assert(WPR == 1 || WPR == WARPS, "a warp or the CTA a leaf");
+  extern __shared__ __align__(16) double e2t_sm[];
+  double* sSam = e2t_sm;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x;
+  const int slice = max(nSurf * SD, 32 * PR * TD);
+  double* sDen = e2t_sm + 3 * nSurf + (size_t)warp * slice;
+  for (int i = threadIdx.x; i < 3 * nSurf; i += blockDim.x) sSam[i] = sam[i];
+  __syncthreads();
+  const int row = blockIdx.x * (WARPS / WPR) + warp / WPR, sub = warp % WPR;
+  if (row >= nRows) return;  // WPR == 1 only: no CTA-wide barrier below then
   const int g = rows[row];
   const int64_t tBeg = trgBeg[g], tn = trgCnt[g];
-  const int64_t e0 = ptr[row], e1 = ptr[row + 1];
-  for (int64_t t0 = (int64_t)blockIdx.y * tb; t0 < tn; t0 += (int64_t)gridDim.y * tb) {
-    const int nt = (int)min((int64_t)tb, tn - t0);  // at most 32 PR
+  const int64_t f0 = farPtr ? farPtr[row] : 0, f1 = farPtr ? farPtr[row + 1] : 1;
+  for (int64_t t0 = 0; t0 < tn; t0 += 32 * PR) {
+    const int nt = (int)min((int64_t)(32 * PR), tn - t0);
     const int TG = (nt + PR - 1) / PR, S = 32 / TG;
     const int tl = lane % TG, sp = lane / TG;
-    double tx[PR], ty[PR], tz[PR], acc[PR][TD];
+    double px[PR], py[PR], pz[PR], acc[PR][TD];
 #pragma unroll
     for (int r = 0; r < PR; r++) {
       const int64_t t = tBeg + t0 + min(tl + r * TG, nt - 1);  // past the last: repeated, not stored
-      tx[r] = trg[3 * t];
-      ty[r] = trg[3 * t + 1];
-      tz[r] = trg[3 * t + 2];
+      px[r] = trg[3 * t];
+      py[r] = trg[3 * t + 1];
+      pz[r] = trg[3 * t + 2];
 #pragma unroll
       for (int c = 0; c < TD; c++) acc[r][c] = 0.0;
     }
-    for (int64_t ec = e0; ec < e1; ec += P2PW_MAXE) {
-      const int ne = (int)min((int64_t)P2PW_MAXE, e1 - ec);
+    // L2T's one surface: every warp of the leaf takes its share of the points
+    const int j0 = farPtr ? sp : sub * S + sp, js = farPtr ? S : WPR * S;
+    for (int64_t e = farPtr ? f0 + sub : f0; e < f1; e += WPR) {
+      const int node = farPtr ? farIdx[e] : g;
+      const double* d = dens + (int64_t)node * nSurf * SD;
       __syncwarp();
-      int running = 0;
-      for (int eb = 0; eb < ne; eb += 32) {
-        const int e = eb + lane;
-        int c = 0;
-        if (e < ne) {
-          const int s2 = idx[ec + e];
-          eBeg[warp][e] = srcBeg[s2];
-          c = (int)srcCnt[s2];
-        }
-        int incl = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += v;
-        }
-        if (e < ne) ePre[warp][e + 1] = running + incl;
-        running += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      if (lane == 0) ePre[warp][0] = 0;
+      for (int i = lane; i < nSurf * SD; i += 32) sDen[i] = d[i];
       __syncwarp();
-      const int total = running;
-      for (int base = warp * P2PW_CH; base < total; base += WS * P2PW_CH) {
-        const int cnt = min(P2PW_CH, total - base);
-        __syncwarp();
-        for (int i = lane; i < cnt; i += 32) {
-          const int j = base + i;
-          int lo = 0, hi = ne;
-          while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (ePre[warp][mid] <= j) lo = mid; else hi = mid;
-          }
-          const int64_t s2 = eBeg[warp][lo] + (j - ePre[warp][lo]);
-          sPos[warp][3 * i] = src[3 * s2];
-          sPos[warp][3 * i + 1] = src[3 * s2 + 1];
-          sPos[warp][3 * i + 2] = src[3 * s2 + 2];
-          if (NRM) {
-            sNrm[warp][3 * i] = nrm[3 * s2];
-            sNrm[warp][3 * i + 1] = nrm[3 * s2 + 1];
-            sNrm[warp][3 * i + 2] = nrm[3 * s2 + 2];
-          }
+      const double cx = ctr[3 * node], cy = ctr[3 * node + 1], cz = ctr[3 * node + 2], rr = rad[node];
+      if (sp < S) {
+        for (int j = j0; j < nSurf; j += js) {
+          const double qx = cx + rr * sSam[3 * j], qy = cy + rr * sSam[3 * j + 1], qz = cz + rr * sSam[3 * j + 2];
 #pragma unroll
-          for (int c = 0; c < SD; c++) sDen[warp][SD * i + c] = den[s2 * SD + c];
-        }
-        __syncwarp();
-        if (sp < S) {
-          for (int i = sp; i < cnt; i += S) {
-            const double qx = sPos[warp][3 * i], qy = sPos[warp][3 * i + 1], qz = sPos[warp][3 * i + 2];
-#pragma unroll
-            for (int r = 0; r < PR; r++)
-              kaccum<KT, double, double>(tx[r] - qx, ty[r] - qy, tz[r] - qz, NRM ? &sNrm[warp][3 * i] : nullptr,
-                                         &sDen[warp][SD * i], acc[r], mu, ve);
-          }
+          for (int r = 0; r < PR; r++)
+            kaccum<KM, double, double>(px[r] - qx, py[r] - qy, pz[r] - qz, nullptr, &sDen[SD * j], acc[r], mu, ve);
         }
       }
     }
@@ -191,97 +151,31 @@ __global__ void __launch_bounds__(32 * P2PW_WARPS)
         const double own = acc[r][c];
         for (int k = 1; k < S; k++) acc[r][c] += __shfl_sync(0xffffffffu, own, (lane + k * TG) & 31);
       }
-    if (sp == 0) {
+    if constexpr (WPR == 1) {
+      if (sp == 0) {
 #pragma unroll
-      for (int r = 0; r < PR; r++)
-        if (tl + r * TG < nt)
+        for (int r = 0; r < PR; r++)
+          if (tl + r * TG < nt)
 #pragma unroll
-          for (int c = 0; c < TD; c++) sRed[warp][(tl + r * TG) * TD + c] = acc[r][c];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nt * TD; i += blockDim.x) {
-      double s = 0.0;
-#pragma unroll
-      for (int w = 0; w < WS; w++) s += sRed[w][i];
-      val[(tBeg + t0) * TD + i] += s;
-    }
-    __syncthreads();
-  }
-}
-
-// k_e2t: target values from equivalent surfaces with the equivalent kernel:
-// the leaf's own DE surface with its downward density (L2T,
-// fmm3d_mpi.cpp:159-202) and the UE surfaces of its W nodes with their
-// upward densities (M2T, fmm3d_mpi.cpp:208-249).
-template <int KM>
-__global__ void __launch_bounds__(P2P_THREADS)
-    k_e2t(const int32_t* __restrict__ rows, const int64_t* __restrict__ farPtr, const int32_t* __restrict__ farIdx,
-          int useOwn, int useFar, const int32_t* __restrict__ depth, const double* __restrict__ ctr,
-          const double* __restrict__ rad, const double* __restrict__ samUE, int nUE,
-          const double* __restrict__ samDE, int nDE, const double* __restrict__ uden,
-          const double* __restrict__ dden, const int64_t* __restrict__ trgBeg, const int64_t* __restrict__ trgCnt,
-          const double* __restrict__ trg, double* __restrict__ val, double mu, double ve) {
-  constexpr int SD = KTraits<KM>::SD, TD = KTraits<KM>::TD;
-  __shared__ double sPos[P2P_TILE * 3];
-  __shared__ double sDen[P2P_TILE * SD];
-  __shared__ double sRed[P2P_THREADS * TD];
-  const int row = blockIdx.x;
-  const int g = rows[row];
-  const int64_t tb = trgBeg[g], tn = trgCnt[g];
-  const int tid = threadIdx.x;
-  const int TG = tn <= 32 ? 32 : (tn <= 64 ? 64 : 128);
-  const int S = P2P_THREADS / TG;
-  const int tl = tid % TG, sp = tid / TG;
-  const int own = (useOwn && depth[g] >= 2) ? 1 : 0;
-  const int64_t f0 = useFar ? farPtr[row] : 0, nf = useFar ? farPtr[row + 1] - f0 : 0;
-  for (int64_t t0 = 0; t0 < tn; t0 += TG) {
-    const int64_t t = t0 + tl;
-    const bool act = t < tn;
-    double tx = 0, ty = 0, tz = 0;
-    if (act) {
-      tx = trg[3 * (tb + t)];
-      ty = trg[3 * (tb + t) + 1];
-      tz = trg[3 * (tb + t) + 2];
-    }
-    double acc[TD];
-#pragma unroll
-    for (int c = 0; c < TD; c++) acc[c] = 0.0;
-    for (int64_t e = 0; e < own + nf; e++) {
-      const bool isOwn = e < own;
-      const int node = isOwn ? g : farIdx[f0 + e - own];
-      const double* sam = isOwn ? samDE : samUE;
-      const int ns = isOwn ? nDE : nUE;
-      const double* dsrc = isOwn ? dden + (int64_t)node * ns * SD : uden + (int64_t)node * ns * SD;
-      const double cx = ctr[3 * node], cy = ctr[3 * node + 1], cz = ctr[3 * node + 2], r = rad[node];
-      for (int base = 0; base < ns; base += P2P_TILE) {
-        const int cnt = min(P2P_TILE, ns - base);
-        __syncthreads();
-        for (int i = tid; i < cnt; i += P2P_THREADS) {
-          const int j = base + i;
-          sPos[3 * i] = cx + r * sam[3 * j];
-          sPos[3 * i + 1] = cy + r * sam[3 * j + 1];
-          sPos[3 * i + 2] = cz + r * sam[3 * j + 2];
-#pragma unroll
-          for (int c = 0; c < SD; c++) sDen[SD * i + c] = dsrc[(int64_t)j * SD + c];
-        }
-        __syncthreads();
-        if (act)
-          for (int i = sp; i < cnt; i += S)
-            kaccum<KM, double, double>(tx - sPos[3 * i], ty - sPos[3 * i + 1], tz - sPos[3 * i + 2], nullptr,
-                                       &sDen[SD * i], acc, mu, ve);
+            for (int c = 0; c < TD; c++) val[(tBeg + t0 + tl + r * TG) * TD + c] += acc[r][c];
       }
-    }
-    __syncthreads();
+    } else {
+      __syncwarp();  // the slice's densities have been read
+      if (sp == 0) {
 #pragma unroll
-    for (int c = 0; c < TD; c++) sRed[tid * TD + c] = acc[c];
-    __syncthreads();
-    if (sp == 0 && act) {
+        for (int r = 0; r < PR; r++)
+          if (tl + r * TG < nt)
 #pragma unroll
-      for (int c = 0; c < TD; c++) {
-        double s = 0;
-        for (int k = 0; k < S; k++) s += sRed[(tl + k * TG) * TD + c];
-        val[(tb + t) * TD + c] += s;
+            for (int c = 0; c < TD; c++) sDen[(tl + r * TG) * TD + c] = acc[r][c];
       }
+      __syncthreads();
+      for (int i = threadIdx.x; i < nt * TD; i += blockDim.x) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < WPR; w++) s += e2t_sm[3 * nSurf + (size_t)w * slice + i];
+        val[(tBeg + t0) * TD + i] += s;
+      }
+      __syncthreads();
     }
   }
 }
@@ -834,8 +728,9 @@ std::string dev_upload(const Plan& P, DevState& D, const double* src, const doub
             ijk.push_back(i | (j << 8) | (k << 16));
     FMMG_TRY(dput(D, D.surfIJK, ijk));
   }
-  D.maxLeafTrg = 0;
+  D.maxLeafTrg = D.maxLeafSrc = 0;
   for (int32_t g : P.evtrLeaves) D.maxLeafTrg = std::max(D.maxLeafTrg, P.trgCnt[g]);
+  for (int32_t g : P.s2mLeaves) D.maxLeafSrc = std::max(D.maxLeafSrc, P.srcCnt[g]);
   lap(0);
   // work lists
   FMMG_TRY(dput(D, D.evtrLeaves, P.evtrLeaves));
@@ -960,10 +855,8 @@ static void launch_near(const Plan& P, DevState& D, const int64_t* ptr, const in
                         cudaStream_t sn) {
   int n = (int)P.evtrLeaves.size();
   if (n == 0) return;
-  constexpr int TB = 16 * p2pw_targets<KT>();  // half the lanes' targets: the sources split in two at least
-  k_p2p_near_w<KT><<<dim3(n, near_blocks(D, TB)), 32 * P2PW_WARPS, 0, sn>>>(
-      TB, D.evtrLeaves, ptr, idx, D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt, D.src, D.nrm, D.den, D.trg, D.val,
-      P.o.coefs[0], P.o.coefs[1]);
+  launch_near_f64<NearP2P<KT>>(sn, n, D.maxLeafTrg, D.evtrLeaves, ptr, idx, D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt,
+                               D.src, D.nrm, D.den, D.trg, nullptr, nullptr, D.val, P.o.coefs[0], P.o.coefs[1]);
   if (ls) ls->launches++;
 }
 
@@ -978,22 +871,32 @@ static void launch_s2surf(const Plan& P, DevState& D, int nrows, const int32_t* 
   if (ls) ls->launches++;
 }
 
-static void launch_e2t(const Plan& P, DevState& D, int useOwn, int useFar, LaunchStats* ls, cudaStream_t se) {
+template <int KM, int WARPS, int WPR>
+static void launch_e2t_w(const Plan& P, DevState& D, bool far, int n, cudaStream_t se) {
+  const int nSurf = far ? P.nUE : P.nDE;
+  const size_t sm = e2t_smem<KM, WARPS>(nSurf);
+  auto* k = k_e2t_w<KM, WARPS, WPR>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k<<<(n + WARPS / WPR - 1) / (WARPS / WPR), 32 * WARPS, sm, se>>>(
+      n, far ? D.farLeaves : D.l2tLeaves, far ? D.farPtr : nullptr, D.farIdx, D.ctr, D.rad, D.sam[far ? 0 : 2], nSurf,
+      far ? D.uden : D.dden, D.trgBeg, D.trgCnt, D.trg, D.val, P.o.coefs[0], P.o.coefs[1]);
+}
+template <int KM>
+static void launch_e2t_km(const Plan& P, DevState& D, bool far, int n, cudaStream_t se) {
+  if (far && n < 16 * D.numSMs) launch_e2t_w<KM, 16, 16>(P, D, far, n, se);
+  else if (far) launch_e2t_w<KM, 8, 8>(P, D, far, n, se);
+  else if (n < 48 * D.numSMs) launch_e2t_w<KM, E2T_L2T_WARPS, E2T_L2T_WARPS>(P, D, far, n, se);
+  else launch_e2t_w<KM, E2T_L2T_WARPS, 1>(P, D, far, n, se);
+}
+
+static void launch_e2t(const Plan& P, DevState& D, bool far, LaunchStats* ls, cudaStream_t se) {
   // L2T runs over the leaves at depth >= 2, M2T over the leaves with W nodes
-  const int n = useFar ? (int)P.farLeaves.size() : (int)P.l2tLeaves.size();
-  const int32_t* rows = useFar ? D.farLeaves : D.l2tLeaves;
+  const int n = far ? (int)P.farLeaves.size() : (int)P.l2tLeaves.size();
   if (n == 0) return;
   switch (P.mm) {
-#define FMMG_E2T(KM)                                                                                          \
-  case KM:                                                                                                    \
-    k_e2t<KM><<<n, P2P_THREADS, 0, se>>>(rows, D.farPtr, D.farIdx, useOwn, useFar, D.depth, D.ctr, D.rad,       \
-                                               D.sam[0], P.nUE, D.sam[2], P.nDE, D.uden, D.dden, D.trgBeg,     \
-                                               D.trgCnt, D.trg, D.val, P.o.coefs[0], P.o.coefs[1]);            \
-    break;
-    FMMG_E2T(LAP_S_U)
-    FMMG_E2T(STK_F_U)
-    FMMG_E2T(NAV_S_U)
-#undef FMMG_E2T
+    case LAP_S_U: launch_e2t_km<LAP_S_U>(P, D, far, n, se); break;
+    case STK_F_U: launch_e2t_km<STK_F_U>(P, D, far, n, se); break;
+    case NAV_S_U: launch_e2t_km<NAV_S_U>(P, D, far, n, se); break;
   }
   if (ls) ls->launches++;
 }
@@ -1175,7 +1078,7 @@ static void run_stages(const Plan& P, DevState& D, int mask, LaunchStats* ls, bo
     cudaEventRecord(D.ev[EV_M2L_HAD], st);
   }
   cudaEventRecord(D.ev[EV_M2L_INV], st);
-  if ((mask & 8) && trgOut) launch_e2t(P, D, 0, 1, ls, sn);
+  if ((mask & 8) && trgOut) launch_e2t(P, D, true, ls, sn);
   if (ovl) cudaEventRecord(D.evSide, D.side);
   cudaEventRecord(D.ev[EV_M2T], st);
   if (mask & 16)
@@ -1195,7 +1098,7 @@ static void run_stages(const Plan& P, DevState& D, int mask, LaunchStats* ls, bo
   }
   cudaEventRecord(D.ev[EV_DN_GEMM], st);
   if (ovl) cudaStreamWaitEvent(st, D.evSide, 0);  // join before the last writer of the target values
-  if ((mask & 32) && trgOut) launch_e2t(P, D, 1, 0, ls, st);  // L2T
+  if ((mask & 32) && trgOut) launch_e2t(P, D, false, ls, st);  // L2T
   cudaEventRecord(D.ev[EV_L2T], st);
 }
 
