@@ -64,6 +64,7 @@ static void drop_graph(fmmg_handle* h) {
 }
 
 static fmmg_status fail(fmmg_handle* h, fmmg_status s, const std::string& msg) {
+  cudaGetLastError();  // reported now: a later call's check of its launches must not find it again
   if (h) h->err = msg;
   else g_create_err = msg;
   return s;

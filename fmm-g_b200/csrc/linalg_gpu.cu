@@ -15,10 +15,14 @@
 
 namespace fmmg {
 
-#define LG_CK(x)                                                                           \
-  do {                                                                                     \
-    cudaError_t e_ = (x);                                                                  \
-    if (e_ != cudaSuccess) return std::string("linalg device: ") + cudaGetErrorString(e_); \
+// (the host computes instead of a failed device run, so the error is taken here)
+#define LG_CK(x)                                                         \
+  do {                                                                   \
+    cudaError_t e_ = (x);                                                \
+    if (e_ != cudaSuccess) {                                             \
+      cudaGetLastError();                                                \
+      return std::string("linalg device: ") + cudaGetErrorString(e_);    \
+    }                                                                    \
   } while (0)
 
 // sqrt(1 + z^2) as the host computes it (jacobi_hyp1 in linalg.cpp)
