@@ -972,6 +972,7 @@ fmmg_status fmmg_operator(fmmg_handle* h, int which, int idx, double* get, const
   if (set) {
     h->opsDirty = true;
     h->tablesReplaced = true;
+    h->dev.opsHeld = false;  // a setup uploads them also where it keeps the blocks (after one that failed)
     if (which == 0 || which == 1) P.drop_folded_upward();
     try {
       if (which == 0 || which == 2) P.refactor_c2e(which);  // the FP32 pass applies the pinv factored

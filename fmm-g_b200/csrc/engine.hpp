@@ -160,7 +160,7 @@ struct DevState {
   std::vector<void*> opAllocs;
   std::vector<size_t> opAllocBytes;
   bool allocOps = false;
-  bool opsHeld = false;  // the FP64 tables are on the device
+  bool opsHeld = false;  // the plan's FP64 tables are on the device (cleared when the caller replaces one)
   struct Block {
     void* p;
     size_t bytes;

@@ -45,3 +45,45 @@ def test_setup_after_a_setup_out_of_memory():
     _fail_setup(f, rng)
     f.setup(x)
     assert np.array_equal(f.evaluate(den), want)
+
+
+def _outputs(f, den, w):
+    """FP64, mixed (2 right-hand sides) and transposed results of f."""
+    import torch
+    d = torch.from_numpy(den).cuda()
+    out = torch.zeros(2, f.nt * f.td, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    f.evaluate_device(d, out, 2, fmmg.PREC_MIXED)
+    f.sync()
+    return {"fp64": f.evaluate(den[0]), "mixed": out.cpu().numpy(), "adjoint": f.adjoint(w)[0]}
+
+
+def _inputs(kt, n, rng):
+    x, den = rng.random((n, 3)), rng.normal(size=(2, n * fmmg.KERNELS[kt][0]))
+    return x, den, rng.normal(size=n * fmmg.KERNELS[kt][1])
+
+
+# both forms of a handle run the same kernels on the same tables, so the
+# results are the same bit for bit but for the mixed form's split-K sums, which
+# run in one order too
+@pytest.mark.parametrize("kt", [111, 311])
+@pytest.mark.parametrize("when", ["evaluated", "not evaluated"])
+def test_replaced_table_after_a_failed_setup(kt, when):
+    """A table replaced between a setup that failed and the next one is the one
+    that the next setup's evaluates use, as on a fresh handle."""
+    rng = np.random.default_rng(SEED + kt)
+    x, den, w = _inputs(kt, 3000, rng)
+    f = fmmg.FMM3d(kt, np_=4, pts_max=40)
+    f.setup(x)
+    if when == "evaluated":
+        _outputs(f, den, w)
+    _fail_setup(f, rng)
+    g = fmmg.FMM3d(kt, np_=4, pts_max=40)
+    for h in (f, g):
+        h.set_operator(2, 0, h.operator(2, 0) * 1.5)
+        for i in range(0, 316, 5):
+            h.set_operator(4, i, h.operator(4, i) * 0.75)
+        h.setup(x)
+    got, want = _outputs(f, den, w), _outputs(g, den, w)
+    for key in want:
+        assert np.array_equal(got[key], want[key]), key
