@@ -646,6 +646,10 @@ static std::string hv_layout(const Plan& P, DevState& D) {
 
 std::string dev_upload_operators(const Plan& P, DevState& D) {
   FMMG_CK(cudaSetDevice(D.device));
+  // the tables are overwritten in place by the legacy stream, which does not
+  // wait for the handle's: evaluates already queued read the old ones
+  FMMG_CK(cudaStreamSynchronize(D.stream));
+  if (D.side) FMMG_CK(cudaStreamSynchronize(D.side));
   OpBlocks scope(D);
   auto put = [&](double*& dst, const std::vector<double>& v) -> std::string {
     if (!dst) return dput(D, dst, v);

@@ -87,3 +87,40 @@ def test_replaced_table_after_a_failed_setup(kt, when):
     got, want = _outputs(f, den, w), _outputs(g, den, w)
     for key in want:
         assert np.array_equal(got[key], want[key]), key
+
+
+@pytest.mark.parametrize("kt,form", [(111, fmmg.PREC_FP64), (311, fmmg.PREC_FP64), (311, fmmg.PREC_MIXED)])
+def test_replaced_table_waits_for_queued_evaluates(kt, form):
+    """evaluate_device only queues work: tables replaced right after it serve the
+    calls that follow and not the ones that still run (several milliseconds of
+    them), down to the last bit."""
+    import torch
+    rng = np.random.default_rng(SEED)
+    n, calls = 100000, 6
+    st = torch.cuda.Stream()
+    f = fmmg.FMM3d(kt, np_=4, pts_max=40, stream=st.cuda_stream)
+    f.setup(rng.random((n, 3)))
+    den = torch.from_numpy(rng.normal(size=n * f.sd)).cuda()
+    out = torch.zeros(calls + 1, n * f.td, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    tables = [f.operator(4, i) for i in range(0, 316, 7)]
+    values = {}
+    for scale in (1.0, 0.5):
+        for j, i in enumerate(range(0, 316, 7)):
+            f.set_operator(4, i, tables[j] * scale)
+        f.evaluate_device(den, out[0], 1, form)
+        f.sync()
+        values[scale] = out[0].cpu().numpy()
+    now = 0.5
+    for scale in (1.0, 0.5, 1.0):
+        for c in range(calls):
+            f.evaluate_device(den, out[c], 1, form)
+        for j, i in enumerate(range(0, 316, 7)):
+            f.set_operator(4, i, tables[j] * scale)
+        f.evaluate_device(den, out[calls], 1, form)
+        f.sync()
+        got = out.cpu().numpy()
+        for c in range(calls):
+            assert np.array_equal(got[c], values[now])
+        assert np.array_equal(got[calls], values[scale])
+        now = scale
