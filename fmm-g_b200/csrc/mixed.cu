@@ -30,7 +30,6 @@
 #include "had_smem.cuh"
 #include "had_vec.cuh"
 #include "kernels.hpp"
-#include "plan_pool.cuh"
 
 namespace fmmg {
 
@@ -1221,6 +1220,29 @@ static std::vector<double> pad_cols(const std::vector<double>& F, int m, int k) 
   return r;
 }
 
+// The operator layout's device staging, up to a few hundred MB once a handle:
+// given back at its end, when the stream has drained, on an error's return too.
+struct OpStaging {
+  cudaStream_t st;
+  std::vector<void*> held;
+  explicit OpStaging(cudaStream_t s) : st(s) {}
+  ~OpStaging() {
+    cudaStreamSynchronize(st);
+    for (void* p : held) cudaFree(p);
+  }
+  OpStaging(const OpStaging&) = delete;
+  OpStaging& operator=(const OpStaging&) = delete;
+  template <typename T>
+  std::string get(T*& p, size_t n) {
+    void* q = nullptr;
+    cudaError_t e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
+    if (e != cudaSuccess) return std::string("cudaMalloc: ") + cudaGetErrorString(e);
+    held.push_back(q);
+    p = (T*)q;
+    return std::string();
+  }
+};
+
 // t[o][j][c] = l2l[(o dc + c) de + j]: the transposes of L2L's 8 octant blocks
 static __global__ void k_l2l_blocks_t(int64_t n, int dc, int de, const double* __restrict__ l2l,
                                       double* __restrict__ t) {
@@ -1241,12 +1263,12 @@ static __global__ void k_iota(int n, int32_t* p) {
 // level, G = C2E x L2L (8 de x de, formed here in FP64).  As for the upward
 // fold the product's norm is O(1) where the pseudo-inverse's is ~1e6, so it
 // loses nothing in FP32 (the L2L part no longer passes the inverse in FP32).
-static std::string dn_fold(const Plan& P, DevState& D, double* G, PlanBufs& tmp) {
+static std::string dn_fold(const Plan& P, DevState& D, double* G, OpStaging& tmp) {
   const int de = P.nDE * P.sdm, dc = P.nDC * P.tdm;
   double* lt = nullptr;
   int32_t* iota = nullptr;
-  FMMG_CK(tmp.get(lt, (size_t)8 * de * dc));
-  FMMG_CK(tmp.get(iota, (size_t)de));
+  FMMG_TRY(tmp.get(lt, (size_t)8 * de * dc));
+  FMMG_TRY(tmp.get(iota, (size_t)de));
   const int64_t n = (int64_t)8 * de * dc;
   k_l2l_blocks_t<<<(unsigned)((n + 255) / 256), 256, 0, D.stream>>>(n, dc, de, D.l2l, lt);
   k_iota<<<(de + 255) / 256, 256, 0, D.stream>>>(de, iota);
@@ -1402,12 +1424,11 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     // rank that is a multiple of 4 (zero rows of F1, zero columns of F2), so the
     // intermediate rows allow 16-byte tile fetches
     auto alloc = [&](float*& p, size_t n) { return dalloc(D, p, n); };
-    PlanBufs tmp;
-    tmp.device = D.device;
+    OpStaging tmp(D.stream);
     auto prep = [&](TcOp& op, DevState::OpT& wt, float* plain, const std::vector<double>& W, int n,
                     int k) -> std::string {
       double* dW = nullptr;
-      FMMG_CK(tmp.get(dW, W.size()));
+      FMMG_TRY(tmp.get(dW, W.size()));
       FMMG_CK(cudaMemcpyAsync(dW, W.data(), W.size() * sizeof(double), cudaMemcpyHostToDevice, D.stream));
       return prepare_operator(D.stream, op, wt, plain, dW, n, k, alloc);
     };
@@ -1424,10 +1445,9 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     FMMG_TRY(prep(D.cM2MUp, D.tM2MUp, D.m2mUp32, fold, (int)ue, (int)(8 * ue)));
     // the parent's part of a child's downward density: C2E down x L2L
     double* G = nullptr;
-    FMMG_CK(tmp.get(G, 8 * de * de));
+    FMMG_TRY(tmp.get(G, 8 * de * de));
     FMMG_TRY(dn_fold(P, D, G, tmp));
     FMMG_TRY(prepare_operator(D.stream, D.cDnFold, D.tDnFold, D.dnFold32, G, (int)(8 * de), (int)de, alloc));
-    FMMG_CK(cudaStreamSynchronize(D.stream));  // tmp's blocks go back to the pool
     std::vector<float2> t(P.m2lT32.size());
     for (size_t i = 0; i < t.size(); i++) t[i] = make_float2((float)P.m2lT32[i].real(), (float)P.m2lT32[i].imag());
     FMMG_CK(cudaMemcpyAsync(D.m2lT32, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice, D.stream));

@@ -124,3 +124,26 @@ def test_replaced_table_waits_for_queued_evaluates(kt, form):
             assert np.array_equal(got[c], values[now])
         assert np.array_equal(got[calls], values[scale])
         now = scale
+
+
+def test_mixed_staging_is_given_back():
+    """What a handle's first mixed call stages on the device (some 300 MB of FP64
+    operators for Navier at np = 8) does not stay with the process."""
+    import torch
+    rng = np.random.default_rng(SEED)
+    x, den, w = _inputs(511, 500, rng)
+
+    def free_after(mixed):
+        f = fmmg.FMM3d(511, np_=8, pts_max=40, coefs=(1.0, 0.3))
+        f.setup(x)
+        f.evaluate(den[0])
+        if mixed:
+            _outputs(f, den, w)
+        f.close()
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info()[0]
+
+    free_after(False)
+    before = free_after(False)
+    free_after(True)  # the kernels' code
+    assert free_after(True) >= before - 64 * MB
