@@ -1365,13 +1365,11 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     std::vector<int4> items;
     std::vector<int32_t> sl, sb, sc;
     m2t_items(P, D.numSMs, items, sl, sb, sc, D.m2tPartTargets);
-    FMMG_TRY(dalloc(D, D.m2tItems, items.size()));
-    FMMG_CK(cudaMemcpyAsync(D.m2tItems, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, D.stream));
     D.nM2tItems = (int)items.size();
     D.nM2tSplit = (int)sl.size();
-    auto put = [&](int32_t*& dst, const std::vector<int32_t>& v) -> std::string {
+    auto put = [&](auto*& dst, const auto& v) -> std::string {
       FMMG_TRY(dalloc(D, dst, v.size()));
-      FMMG_CK(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(int32_t), cudaMemcpyHostToDevice, D.stream));
+      FMMG_CK(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, D.stream));
       return std::string();
     };
     if (!sl.empty()) {
@@ -1379,6 +1377,7 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
       FMMG_TRY(put(D.m2tSplitBase, sb));
       FMMG_TRY(put(D.m2tSplitCnt, sc));
     }
+    FMMG_TRY(put(D.m2tItems, items));  // last: its pointer says that all four are there
   }
   // rank-sized buffers take the largest rank a pinv can have, so factors
   // recomputed for a replaced table (Plan::refactor_c2e) always fit
@@ -1404,17 +1403,16 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     FMMG_TRY(dalloc(D, D.den32, kc8 * P.ns * P.sd));
     FMMG_TRY(dalloc(D, D.valK, (size_t)kc * std::max<int64_t>(P.nt, 1) * P.td));
     FMMG_TRY(dalloc(D, D.m2tPart, (size_t)kc * std::max<int64_t>(D.m2tPartTargets, 1) * P.tdm));
-    if (!D.dnFold32) {
-      OpBlocks scope(D);
-      FMMG_TRY(dalloc(D, D.dnFold32, 8 * de * de));
-      FMMG_TRY(dalloc(D, D.m2lT32, P.m2lT32.size()));
-      if (P.sdm == 1 && P.tdm == 1) FMMG_TRY(dalloc(D, D.m2lTw32, (size_t)27 * 27 * P.nEff32));
-      FMMG_TRY(dalloc(D, D.upF1, (size_t)kUpMax * uc));
-      FMMG_TRY(dalloc(D, D.upF2, ue * kUpMax));
-      FMMG_TRY(dalloc(D, D.dnF1, (size_t)kDnMax * dc));
-      FMMG_TRY(dalloc(D, D.dnF2, de * kDnMax));
-      FMMG_TRY(dalloc(D, D.m2mUp32, ue * 8 * ue));
-    }
+    OpBlocks scope(D);
+    auto need = [&](auto*& p, size_t n) { return p ? std::string() : dalloc(D, p, n); };  // kept where held
+    FMMG_TRY(need(D.dnFold32, 8 * de * de));
+    FMMG_TRY(need(D.m2lT32, P.m2lT32.size()));
+    if (P.sdm == 1 && P.tdm == 1) FMMG_TRY(need(D.m2lTw32, (size_t)27 * 27 * P.nEff32));
+    FMMG_TRY(need(D.upF1, (size_t)kUpMax * uc));
+    FMMG_TRY(need(D.upF2, ue * kUpMax));
+    FMMG_TRY(need(D.dnF1, (size_t)kDnMax * dc));
+    FMMG_TRY(need(D.dnF2, de * kDnMax));
+    FMMG_TRY(need(D.m2mUp32, ue * 8 * ue));
     D.mixedReady = true;
     D.mixedK = kc;
   }

@@ -1228,6 +1228,7 @@ std::string dev_dense(const Plan& P, DevState& D, const double* dDen, int64_t nc
   cudaStream_t st = D.stream;
   if ((size_t)nchk > D.chkCap) {
     size_t cap = (size_t)std::max<int64_t>(nchk, 1024);
+    D.chkCap = 0;
     FMMG_TRY(dput<double>(D, D.chkPos, nullptr, 3 * cap));
     FMMG_TRY(dput<double>(D, D.chkOut, nullptr, 3 * cap));
     D.chkCap = cap;

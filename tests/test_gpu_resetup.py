@@ -147,3 +147,33 @@ def test_mixed_staging_is_given_back():
     before = free_after(False)
     free_after(True)  # the kernels' code
     assert free_after(True) >= before - 64 * MB
+
+
+@pytest.mark.parametrize("kt", [111, 311])
+def test_mixed_call_after_mixed_calls_out_of_memory(kt):
+    """First mixed calls that run out of device memory at any of their
+    allocations are refused, and the next call of the handle with the memory
+    back is the fresh handle's."""
+    rng = np.random.default_rng(SEED + kt)
+    x, den, w = _inputs(kt, 2000, rng)
+    x[::2] *= 0.1  # a corner refined deeper: W lists
+    g = fmmg.FMM3d(kt, np_=6, pts_max=40)
+    g.setup(x)
+    want = _outputs(g, den, w)
+    refused = 0
+    f = fmmg.FMM3d(kt, np_=6, pts_max=40)
+    f.setup(x)
+    f.set_precision(fmmg.PREC_MIXED)
+    for leave in list(range(2, 40, 6)) + list(range(40, 200, 20)):
+        with _little_memory(leave * MB):
+            try:
+                assert rel_l2(f.evaluate(den[0]), want["mixed"][0]) <= 1e-5
+            except fmmg.FmmgError:
+                refused += 1
+        if leave % 4 == 0:  # a new setup keeps the operator tables' blocks that were allocated
+            f.setup(x)
+    assert refused >= 3
+    f.set_precision(fmmg.PREC_FP64)
+    got = _outputs(f, den, w)
+    for key in want:
+        assert np.array_equal(got[key], want[key]), key
