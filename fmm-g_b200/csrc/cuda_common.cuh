@@ -42,6 +42,9 @@ inline Scale4 unit_scale() {
   return s;
 }
 
+// points of the largest order's equivalent surface, 6 (np - 1)^2 + 2 at np = 8
+constexpr int MAX_SURF = 296;
+
 // (2np)^3 grid of the spectral M2L: N points per axis, NH kept x frequencies,
 // the np^3 lattice sits at offset H = np/2 (matmgnt3d_mpi.cpp:321)
 template <int NP>

@@ -1753,8 +1753,12 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
         ls->launches++;
       }
     } else {
-      const size_t smem = (size_t)P.nDE * sizeof(float4) + (size_t)L2T_WARPS * P.nDE * KB * P.sdm * sizeof(float);
-      cudaFuncSetAttribute(k_l2t32w<KM, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      auto bytes = [&](int nSurf) {
+        return (size_t)nSurf * sizeof(float4) + (size_t)L2T_WARPS * nSurf * KB * P.sdm * sizeof(float);
+      };
+      const size_t smem = bytes(P.nDE);
+      cudaFuncSetAttribute(k_l2t32w<KM, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)bytes(MAX_SURF));  // of any order: see launch_e2t_w
       k_l2t32w<KM, KB><<<dim3((nr + L2T_WARPS - 1) / L2T_WARPS, kb), 32 * L2T_WARPS, smem, se>>>(
           nr, rows, D.ctr, D.rad, D.sam[2], P.nDE, D.dden32, nn * de, D.trgBeg, D.trgCnt, D.trg, D.valK, valStride,
           kc, mu, ve);

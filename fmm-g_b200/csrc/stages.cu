@@ -924,7 +924,9 @@ static void launch_e2t_w(const Plan& P, DevState& D, bool far, int n, cudaStream
   const int nSurf = far ? P.nUE : P.nDE;
   const size_t sm = e2t_smem<KM, WARPS>(nSurf);
   auto* k = k_e2t_w<KM, WARPS, WPR>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  // the largest order's: the attribute is the function's, and another thread's
+  // handle of a lower order would set a smaller one between this and the launch
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e2t_smem<KM, WARPS>(MAX_SURF));
   k<<<(n + WARPS / WPR - 1) / (WARPS / WPR), 32 * WARPS, sm, se>>>(
       n, far ? D.farLeaves : D.l2tLeaves, far ? D.farPtr : nullptr, D.farIdx, D.ctr, D.rad, D.sam[far ? 0 : 2], nSurf,
       far ? D.uden : D.dden, D.trgBeg, D.trgCnt, D.trg, D.val, P.o.coefs[0], P.o.coefs[1]);
