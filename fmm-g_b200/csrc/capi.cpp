@@ -227,28 +227,27 @@ fmmg_status fmmg_setup(fmmg_handle* h, int64_t ns, const double* src, const doub
   if (nrm && !finite(nrm, 3 * ns)) return fail(h, FMMG_INVALID_ARG, "a normal is not finite");
   try {
     if (h->setupDone) {
+      fmmg::Plan fresh;
+      fresh.o = h->opt;
+      if (h->tablesReplaced) {  // back to the built tables; until they are there the handle stays as it is
+        fmmg::LinalgDeviceScope scope(h->hostOnly ? -1 : h->device);
+        std::string e = fresh.build_operators();
+        if (!e.empty()) return fail(h, FMMG_NOT_SUPPORTED, e);
+      }
       drop_graph(h);
       // the blocks of this setup serve the next one (dev_alloc), and what is
       // left over is freed at its end; the operator tables stay on the device
       // unless the caller replaced some
       fmmg::dev_release_for_reuse(h->dev, !h->tablesReplaced && !h->opsDirty);
+      h->setupDone = false;
       h->dDenIO = h->dValIO = nullptr;
       h->dDenK = h->dValK = nullptr;
       h->dAdjW = h->dAdjG = h->dAdjGrad = h->dAdjDen = nullptr;
       h->adjK = 0;
       h->ioK = 0;
-      fmmg::Plan fresh;
-      fresh.o = h->opt;
-      if (h->tablesReplaced) {  // back to the built tables
-        fmmg::LinalgDeviceScope scope(h->hostOnly ? -1 : h->device);
-        std::string e = fresh.build_operators();
-        if (!e.empty()) return fail(h, FMMG_NOT_SUPPORTED, e);
-      } else {
-        fresh.take_operators(std::move(h->plan));  // the handle's own, never replaced
-      }
+      if (!h->tablesReplaced) fresh.take_operators(std::move(h->plan));  // the handle's own, never replaced
       h->plan = std::move(fresh);
       h->tablesReplaced = false;
-      h->setupDone = false;
     }
     lap(0);
     std::string e = h->plan.build(h->opt, ns, src, nrm, nt, nt > 0 ? trg : src,

@@ -177,3 +177,30 @@ def test_mixed_call_after_mixed_calls_out_of_memory(kt):
     got = _outputs(f, den, w)
     for key in want:
         assert np.array_equal(got[key], want[key]), key
+
+
+def test_setup_out_of_host_memory_leaves_the_handle_as_it_was():
+    """A new setup that cannot hold the built tables again (host memory) is
+    refused before it gives up anything: the handle still evaluates, on its
+    replaced tables, and the next setup works."""
+    import resource
+    rng = np.random.default_rng(SEED)
+    x, den, w = _inputs(311, 2000, rng)
+    f = fmmg.FMM3d(311, np_=6, pts_max=40)
+    f.setup(x)
+    built = f.evaluate(den[0])
+    f.set_operator(3, 2, f.operator(3, 2) * 1.5)
+    want = _outputs(f, den, w)
+    old = resource.getrlimit(resource.RLIMIT_AS)
+    resource.setrlimit(resource.RLIMIT_AS, (1 << 20, old[1]))  # no further mappings: the tables take 46 MB
+    try:
+        with pytest.raises(fmmg.FmmgError) as e:
+            f.setup(x)
+    finally:
+        resource.setrlimit(resource.RLIMIT_AS, old)
+    assert e.value.status == fmmg.FMMG_OOM
+    got = _outputs(f, den, w)
+    for key in want:
+        assert np.array_equal(got[key], want[key]), key
+    f.setup(x)
+    assert np.array_equal(f.evaluate(den[0]), built)
