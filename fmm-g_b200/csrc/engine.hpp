@@ -73,6 +73,7 @@ struct DevState {
   // and whether their 3 x 3 parts are symmetric
   double2* hvT = nullptr;
   float2* hvT32 = nullptr;
+  size_t hvTCap = 0, hvT32Cap = 0;  // values allocated
   bool hvSym = true, hvSymOf64 = true, hvSymOf32 = true;  // of the tables; of the layouts held
   int16_t* transIdDev = nullptr;  // (rx+3)*49+(ry+3)*7+(rz+3) -> translation 0..315 or -1
   // per-evaluate work arrays

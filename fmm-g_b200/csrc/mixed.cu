@@ -1329,10 +1329,11 @@ static void m2t_items(const Plan& P, int numSMs, std::vector<int4>& items, std::
 // where the FP64 tables are symmetric (D.hvSym)
 template <int SDM, int TDM>
 static std::string hv_layout32(const Plan& P, DevState& D) {
-  if (!D.hvT32 || D.hvSymOf32 != D.hvSym) {
-    const int64_t n = D.hvSym ? hv_table_size<float2, SDM, TDM, true>(P.nEff32)
-                              : hv_table_size<float2, SDM, TDM, false>(P.nEff32);
-    FMMG_TRY(dalloc(D, D.hvT32, (size_t)n));
+  const size_t n = (size_t)(D.hvSym ? hv_table_size<float2, SDM, TDM, true>(P.nEff32)
+                                    : hv_table_size<float2, SDM, TDM, false>(P.nEff32));
+  if (n > D.hvT32Cap) {
+    FMMG_TRY(dalloc(D, D.hvT32, n));
+    D.hvT32Cap = n;
   }
   D.hvSymOf32 = D.hvSym;
   if (D.hvSym) launch_hv_pack<float2, SDM, TDM, true>(D.stream, D.m2lT32, D.transIdDev, P.nEff32, D.hvT32);

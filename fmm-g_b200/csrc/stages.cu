@@ -567,6 +567,7 @@ static void dev_clear_ops(DevState& D) {
   D.transIdDev = nullptr;
   D.hvT = nullptr;
   D.hvT32 = nullptr;
+  D.hvTCap = D.hvT32Cap = 0;
   D.m2lT32 = nullptr;
   D.m2lTw32 = nullptr;
   D.uc2ueT = D.m2mT = D.dc2deT = D.l2lT = nullptr;
@@ -631,10 +632,12 @@ static std::string hv_layout(const Plan& P, DevState& D) {
   k_hv_asym<double2, SDM, TDM><<<316, 256>>>(D.m2lT, P.nEff, 64 * 2.2e-16, dFlag);
   FMMG_CK(cudaMemcpy(&flag, dFlag, sizeof(int), cudaMemcpyDeviceToHost));
   D.hvSym = flag == 0;
-  if (!D.hvT || D.hvSymOf64 != D.hvSym) {
-    const int64_t n = D.hvSym ? hv_table_size<double2, SDM, TDM, true>(P.nEff)
-                              : hv_table_size<double2, SDM, TDM, false>(P.nEff);
-    FMMG_TRY(dput<double2>(D, D.hvT, nullptr, (size_t)n));
+  const size_t n = (size_t)(D.hvSym ? hv_table_size<double2, SDM, TDM, true>(P.nEff)
+                                    : hv_table_size<double2, SDM, TDM, false>(P.nEff));
+  if (n > D.hvTCap) {  // replaced tables change the layout in the larger one's block
+    D.hvTCap = 0;
+    FMMG_TRY(dput<double2>(D, D.hvT, nullptr, n));
+    D.hvTCap = n;
   }
   D.hvSymOf64 = D.hvSym;
   if (D.hvSym) launch_hv_pack<double2, SDM, TDM, true>(0, D.m2lT, D.transIdDev, P.nEff, D.hvT);

@@ -204,3 +204,24 @@ def test_setup_out_of_host_memory_leaves_the_handle_as_it_was():
         assert np.array_equal(got[key], want[key]), key
     f.setup(x)
     assert np.array_equal(f.evaluate(den[0]), built)
+
+
+def test_translation_layouts_change_in_place():
+    """Tables replaced back and forth between symmetric and general 3 x 3 blocks
+    take no more device memory each time (77 and 112 MB in FP64 at np = 7) than
+    the first."""
+    import torch
+    rng = np.random.default_rng(SEED)
+    x, den, w = _inputs(311, 500, rng)
+    f = fmmg.FMM3d(311, np_=7, pts_max=40)
+    f.setup(x)
+    table = f.operator(4, 0)
+    general = (table.reshape(-1, 12, 2) * np.linspace(1.0, 1.1, 12)[None, :, None]).ravel()
+    free = []
+    for _ in range(4):
+        for t in (general, table):
+            f.set_operator(4, 0, t)
+            _outputs(f, den, w)
+        torch.cuda.empty_cache()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[-1] >= free[0] - 16 * MB
