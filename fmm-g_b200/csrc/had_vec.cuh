@@ -79,19 +79,21 @@ constexpr size_t hv_smem_bytes() {
 }
 
 // flag[0] |= 1 where the 3 x 3 part of a translation is not symmetric to
-// rounding (tol times its largest value over the frequencies); one CTA each
+// rounding (tol times its largest value over the frequencies) or holds a value
+// that is not finite; one CTA each
 template <typename C, int SDM, int TDM>
 __global__ void __launch_bounds__(256) k_hv_asym(const C* __restrict__ T, int nEff, double tol, int* flag) {
   __shared__ double sMax[256], sDif[256];
   const C* Ti = T + (int64_t)blockIdx.x * nEff * SDM * TDM;
   double mx = 0, df = 0;
+  bool bad = false;
   for (int f = threadIdx.x; f < nEff; f += blockDim.x)
     for (int s = 0; s < 3; s++)
       for (int t = 0; t < 3; t++) {
         const C a = Ti[(int64_t)f * SDM * TDM + s * TDM + t], b = Ti[(int64_t)f * SDM * TDM + t * TDM + s];
         mx = fmax(mx, fmax(fabs((double)a.x), fabs((double)a.y)));
-        const double d = fmax(fabs((double)a.x - b.x), fabs((double)a.y - b.y));
-        if (!(d <= df)) df = d;  // a NaN stays
+        df = fmax(df, fmax(fabs((double)a.x - b.x), fabs((double)a.y - b.y)));
+        bad |= !isfinite(a.x) || !isfinite(a.y);
       }
   sMax[threadIdx.x] = mx;
   sDif[threadIdx.x] = df;
@@ -99,10 +101,11 @@ __global__ void __launch_bounds__(256) k_hv_asym(const C* __restrict__ T, int nE
   if (threadIdx.x == 0) {
     for (int i = 1; i < 256; i++) {
       mx = fmax(mx, sMax[i]);
-      if (!(sDif[i] <= df)) df = sDif[i];
+      df = fmax(df, sDif[i]);
     }
-    if (!(df <= tol * mx)) atomicOr(flag, 1);
+    if (df > tol * mx) atomicOr(flag, 1);
   }
+  if (bad) atomicOr(flag, 1);
 }
 
 // T [316][nEff][s][t] -> out [slice of FW frequencies][343 positions][rows][FW]
