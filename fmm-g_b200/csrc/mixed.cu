@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(32 * NX_WARPS)
       if (lane == 0) ePre[warp][0] = 0;
       __syncwarp();
       const int total = running;
-      // FP32 partial sums over up to 128 sources of the warp, then FP64
+      // FP32 partial sums over up to 64 sources of the warp (a lane's 64 / S), then FP64
       float part[NX_R][NA];
       for (int base = sub * NX_CH, round = 0; base < total; base += WS * NX_CH, round++) {
         const int cnt = min(NX_CH, total - base);
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(32 * NX_WARPS)
           for (int r = 0; r < KB * SD; r++) sDen[warp][i * KB * SD + r] = ds[r];
         }
         __syncwarp();
-        if ((round & 3) == 0) {
+        if ((round & 1) == 0) {
 #pragma unroll
           for (int r = 0; r < NX_R; r++)
 #pragma unroll
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(32 * NX_WARPS)
             }
           }
         }
-        if ((round & 3) == 3 || base + WS * NX_CH >= total) {
+        if ((round & 1) == 1 || base + WS * NX_CH >= total) {
 #pragma unroll
           for (int r = 0; r < NX_R; r++)
 #pragma unroll
