@@ -285,13 +285,7 @@ __global__ void __launch_bounds__(32 * NX_WARPS)
         }
       }
     }
-#pragma unroll
-    for (int r = 0; r < NX_R; r++)
-#pragma unroll
-      for (int c = 0; c < NA; c++) {
-        const double own = acc[r][c];
-        for (int k = 1; k < S; k++) acc[r][c] += __shfl_sync(0xffffffffu, own, (lane + k * TG) & 31);
-      }
+    group_sum(acc, lane, sp, TG, S);
     auto store = [&]() {
 #pragma unroll
       for (int r = 0; r < NX_R; r++) {
@@ -505,14 +499,7 @@ __global__ void __launch_bounds__(32 * NW_WARPS, 6)
         }
       }
     }
-#pragma unroll
-    for (int r = 0; r < KB; r++) {
-      const double a = acc[0][r], b = acc[1][r];
-      for (int k = 1; k < S; k++) {
-        acc[0][r] += __shfl_sync(0xffffffffu, a, (lane + k * TG) & 31);
-        acc[1][r] += __shfl_sync(0xffffffffu, b, (lane + k * TG) & 31);
-      }
-    }
+    group_sum(acc, lane, sp, TG, S);
     if constexpr (WS > 1) {  // the warps' sums meet in the first one, in warp order
       for (int w = 1; w < WS; w++) {
         __syncthreads();

@@ -144,13 +144,7 @@ __global__ void __launch_bounds__(32 * WARPS)
         }
       }
     }
-#pragma unroll
-    for (int r = 0; r < PR; r++)
-#pragma unroll
-      for (int c = 0; c < TD; c++) {
-        const double own = acc[r][c];
-        for (int k = 1; k < S; k++) acc[r][c] += __shfl_sync(0xffffffffu, own, (lane + k * TG) & 31);
-      }
+    group_sum(acc, lane, sp, TG, S);
     if constexpr (WPR == 1) {
       if (sp == 0) {
 #pragma unroll
