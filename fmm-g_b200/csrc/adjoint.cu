@@ -526,9 +526,9 @@ static void run_adjoint(const Plan& P, DevState& D, int& launches) {
   }
   // near field, transposed: targets -> sources of the U, direct W and direct X leaves
   if (!P.adjNearRows.empty()) {
-    launch_near_f64<NearP2PT<KT>>(st, (int)P.adjNearRows.size(), D.maxLeafSrc, D.adjNearRows, D.adjNearPtr,
-                                  D.adjNearIdx, D.trgBeg, D.trgCnt, D.srcBeg, D.srcCnt, D.trg, nullptr, w, D.src, D.nrm,
-                                  nullptr, g, mu, ve);
+    launch_near_f64<NearP2PT<KT>>(st, D.numSMs, (int)P.adjNearRows.size(), D.maxLeafSrc, P.nt, D.adjNearRows,
+                                  D.adjNearPtr, D.adjNearIdx, D.trgBeg, D.trgCnt, D.srcBeg, D.srcCnt, D.trg, nullptr, w,
+                                  D.src, D.nrm, nullptr, g, mu, ve);
     launches++;
   }
   // upward, transposed: C2E^T then M2M^T per level, root side first (nothing
@@ -561,9 +561,9 @@ template <int KT>
 static void run_target_grad(const Plan& P, DevState& D, int& launches) {
   cudaStream_t st = D.stream;
   if (!P.evtrLeaves.empty()) {
-    launch_near_f64<NearGrad<KT>>(st, (int)P.evtrLeaves.size(), D.maxLeafTrg, D.evtrLeaves, D.nearPtr, D.nearIdx,
-                                  D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt, D.src, D.nrm, D.den, D.trg, nullptr, D.val,
-                                  D.gradT, 0.0, 0.0);
+    launch_near_f64<NearGrad<KT>>(st, D.numSMs, (int)P.evtrLeaves.size(), D.maxLeafTrg, P.ns, D.evtrLeaves,
+                                  D.nearPtr, D.nearIdx, D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt, D.src, D.nrm, D.den,
+                                  D.trg, nullptr, D.val, D.gradT, 0.0, 0.0);
     launches++;
   }
   if (!P.l2tLeaves.empty()) {

@@ -14,8 +14,9 @@
 // latency of the FP64 pipe.  The groups' partial sums meet through shuffles.
 // The 4 warps of a CTA share a leaf and take its chunks in turn (one warp a leaf
 // left the GPU idle behind the longest leaves, and all of it with few leaves),
-// their sums meet in shared memory in warp order; blocks of tb own points of a
-// leaf run as separate CTAs (grid.y).  No CTA-wide barrier in the loops.
+// their sums meet in shared memory in warp order; where leaves hold a few points
+// each warp has its own (launch_near_f64).  Blocks of tb own points of a leaf run
+// as separate CTAs (grid.y).  No CTA-wide barrier in the loops.
 // Against one warp (evaluate) or one barrier-bound CTA (adjoint) a leaf with one
 // point a lane: 65,536 points in 554 leaves 2.58 -> 0.37 ms, Stokes 60,007 points
 // 1.28 -> 0.28, 1M points in 62,000 leaves 2.15 -> 1.54; target gradient of 131,072
@@ -43,10 +44,11 @@ struct NearP2P {
   }
 };
 
-// weight: the sums of an own point are multiplied by weight[point] (null: not)
-template <class Op>
+// weight: the sums of an own point are multiplied by weight[point] (null: not).
+// WS: the warps a leaf, 4 or 1
+template <class Op, int WS>
 __global__ void __launch_bounds__(32 * NF_WARPS)
-    k_near_f64(int tb, const int32_t* __restrict__ rows, const int64_t* __restrict__ ptr,
+    k_near_f64(int nRows, int tb, const int32_t* __restrict__ rows, const int64_t* __restrict__ ptr,
                const int32_t* __restrict__ idx, const int64_t* __restrict__ stBeg, const int64_t* __restrict__ stCnt,
                const int64_t* __restrict__ ownBeg, const int64_t* __restrict__ ownCnt, const double* __restrict__ stPos,
                const double* __restrict__ stNrm, const double* __restrict__ stVal, const double* __restrict__ ownPos,
@@ -58,9 +60,10 @@ __global__ void __launch_bounds__(32 * NF_WARPS)
   __shared__ double sVal[NF_WARPS][NF_CH * SV];
   __shared__ int64_t eBeg[NF_WARPS][NF_MAXE];
   __shared__ int32_t ePre[NF_WARPS][NF_MAXE + 1];
-  __shared__ double sRed[NF_WARPS][32 * PR * OC];
+  __shared__ double sRed[WS > 1 ? NF_WARPS : 1][WS > 1 ? 32 * PR * OC : 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x;
+  const int row = blockIdx.x * (NF_WARPS / WS) + warp / WS, sub = warp % WS;
+  if (row >= nRows) return;  // WS == 1 only: no CTA-wide barrier below then
   const int g = rows[row];
   const int64_t oBeg = ownBeg[g], on = ownCnt[g];
   const int64_t e0 = ptr[row], e1 = ptr[row + 1];
@@ -104,7 +107,7 @@ __global__ void __launch_bounds__(32 * NF_WARPS)
       if (lane == 0) ePre[warp][0] = 0;
       __syncwarp();
       const int total = running;
-      for (int base = warp * NF_CH; base < total; base += NF_WARPS * NF_CH) {
+      for (int base = sub * NF_CH; base < total; base += WS * NF_CH) {
         const int cnt = min(NF_CH, total - base);
         __syncwarp();
         for (int i = lane; i < cnt; i += 32) {
@@ -143,27 +146,39 @@ __global__ void __launch_bounds__(32 * NF_WARPS)
       }
     }
     group_sum(acc, lane, sp, TG, S);
-    if (sp == 0) {
+    if constexpr (WS == 1) {
+      if (sp == 0) {
 #pragma unroll
-      for (int r = 0; r < PR; r++)
-        if (tl + r * TG < nt)
+        for (int r = 0; r < PR; r++) {
+          const int64_t t = oBeg + t0 + tl + r * TG;
+          if (tl + r * TG < nt)
 #pragma unroll
-          for (int c = 0; c < OC; c++) sRed[warp][(tl + r * TG) * OC + c] = acc[r][c];
+            for (int c = 0; c < OC; c++) out[t * OC + c] += weight ? weight[t] * acc[r][c] : acc[r][c];
+        }
+      }
+    } else {
+      if (sp == 0) {
+#pragma unroll
+        for (int r = 0; r < PR; r++)
+          if (tl + r * TG < nt)
+#pragma unroll
+            for (int c = 0; c < OC; c++) sRed[warp][(tl + r * TG) * OC + c] = acc[r][c];
+      }
+      __syncthreads();
+      for (int i = threadIdx.x; i < nt * OC; i += blockDim.x) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < NF_WARPS; w++) s += sRed[w][i];
+        out[(oBeg + t0) * OC + i] += weight ? weight[oBeg + t0 + i / OC] * s : s;
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nt * OC; i += blockDim.x) {
-      double s = 0.0;
-#pragma unroll
-      for (int w = 0; w < NF_WARPS; w++) s += sRed[w][i];
-      out[(oBeg + t0) * OC + i] += weight ? weight[oBeg + t0 + i / OC] * s : s;
-    }
-    __syncthreads();
   }
 }
 
-// maxOwn: the own points of the fullest row
+// maxOwn: the own points of the fullest row; nStaged: all staged points
 template <class Op>
-inline void launch_near_f64(cudaStream_t st, int nRows, int64_t maxOwn, const int32_t* rows, const int64_t* ptr,
+inline void launch_near_f64(cudaStream_t st, int numSMs, int nRows, int64_t maxOwn, int64_t nStaged, const int32_t* rows, const int64_t* ptr,
                             const int32_t* idx, const int64_t* stBeg, const int64_t* stCnt, const int64_t* ownBeg,
                             const int64_t* ownCnt, const double* stPos, const double* stNrm, const double* stVal,
                             const double* ownPos, const double* ownNrm, const double* weight, double* out, double mu,
@@ -171,8 +186,17 @@ inline void launch_near_f64(cudaStream_t st, int nRows, int64_t maxOwn, const in
   constexpr int TB = 16 * Op::PR;  // half the lanes' points: the staged ones split in two at least
   int64_t blocks = (maxOwn + TB - 1) / TB;  // a leaf of more than 64 blocks loops
   blocks = blocks < 1 ? 1 : (blocks > 64 ? 64 : blocks);
-  k_near_f64<Op><<<dim3(nRows, (unsigned)blocks), 32 * NF_WARPS, 0, st>>>(
-      TB, rows, ptr, idx, stBeg, stCnt, ownBeg, ownCnt, stPos, stNrm, stVal, ownPos, ownNrm, weight, out, mu, ve);
+  // With few points a leaf the list fits one warp's first chunks and the others
+  // only build its table: below 2.5 PR points a leaf a warp takes it alone.
+  // ms with 4 warps and with 1, scalar: 6.9 points a leaf 0.35 and 0.26, 9.2 0.26
+  // and 0.22, 11.4 0.37 and 0.46, 1.5 0.98 and 0.33; Stokes: 3.2 0.22 and 0.11, 7.0
+  // 0.19 and 0.21.  16 leaves an SM: the warps of fewer would not fill it.
+  const bool one = nRows > 16 * numSMs && 2 * nStaged < 5 * (int64_t)Op::PR * nRows;
+  auto* k = one ? k_near_f64<Op, 1> : k_near_f64<Op, NF_WARPS>;
+  const int perCta = one ? NF_WARPS : 1;
+  k<<<dim3((nRows + perCta - 1) / perCta, (unsigned)blocks), 32 * NF_WARPS, 0, st>>>(
+      nRows, TB, rows, ptr, idx, stBeg, stCnt, ownBeg, ownCnt, stPos, stNrm, stVal, ownPos, ownNrm, weight, out, mu,
+      ve);
 }
 
 }  // namespace fmmg

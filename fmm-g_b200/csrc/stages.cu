@@ -900,8 +900,9 @@ static void launch_near(const Plan& P, DevState& D, const int64_t* ptr, const in
                         cudaStream_t sn) {
   int n = (int)P.evtrLeaves.size();
   if (n == 0) return;
-  launch_near_f64<NearP2P<KT>>(sn, n, D.maxLeafTrg, D.evtrLeaves, ptr, idx, D.srcBeg, D.srcCnt, D.trgBeg, D.trgCnt,
-                               D.src, D.nrm, D.den, D.trg, nullptr, nullptr, D.val, P.o.coefs[0], P.o.coefs[1]);
+  launch_near_f64<NearP2P<KT>>(sn, D.numSMs, n, D.maxLeafTrg, P.ns, D.evtrLeaves, ptr, idx, D.srcBeg, D.srcCnt,
+                               D.trgBeg, D.trgCnt, D.src, D.nrm, D.den, D.trg, nullptr, nullptr, D.val,
+                               P.o.coefs[0], P.o.coefs[1]);
   if (ls) ls->launches++;
 }
 

@@ -46,3 +46,33 @@ def test_near_field_blocks(kt, n, n_trg, pts, levels):
         lib.evaluate_device(d[kk - 1].contiguous(), one, 1, fmmg.PREC_MIXED)
         lib.sync()
         assert rel_l2(full[kk - 1].cpu().numpy(), one.cpu().numpy()) <= 2e-5
+
+
+@pytest.mark.parametrize("kt", [111, 121, 311])
+@pytest.mark.parametrize("pts", [2, 9, 12])
+def test_near_field_of_small_leaves(kt, pts):
+    """Trees on either side of the points a leaf below which one warp takes it
+    (near_f64.cuh), with more than 16 leaves an SM: the evaluate against dense
+    sums at some targets (np = 6 truncates at 1e-6 to 1e-5; a near pair missed
+    or counted twice is 1e-2 here), the transposed sums through <w, A s> =
+    <A^T w, s>, and the target gradient against dense sums."""
+    rng = np.random.default_rng(SEED + kt + pts)
+    n = 9000 if pts < 5 else 60000
+    src, nrm = rng.random((n, 3)), unit_normals(rng, n)
+    lib = fmmg.FMM3d(kt, np_=6, pts_max=pts)
+    lib.setup(src, nrm)
+    assert len(lib.worklist(0)[0]) > 16 * 148
+    s, w = rng.uniform(-1, 1, n * lib.sd), rng.uniform(-1, 1, n * lib.td)
+    v = gpu_eval(lib, s)
+    idx = rng.choice(n, 300, replace=False)
+    rel, _, _ = lib.check(s, v, idx)
+    assert rel <= 1e-4
+    g, _ = lib.adjoint(w)
+    assert abs(float(w @ v) - float(g.ravel() @ s)) <= 1e-11 * np.linalg.norm(w) * np.linalg.norm(v)
+    if kt == 111:  # d/dx of w(x) sum_y den(y) / (4 pi |x - y|)
+        _, grad = lib.adjoint(w, s, target_grad=True)
+        d = src[idx, None, :] - src[None, :, :]
+        r = np.sqrt((d * d).sum(-1))
+        r[r == 0] = np.inf
+        dense = -(w[idx, None] / (4 * np.pi)) * (d * (s[None, :] / r**3)[..., None]).sum(1)
+        assert rel_l2(grad[idx], dense) <= 1e-4
