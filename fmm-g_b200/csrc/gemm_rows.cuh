@@ -43,12 +43,14 @@ __device__ __forceinline__ T gr_sel(const GrScale<T>& s, int i) {
 
 // Rows of several levels in one launch: with rowDepth, ys holds the degrees and
 // a row's scale is 2^(-(its node's depth + rootLevel) degree)
-template <typename T>
-__device__ __forceinline__ GrScale<T> gr_row_scale(const GrScale<T>& ys, const int32_t* rowDepth, int level) {
-  GrScale<T> r = ys;
+__device__ __forceinline__ GrScale<float> gr_row_scale(const GrScale<float>& ys, const int32_t* rowDepth, int level) {
+  GrScale<float> r = ys;
   if (rowDepth) {
+    r.v[0] = scalbnf(1.f, -(int)(level * ys.v[0]));
+    if (ys.mod != 1) {
 #pragma unroll
-    for (int c = 0; c < 4; c++) r.v[c] = (T)scalbn(1.0, -(int)(level * ys.v[c]));
+      for (int c = 1; c < 4; c++) r.v[c] = scalbnf(1.f, -(int)(level * ys.v[c]));
+    }
   }
   return r;
 }

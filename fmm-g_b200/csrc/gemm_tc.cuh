@@ -389,8 +389,13 @@ __global__ void __launch_bounds__(T3_THREADS, 1)
         }
       } else if (yr) {
         float a[16];
+        if (yv.mod == 1) {
 #pragma unroll
-        for (int j = 0; j < 16; j++) a[j] = R[cb * 16 + j] * gr_sel(yv, nb + j);
+          for (int j = 0; j < 16; j++) a[j] = R[cb * 16 + j] * yv.v[0];
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; j++) a[j] = R[cb * 16 + j] * gr_sel(yv, nb + j);
+        }
         if (vecY && nb + 16 <= N) {
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
