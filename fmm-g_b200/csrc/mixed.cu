@@ -1067,11 +1067,13 @@ __global__ void __launch_bounds__(256)
   }
   __syncthreads();
   // z pass: a thread owns one z line (kx, ky) of one plane and all N kz outputs
+  // (RW divides 8: (p0 + r) / RW = p0 / RW + r / RW)
+  float2* outB = effDen + blockIdx.y * blkStride + (int64_t)(p0 >> lgRW) * nEff * RW;
   for (int i = tid; i < NH * N * 8; i += blockDim.x) {
     int r, kx, ky;
     r8_item<NH>(i, lgRW, r, kx, ky);
-    if (p0 + r >= nPlanes) continue;
-    float2* out = effDen + blockIdx.y * blkStride + (int64_t)((p0 + r) >> lgRW) * nEff * RW + (r & (RW - 1));
+    if (LG != 3 && p0 + r >= nPlanes) continue;  // with 8 right-hand sides a block the 8 planes are one slot's
+    float2* out = outB + (r >> lgRW) * nEff * RW + (r & (RW - 1));
     unsigned long long axx[NP], nayy[NP];
 #pragma unroll
     for (int zb = 0; zb < NP; zb++) {
@@ -1111,7 +1113,12 @@ __global__ void __launch_bounds__(256)
   const int p0 = blockIdx.x * 8, RW = 1 << lgRW;
   const int tid = threadIdx.x;
   using IX = R8Idx<N, F::H>;
-  if (tid < 8) {
+  // 8 right-hand sides a block (LG 3): the planes are one component of one slot
+  float* dst0 = nullptr;
+  if (LG == 3) {
+    const int sm = p0 >> 3;
+    dst0 = dchk + (int64_t)blockIdx.y * 8 * dchkRhs + (int64_t)nodes[sm / tdm] * nDC * tdm + sm % tdm;
+  } else if (tid < 8) {
     const int p = p0 + tid, sm = p >> lgRW, rhs = blockIdx.y * RW + (p & (RW - 1));
     pOut[tid] = p < nPlanes && rhs < kc
                     ? dchk + (int64_t)rhs * dchkRhs + (int64_t)nodes[sm / tdm] * nDC * tdm + sm % tdm
@@ -1127,11 +1134,12 @@ __global__ void __launch_bounds__(256)
     wyy[m] = pq_pk(w.y, w.y);
   }
   // z pass, band outputs only: a thread owns one z line (kx, ky) of one plane
+  const float2* inB = effVal + blockIdx.y * blkStride + (int64_t)(p0 >> lgRW) * nEff * RW;
   for (int i = tid; i < NH * N * 8; i += blockDim.x) {
     int r, kx, ky;
     r8_item<NH>(i, lgRW, r, kx, ky);
-    if (p0 + r >= nPlanes) continue;
-    const float2* Xg = effVal + blockIdx.y * blkStride + (int64_t)((p0 + r) >> lgRW) * nEff * RW + (r & (RW - 1));
+    if (LG != 3 && p0 + r >= nPlanes) continue;
+    const float2* Xg = inB + (r >> lgRW) * nEff * RW + (r & (RW - 1));
     float2 c[N];
 #pragma unroll
     for (int kz = 0; kz < N; kz++) c[kz] = Xg[((kz * N + ky) * NH + kx) * RW];  // all loads of the line first
@@ -1167,8 +1175,8 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   for (int i = tid; i < nDC * 8; i += blockDim.x) {  // x pass (c2r) at the surface points
     const int j = i % nDC, r = i / nDC;
-    float* dst = pOut[r];
-    if (!dst) continue;
+    float* dst = LG == 3 ? dst0 + r * dchkRhs : pOut[r];
+    if (LG == 3 ? (int)blockIdx.y * 8 + r >= kc : !dst) continue;
     const int p = ijk[j];
     const int a = p & 255, b = (p >> 8) & 255, cc = p >> 16;
     const float2* y1 = &Y1[r * S1 + (cc * NP + b) * NH];
