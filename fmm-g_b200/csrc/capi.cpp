@@ -782,18 +782,20 @@ fmmg_status fmmg_plan_stats(const fmmg_handle* h, int64_t* st, int n) {
   for (int g : P.s2mLeaves) s2mPairs += P.srcCnt[g] * P.nUC;
   for (size_t r = 0; r < P.s2lNodes.size(); r++)
     for (int64_t e = P.s2lSrc.ptr[r]; e < P.s2lSrc.ptr[r + 1]; e++) s2lPairs += P.srcCnt[P.s2lSrc.idx[e]] * P.nDC;
-  for (int d = 0; d <= P.maxDepth; d++) {
+  // from depth 2: nothing reads the densities of depth 1 (run_stages)
+  for (int d = 2; d <= P.maxDepth; d++) {
     upFlops += (int64_t)P.upM2M[d].size() * 2 * uc * 8 * ue + (int64_t)P.upC2E[d].size() * 2 * ue * uc;
     if (d >= 3) dnFlops += (int64_t)P.dnL2L[d - 1].size() * 2 * 8 * dc * de;
     dnFlops += (int64_t)P.dnC2E[d].size() * 2 * de * dc;
   }
-  // the FP32 pass: parents take the folded C2E x M2M product, leaves and the
-  // downward pass the factored pseudo-inverses (ranks padded to 4)
+  // the FP32 pass: parents take the folded C2E x M2M product and hand theirs down
+  // through the folded C2E x L2L one, leaves and the nodes' own check potentials
+  // take the factored pseudo-inverses (ranks padded to 4)
   const int64_t kUp4 = (P.kUp + 3) & ~3, kDn4 = (P.kDn + 3) & ~3;
   int64_t upFlops32 = 0, dnFlops32 = 0;
-  for (int d = 0; d <= P.maxDepth; d++) {
+  for (int d = 2; d <= P.maxDepth; d++) {
     upFlops32 += (int64_t)P.upM2M[d].size() * 2 * ue * 8 * ue + (int64_t)P.upLeaf[d].size() * 2 * kUp4 * (uc + ue);
-    if (d >= 3) dnFlops32 += (int64_t)P.dnL2L[d - 1].size() * 2 * 8 * dc * de;
+    if (d >= 3) dnFlops32 += (int64_t)P.dnL2L[d - 1].size() * 2 * 8 * de * de;
     dnFlops32 += (int64_t)P.dnC2E[d].size() * 2 * kDn4 * (dc + de);
   }
   int64_t v[19] = {nearPairs, s2mPairs, s2lPairs, m2tPairs, l2tPairs,

@@ -190,3 +190,25 @@ def test_lazy_lists_follow_each_setup():
         for x, y in zip(f.worklist(which), g.worklist(which)):
             assert np.array_equal(x, y)
     assert not all(np.array_equal(x, y) for x, y in zip(first, f.worklist(6)))
+
+
+@pytest.mark.parametrize("kt,np_", [(111, 4), (311, 4), (511, 3)])
+def test_gemm_figures_count_the_products_of_depth_2_and_below(kt, np_):
+    """The row-GEMM figures of plan_stats from the tree: FP64 C2E and M2M of the
+    nodes with sources, L2L and C2E of those with targets; in the mixed form the
+    parents' folded products (8 ue x ue, 8 de x de) and the factored
+    pseudo-inverses of a rank (padded to 4) that both counts have to share."""
+    f = _case(kt, np_, 30, "clustered", 5000, 2500)
+    rec, _, _ = f.tree()
+    st = f.plan_stats()
+    depth, leaf, tag = rec[:, 0], rec[:, 5] < 0, rec[:, 6]
+    ue = de = (6 * (np_ - 1) ** 2 + 2) * st["sdm"]
+    uc, dc = (6 * (np_ + 1) ** 2 + 2) * st["tdm"], (6 * (np_ - 1) ** 2 + 2) * st["tdm"]
+    src, trg = (tag & 1 > 0) & (depth >= 2), (tag & EVTR > 0) & (depth >= 2)
+    parents_up, parents_dn = int((src & ~leaf).sum()), int((trg & ~leaf).sum())
+    assert st["up_gemm_flops"] == 2 * ue * uc * int(src.sum()) + 16 * ue * uc * parents_up
+    assert st["dn_gemm_flops"] == 2 * de * dc * int(trg.sum()) + 16 * de * dc * parents_dn
+    for total, parents, rows, m, n in ((st["up_gemm_flops_mixed"], parents_up, int((src & leaf).sum()), ue, uc),
+                                       (st["dn_gemm_flops_mixed"], parents_dn, int(trg.sum()), de, dc)):
+        rank, rest = divmod(total - 16 * m * m * parents, 2 * (m + n) * rows)
+        assert rest == 0 and rank % 4 == 0 and 0 < rank <= min(m, n) + 3
