@@ -55,35 +55,22 @@ __device__ __forceinline__ GrScale<float> gr_row_scale(const GrScale<float>& ys,
   return r;
 }
 
-template <typename T>
-struct GrVec;
-template <>
-struct GrVec<float> {
-  typedef float4 V;
-};
-template <>
-struct GrVec<double> {
-  typedef double2 V;
-};
-
 // VEC: X rows and W rows are 16-byte aligned with K a multiple of the vector
 // width, so the tiles are fetched as 16-byte vectors along K (4 vectors per
 // row of a K step, consecutive threads on consecutive vectors); otherwise
 // element by element.  Shared tiles are padded against bank conflicts.
-template <typename T, int BK, bool VEC>
+template <bool VEC>
 __global__ void __launch_bounds__(GR_THREADS, 2)
     k_gemm_rows_t(int nrows, int nrhs, const int32_t* __restrict__ rows, const int32_t* __restrict__ chd, int xChild,
-                  int yChild, const T* __restrict__ X, int64_t ldx, int64_t xRhs, const T* __restrict__ W,
-                  T* __restrict__ Y, int64_t ldy, int64_t yRhs, int K, int N, GrScale<T> xs, GrScale<T> ys, T beta,
-                  int kChunk, T* __restrict__ part, const int32_t* __restrict__ rowDepth, int rootLevel) {
-  typedef typename GrVec<T>::V V;
-  constexpr int VW = sizeof(V) / sizeof(T);  // 4 floats or 2 doubles
-  static_assert(BK / VW == 4, "four vectors per tile row");
-  constexpr int PA = GR_BM + VW, PB = GR_BN + VW;  // padded tile rows
-  __shared__ __align__(16) T As[2][BK][PA];
-  __shared__ __align__(16) T Bs[2][BK][PB];
-  __shared__ const T* xrow[GR_BM];
-  __shared__ T* yrow[GR_BM];
+                  int yChild, const float* __restrict__ X, int64_t ldx, int64_t xRhs, const float* __restrict__ W,
+                  float* __restrict__ Y, int64_t ldy, int64_t yRhs, int K, int N, GrScale<float> xs,
+                  GrScale<float> ys, float beta, int kChunk, float* __restrict__ part, const int32_t* __restrict__ rowDepth, int rootLevel) {
+  static_assert(GR_BK == 16, "four vectors per tile row");
+  constexpr int PA = GR_BM + 4, PB = GR_BN + 4;  // padded tile rows
+  __shared__ __align__(16) float As[2][GR_BK][PA];
+  __shared__ __align__(16) float Bs[2][GR_BK][PB];
+  __shared__ const float* xrow[GR_BM];
+  __shared__ float* yrow[GR_BM];
   __shared__ int ylev[GR_BM];
   const int tid = threadIdx.x;
   const int r0 = blockIdx.x * GR_BM, n0 = blockIdx.y * GR_BN;
@@ -104,78 +91,77 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
   // K range of this split (blockIdx.z); the whole of K without splitting
   const int kBeg = blockIdx.z * kChunk, kEnd = min(K, kBeg + kChunk);
   // fetch mapping: A vectors (row tid/4 and 64 + tid/4, K quad tid%4), B vector (output tid/4, K quad tid%4)
-  const int fr = tid >> 2, fq = (tid & 3) * VW;
-  const T* xa0 = xrow[fr];
-  const T* xa1 = xrow[fr + 64];
+  const int fr = tid >> 2, fq = (tid & 3) * 4;
+  const float* xa0 = xrow[fr];
+  const float* xa1 = xrow[fr + 64];
   const bool bIn = n0 + fr < N;
-  const T* wr = W + (int64_t)(bIn ? n0 + fr : 0) * K;
-  T fa0[VW], fa1[VW], fb[VW];
+  const float* wr = W + (int64_t)(bIn ? n0 + fr : 0) * K;
+  float fa0[4], fa1[4], fb[4];
   auto fetch = [&](int k0) {
     const int k = k0 + fq;
     if (VEC) {
-      const bool kin = k < kEnd;  // VW | K and VW | kChunk: the whole vector is in range
-      V a0 = {}, a1 = {}, bv = {};
-      if (xa0 && kin) a0 = *reinterpret_cast<const V*>(xa0 + k);
-      if (xa1 && kin) a1 = *reinterpret_cast<const V*>(xa1 + k);
-      if (bIn && kin) bv = *reinterpret_cast<const V*>(wr + k);
-      const T* pa0 = reinterpret_cast<const T*>(&a0);
-      const T* pa1 = reinterpret_cast<const T*>(&a1);
-      const T* pb = reinterpret_cast<const T*>(&bv);
+      const bool kin = k < kEnd;  // 4 | K and 4 | kChunk: the whole vector is in range
+      float4 a0 = {}, a1 = {}, bv = {};
+      if (xa0 && kin) a0 = *reinterpret_cast<const float4*>(xa0 + k);
+      if (xa1 && kin) a1 = *reinterpret_cast<const float4*>(xa1 + k);
+      if (bIn && kin) bv = *reinterpret_cast<const float4*>(wr + k);
+      const float* pa0 = reinterpret_cast<const float*>(&a0);
+      const float* pa1 = reinterpret_cast<const float*>(&a1);
+      const float* pb = reinterpret_cast<const float*>(&bv);
 #pragma unroll
-      for (int j = 0; j < VW; j++) {
-        const T sc = gr_sel(xs, k + j);
+      for (int j = 0; j < 4; j++) {
+        const float sc = gr_sel(xs, k + j);
         fa0[j] = pa0[j] * sc;
         fa1[j] = pa1[j] * sc;
         fb[j] = pb[j];
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < VW; j++) {
+      for (int j = 0; j < 4; j++) {
         const bool kin = k + j < kEnd;
-        const T sc = gr_sel(xs, k + j);
-        fa0[j] = (xa0 && kin) ? xa0[k + j] * sc : T(0);
-        fa1[j] = (xa1 && kin) ? xa1[k + j] * sc : T(0);
-        fb[j] = (bIn && kin) ? wr[k + j] : T(0);
+        const float sc = gr_sel(xs, k + j);
+        fa0[j] = (xa0 && kin) ? xa0[k + j] * sc : 0.f;
+        fa1[j] = (xa1 && kin) ? xa1[k + j] * sc : 0.f;
+        fb[j] = (bIn && kin) ? wr[k + j] : 0.f;
       }
     }
   };
   auto stash = [&](int b) {
 #pragma unroll
-    for (int j = 0; j < VW; j++) {
+    for (int j = 0; j < 4; j++) {
       As[b][fq + j][fr] = fa0[j];
       As[b][fq + j][fr + 64] = fa1[j];
       Bs[b][fq + j][fr] = fb[j];
     }
   };
   const int tm = tid >> 4, tn = tid & 15;  // rows tm*8 .. +7, outputs tn*4 .. +3
-  T acc[8][4];
+  float acc[8][4];
 #pragma unroll
   for (int i = 0; i < 8; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = T(0);
+    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
   fetch(kBeg);
   stash(0);
   __syncthreads();
   int buf = 0;
-  for (int k0 = kBeg; k0 < kEnd; k0 += BK) {
-    const bool more = k0 + BK < kEnd;
-    if (more) fetch(k0 + BK);
+  for (int k0 = kBeg; k0 < kEnd; k0 += GR_BK) {
+    const bool more = k0 + GR_BK < kEnd;
+    if (more) fetch(k0 + GR_BK);
 #pragma unroll
-    for (int k = 0; k < BK; k++) {
-      T a[8], b[4];
+    for (int k = 0; k < GR_BK; k++) {
+      float a[8], b[4];
 #pragma unroll
-      for (int i = 0; i < 8; i += VW) {
-        const V v = *reinterpret_cast<const V*>(&As[buf][k][tm * 8 + i]);
-        const T* pv = reinterpret_cast<const T*>(&v);
+      for (int i = 0; i < 8; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(&As[buf][k][tm * 8 + i]);
+        const float* pv = reinterpret_cast<const float*>(&v);
 #pragma unroll
-        for (int j = 0; j < VW; j++) a[i + j] = pv[j];
+        for (int j = 0; j < 4; j++) a[i + j] = pv[j];
       }
+      {
+        const float4 v = *reinterpret_cast<const float4*>(&Bs[buf][k][tn * 4]);
+        const float* pv = reinterpret_cast<const float*>(&v);
 #pragma unroll
-      for (int j0 = 0; j0 < 4; j0 += VW) {
-        const V v = *reinterpret_cast<const V*>(&Bs[buf][k][tn * 4 + j0]);
-        const T* pv = reinterpret_cast<const T*>(&v);
-#pragma unroll
-        for (int j = 0; j < VW; j++) b[j0 + j] = pv[j];
+        for (int j = 0; j < 4; j++) b[j] = pv[j];
       }
 #pragma unroll
       for (int i = 0; i < 8; i++)
@@ -194,7 +180,7 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
     for (int i = 0; i < 8; i++) {
       const int r = r0 + tm * 8 + i;
       if (r >= M) continue;
-      T* pr = part + ((int64_t)blockIdx.z * M + r) * N;
+      float* pr = part + ((int64_t)blockIdx.z * M + r) * N;
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int n = n0 + tn * 4 + j;
@@ -205,39 +191,38 @@ __global__ void __launch_bounds__(GR_THREADS, 2)
   }
 #pragma unroll
   for (int i = 0; i < 8; i++) {
-    T* yr = yrow[tm * 8 + i];
+    float* yr = yrow[tm * 8 + i];
     if (!yr) continue;
-    const GrScale<T> yv = gr_row_scale(ys, rowDepth, ylev[tm * 8 + i]);
+    const GrScale<float> yv = gr_row_scale(ys, rowDepth, ylev[tm * 8 + i]);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const int n = n0 + tn * 4 + j;
       if (n < N) {
-        const T v = acc[i][j] * gr_sel(yv, n);
-        yr[n] = beta == T(0) ? v : beta * yr[n] + v;
+        const float v = acc[i][j] * gr_sel(yv, n);
+        yr[n] = beta == 0.f ? v : beta * yr[n] + v;
       }
     }
   }
 }
 
 // Y[row] = beta * Y[row] + ys .* sum over splits of part[split][row]
-template <typename T>
-__global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(256)
     k_gemm_reduce_t(int nrows, int nrhs, const int32_t* __restrict__ rows, const int32_t* __restrict__ chd,
-                    int yChild, T* __restrict__ Y, int64_t ldy, int64_t yRhs, int N, int splits,
-                    const T* __restrict__ part, GrScale<T> ys, T beta, const int32_t* __restrict__ rowDepth,
-                    int rootLevel) {
+                    int yChild, float* __restrict__ Y, int64_t ldy, int64_t yRhs, int N, int splits,
+                    const float* __restrict__ part, GrScale<float> ys, float beta,
+                    const int32_t* __restrict__ rowDepth, int rootLevel) {
   const int64_t M = (int64_t)nrows * nrhs;
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= M * N) return;
   const int64_t r = i / N;
   const int n = (int)(i - r * N);
-  T s = T(0);
+  float s = 0.f;
   for (int z = 0; z < splits; z++) s += part[((int64_t)z * M + r) * N + n];
   const int q = (int)(r / nrows);
   const int node = rows[r - (int64_t)q * nrows];
-  T* yr = Y + q * yRhs + (int64_t)(yChild ? chd[node] : node) * ldy;
-  const T v = s * gr_sel(gr_row_scale(ys, rowDepth, rowDepth ? rowDepth[node] + rootLevel : 0), n);
-  yr[n] = beta == T(0) ? v : beta * yr[n] + v;
+  float* yr = Y + q * yRhs + (int64_t)(yChild ? chd[node] : node) * ldy;
+  const float v = s * gr_sel(gr_row_scale(ys, rowDepth, rowDepth ? rowDepth[node] + rootLevel : 0), n);
+  yr[n] = beta == 0.f ? v : beta * yr[n] + v;
 }
 
 // ------------------------------------------------------------------ FP32 wide tile
@@ -449,48 +434,47 @@ inline int launch_gemm_rows_w(cudaStream_t st, int splitCtas, float* scratch, si
                                              yRhs, K, N, xs, ys, beta, kChunk, pt, yVec, rowDepth, rootLevel);
   if (splits == 1) return 1;
   const int64_t tot = M * N;
-  k_gemm_reduce_t<float><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(nrows, nrhs, rows, chd, yChild, Y, ldy, yRhs,
+  k_gemm_reduce_t<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(nrows, nrhs, rows, chd, yChild, Y, ldy, yRhs,
                                                                          N, splits, scratch, ys, beta, rowDepth, rootLevel);
   return 2;
 }
 
 // Launches the row GEMM; when the output tiles alone would leave the GPU
 // underfilled (fewer than splitCtas CTAs: 2 per SM by default, set by the
-// autotuner, 0 never splits) and K is long, K is split into up to 8 chunks whose partial tiles go to `scratch` (scratchElems values) and are
-// summed in a fixed order by k_gemm_reduce_t, so results stay deterministic.
+// autotuner, 0 never splits) and K is long, K is split into up to 8 chunks whose
+// partial tiles go to `scratch` (scratchElems values) and are summed in a fixed order by k_gemm_reduce_t, so results stay deterministic.
 // Returns the number of kernels launched.
-template <typename T, int BK>
-inline int launch_gemm_rows(cudaStream_t st, int splitCtas, T* scratch, size_t scratchElems, int nrows, int nrhs,
-                            const int32_t* rows, const int32_t* chd, int xChild, int yChild, const T* X, int64_t ldx,
-                            int64_t xRhs, const T* W, T* Y, int64_t ldy, int64_t yRhs, int K, int N, GrScale<T> xs,
-                            GrScale<T> ys, T beta, const int32_t* rowDepth, int rootLevel) {
+inline int launch_gemm_rows(cudaStream_t st, int splitCtas, float* scratch, size_t scratchElems, int nrows, int nrhs,
+                            const int32_t* rows, const int32_t* chd, int xChild, int yChild, const float* X,
+                            int64_t ldx, int64_t xRhs, const float* W, float* Y, int64_t ldy, int64_t yRhs, int K,
+                            int N, GrScale<float> xs, GrScale<float> ys, float beta, const int32_t* rowDepth,
+                            int rootLevel) {
   if (nrows <= 0 || nrhs <= 0) return 0;
   const int64_t M = (int64_t)nrows * nrhs;
   const int tiles = (int)((M + GR_BM - 1) / GR_BM) * ((N + GR_BN - 1) / GR_BN);
   int splits = 1;
-  if (scratch && tiles < splitCtas && K >= 8 * BK) {
+  if (scratch && tiles < splitCtas && K >= 8 * GR_BK) {
     splits = std::min(8, (splitCtas + tiles - 1) / tiles);
-    splits = std::min(splits, K / (4 * BK));
+    splits = std::min(splits, K / (4 * GR_BK));
     while (splits > 1 && (size_t)splits * M * N > scratchElems) splits--;
   }
-  const int kChunk = splits > 1 ? ((K + splits - 1) / splits + BK - 1) / BK * BK : K;
+  const int kChunk = splits > 1 ? ((K + splits - 1) / splits + GR_BK - 1) / GR_BK * GR_BK : K;
   if (splits > 1) splits = (K + kChunk - 1) / kChunk;
-  constexpr int VW = 16 / sizeof(T);
-  const bool vec = ((uintptr_t)X % 16 == 0) && ((uintptr_t)W % 16 == 0) && ldx % VW == 0 && xRhs % VW == 0 &&
-                   K % VW == 0;
+  const bool vec = ((uintptr_t)X % 16 == 0) && ((uintptr_t)W % 16 == 0) && ldx % 4 == 0 && xRhs % 4 == 0 &&
+                   K % 4 == 0;
   dim3 grid((unsigned)((M + GR_BM - 1) / GR_BM), (N + GR_BN - 1) / GR_BN, splits);
-  T* pt = splits > 1 ? scratch : nullptr;
+  float* pt = splits > 1 ? scratch : nullptr;
   if (vec)
-    k_gemm_rows_t<T, BK, true><<<grid, GR_THREADS, 0, st>>>(nrows, nrhs, rows, chd, xChild, yChild, X, ldx, xRhs, W,
+    k_gemm_rows_t<true><<<grid, GR_THREADS, 0, st>>>(nrows, nrhs, rows, chd, xChild, yChild, X, ldx, xRhs, W,
                                                              Y, ldy, yRhs, K, N, xs, ys, beta, kChunk, pt,
                                                              rowDepth, rootLevel);
   else
-    k_gemm_rows_t<T, BK, false><<<grid, GR_THREADS, 0, st>>>(nrows, nrhs, rows, chd, xChild, yChild, X, ldx, xRhs, W,
+    k_gemm_rows_t<false><<<grid, GR_THREADS, 0, st>>>(nrows, nrhs, rows, chd, xChild, yChild, X, ldx, xRhs, W,
                                                               Y, ldy, yRhs, K, N, xs, ys, beta, kChunk, pt,
                                                               rowDepth, rootLevel);
   if (splits == 1) return 1;
   const int64_t tot = M * N;
-  k_gemm_reduce_t<T><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(nrows, nrhs, rows, chd, yChild, Y, ldy, yRhs, N,
+  k_gemm_reduce_t<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(nrows, nrhs, rows, chd, yChild, Y, ldy, yRhs, N,
                                                                      splits, scratch, ys, beta, rowDepth, rootLevel);
   return 2;
 }

@@ -580,7 +580,7 @@ inline int launch_gemm_tc3(cudaStream_t st, int splitCtas, float* scratch, size_
                                                                    rootLevel);
   if (splits == 1) return 1;
   const int64_t tot = M * N;
-  k_gemm_reduce_t<float><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(nrows, nrhs, rows, chd, yChild, Y, ldy, yRhs,
+  k_gemm_reduce_t<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(nrows, nrhs, rows, chd, yChild, Y, ldy, yRhs,
                                                                          N, splits, scratch, ys, beta, rowDepth,
                                                                          rootLevel);
   return 2;
@@ -604,7 +604,7 @@ inline int launch_gemm_rows_f32(cudaStream_t st, int splitCtas, float* scratch, 
   if (Wt && xvec && ((uintptr_t)Wt % 16 == 0) && ldw % GW_BN == 0)
     return launch_gemm_rows_w(st, splitCtas, scratch, scratchElems, nrows, nrhs, rows, chd, xChild, yChild, X, ldx,
                               xRhs, Wt, ldw, Y, ldy, yRhs, K, N, xs, ys, beta, rowDepth, rootLevel);
-  return launch_gemm_rows<float, 16>(st, splitCtas, scratch, scratchElems, nrows, nrhs, rows, chd, xChild, yChild, X,
+  return launch_gemm_rows(st, splitCtas, scratch, scratchElems, nrows, nrhs, rows, chd, xChild, yChild, X,
                                      ldx, xRhs, W, Y, ldy, yRhs, K, N, xs, ys, beta, rowDepth, rootLevel);
 }
 

@@ -1907,9 +1907,12 @@ std::string dev_evaluate_mixed(const Plan& P, DevState& D, const double* dDen, d
     // potentials.  The upward C2E reads only the check rows of leaves with
     // sources, which S2M assigns; the upward densities of the nodes with
     // sources are assigned (leaf C2E, the folded product for parents) and the
-    // others stay zero from allocation; every downward density that L2L or
-    // L2T reads is assigned by C2E at its level before.  With the upward stage
-    // masked off the densities are cleared so the V and W stages see zeros.
+    // others stay zero from allocation; the downward densities of the nodes with
+    // targets are assigned by C2E, all levels at once, before the folded products
+    // add the parents' parts level by level (to all 8 children: the rows of
+    // those without targets only ever grow, from zero, and nothing reads them).
+    // With the upward stage masked off the densities are cleared so the V and W
+    // stages see zeros.
     FMMG_CK(cudaMemsetAsync(D.valK, 0, sizeof(double) * kk * valStride, st));
     FMMG_CK(cudaMemsetAsync(D.dchk32, 0, sizeof(float) * kk * P.nn * dc, st));
     if (!(mask & 1)) FMMG_CK(cudaMemsetAsync(D.uden32, 0, sizeof(float) * kk * P.nn * ue, st));

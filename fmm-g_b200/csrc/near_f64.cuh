@@ -178,11 +178,11 @@ __global__ void __launch_bounds__(32 * NF_WARPS)
 
 // maxOwn: the own points of the fullest row; nStaged: all staged points
 template <class Op>
-inline void launch_near_f64(cudaStream_t st, int numSMs, int nRows, int64_t maxOwn, int64_t nStaged, const int32_t* rows, const int64_t* ptr,
-                            const int32_t* idx, const int64_t* stBeg, const int64_t* stCnt, const int64_t* ownBeg,
-                            const int64_t* ownCnt, const double* stPos, const double* stNrm, const double* stVal,
-                            const double* ownPos, const double* ownNrm, const double* weight, double* out, double mu,
-                            double ve) {
+inline void launch_near_f64(cudaStream_t st, int numSMs, int nRows, int64_t maxOwn, int64_t nStaged,
+                            const int32_t* rows, const int64_t* ptr, const int32_t* idx, const int64_t* stBeg,
+                            const int64_t* stCnt, const int64_t* ownBeg, const int64_t* ownCnt, const double* stPos,
+                            const double* stNrm, const double* stVal, const double* ownPos, const double* ownNrm,
+                            const double* weight, double* out, double mu, double ve) {
   constexpr int TB = 16 * Op::PR;  // half the lanes' points: the staged ones split in two at least
   int64_t blocks = (maxOwn + TB - 1) / TB;  // a leaf of more than 64 blocks loops
   blocks = blocks < 1 ? 1 : (blocks > 64 ? 64 : blocks);
