@@ -225,3 +225,38 @@ def test_translation_layouts_change_in_place():
         torch.cuda.empty_cache()
         free.append(torch.cuda.mem_get_info()[0])
     assert free[-1] >= free[0] - 16 * MB
+
+
+@pytest.mark.parametrize("kt", [111, 311])
+def test_replaced_tables_go_with_the_next_setup(kt):
+    """Replaced tables (for 311 with 3 x 3 blocks that are not symmetric) serve
+    the evaluates until the next setup, which goes back to the built ones in
+    every form, and keeps those through further setups."""
+    rng = np.random.default_rng(SEED + kt)
+    x, den, w = _inputs(kt, 3000, rng)
+    y = rng.random((2500, 3))
+    den_y, w_y = den[:, :2500 * fmmg.KERNELS[kt][0]].copy(), w[:2500 * fmmg.KERNELS[kt][1]].copy()
+    g = fmmg.FMM3d(kt, np_=4, pts_max=40)
+    g.setup(x)
+    want = _outputs(g, den, w)
+    f = fmmg.FMM3d(kt, np_=4, pts_max=40)
+    f.setup(x)
+    first = _outputs(f, den, w)
+    n_sp = 12 if kt == 311 else 1
+    scale = np.linspace(1.0, 1.1, n_sp)
+    for i in range(316):
+        f.set_operator(4, i, f.operator(4, i).reshape(-1, n_sp, 2) * scale[None, :, None])
+    f.set_operator(3, 2, f.operator(3, 2) * 1.5)
+    replaced = _outputs(f, den, w)
+    for key in want:
+        assert np.array_equal(first[key], want[key]), key
+        assert rel_l2(replaced[key], want[key]) > 1e-3, key  # the replaced tables are in use
+    f.setup(y)
+    g2 = fmmg.FMM3d(kt, np_=4, pts_max=40)
+    g2.setup(y)
+    got, ref = _outputs(f, den_y, w_y), _outputs(g2, den_y, w_y)
+    f.setup(x)
+    again = _outputs(f, den, w)
+    for key in want:
+        assert np.array_equal(got[key], ref[key]), key
+        assert np.array_equal(again[key], want[key]), key
