@@ -443,6 +443,19 @@ fmmg_status fmmg_selftest_wait(int device, int arrive, int64_t limit_ns) {
   return flag ? FMMG_TIMEOUT : FMMG_OK;
 }
 
+fmmg_status fmmg_selftest_gemm(int device, int tile, int nrows, int K, int N, const double* x, const double* w,
+                               const double* x_scale, int mod, double* y) {
+  if (device < 0 || tile < 0 || tile > 3 || nrows < 1 || K < 2 || K % 2 || N < 1 || nrows > 4096 || K > 16384 ||
+      N > 16384 || (mod != 1 && mod != 3 && mod != 4) || !x || !w || !x_scale || !y)
+    return FMMG_INVALID_ARG;
+  try {
+    std::string e = fmmg::dev_gemm_selftest(device, tile, nrows, K, N, x, w, x_scale, mod, y);
+    if (!e.empty()) return fail(nullptr, FMMG_CUDA_ERROR, e);
+  }
+  FMMG_GUARD(nullptr)
+  return FMMG_OK;
+}
+
 fmmg_status fmmg_device_error(fmmg_handle* h, int* flag) {
   if (!h || !flag) return fail(h, FMMG_INVALID_ARG, "NULL argument");
   *flag = 0;

@@ -235,6 +235,11 @@ void scatter_rows(cudaStream_t st, int64_t n, int dof, const int64_t* perm, cons
 std::string dev_far_field(const Plan& P, DevState& D, const double* dDen);
 // reads and clears the device error flag (synchronises the handle's stream)
 std::string dev_take_error(DevState& D, int* flag);
+// One product Y = W (xs .* X) of the FP64 row GEMM with tile `tile` on host
+// arrays: X [nrows][K], W [N][K], Y [nrows][N]; X's columns scaled by xScale
+// (mod 1, 3 or 4 powers of two in turn).  K even.
+std::string dev_gemm_selftest(int device, int tile, int nrows, int K, int N, const double* X, const double* W,
+                              const double* xScale, int mod, double* Y);
 // Runs the bounded-wait error path on `device` (k_wait_selftest); *flag = 1
 // when the wait ran out.
 std::string dev_wait_selftest(int device, int arrive, long long limitNs, int* flag);

@@ -177,6 +177,22 @@ inline void gd_launch(cudaStream_t st, int nrows, const int32_t* rows, const int
       nrows, rows, chd, xChild, yChild, X, ldx, W, Y, ldy, K, N, xs, ys, beta, rowDepth, rootLevel);
 }
 
+constexpr int GD_TILES = 4;
+// Launches tile 0 (128 x 80), 1 (64 x 80), 2 (64 x 32) or 3 (16 x 16).
+inline void gd_launch_tile(int tile, cudaStream_t st, int nrows, const int32_t* rows, const int32_t* chd, int xChild,
+                           int yChild, const double* X, int64_t ldx, const double* W, double* Y, int64_t ldy, int K,
+                           int N, GrScale<double> xs, GrScale<double> ys, double beta, const int32_t* rowDepth,
+                           int rootLevel) {
+#define FMMG_GD(...)                                                                                           \
+  gd_launch<__VA_ARGS__>(st, nrows, rows, chd, xChild, yChild, X, ldx, W, Y, ldy, K, N, xs, ys, beta, rowDepth, \
+                         rootLevel)
+  if (tile == 0) FMMG_GD(128, 80, 32, 40, 3);
+  else if (tile == 1) FMMG_GD(64, 80, 32, 40, 3);
+  else if (tile == 2) FMMG_GD(64, 32, 16, 16, 4);
+  else FMMG_GD(16, 16, 8, 8, 4);
+#undef FMMG_GD
+}
+
 // The largest tile that still gives every SM a CTA: below that the smaller one
 // is faster (the table above), down to 16 x 16 at any size.
 inline void launch_gemm_f64(cudaStream_t st, int numSMs, int nrows, const int32_t* rows, const int32_t* chd,
@@ -185,14 +201,9 @@ inline void launch_gemm_f64(cudaStream_t st, int numSMs, int nrows, const int32_
                             const int32_t* rowDepth, int rootLevel) {
   if (nrows <= 0) return;
   auto ctas = [&](int bm, int bn) { return (int64_t)((nrows + bm - 1) / bm) * ((N + bn - 1) / bn); };
-#define FMMG_GD(...)                                                                                           \
-  gd_launch<__VA_ARGS__>(st, nrows, rows, chd, xChild, yChild, X, ldx, W, Y, ldy, K, N, xs, ys, beta, rowDepth, \
-                         rootLevel)
-  if (ctas(128, 80) >= numSMs) FMMG_GD(128, 80, 32, 40, 3);
-  else if (ctas(64, 80) >= numSMs) FMMG_GD(64, 80, 32, 40, 3);
-  else if (ctas(64, 32) >= numSMs) FMMG_GD(64, 32, 16, 16, 4);
-  else FMMG_GD(16, 16, 8, 8, 4);
-#undef FMMG_GD
+  const int tile = ctas(128, 80) >= numSMs ? 0 : ctas(64, 80) >= numSMs ? 1 : ctas(64, 32) >= numSMs ? 2 : 3;
+  gd_launch_tile(tile, st, nrows, rows, chd, xChild, yChild, X, ldx, W, Y, ldy, K, N, xs, ys, beta, rowDepth,
+                 rootLevel);
 }
 
 }  // namespace fmmg

@@ -1192,6 +1192,35 @@ std::string dev_evaluate(const Plan& P, DevState& D, const double* dDen, double*
   return std::string();
 }
 
+std::string dev_gemm_selftest(int device, int tile, int nrows, int K, int N, const double* X, const double* W,
+                              const double* xScale, int mod, double* Y) {
+  FMMG_CK(cudaSetDevice(device));
+  double* p = nullptr;
+  const size_t nx = (size_t)nrows * K, nw = (size_t)N * K, ny = (size_t)nrows * N;
+  std::vector<int32_t> rows(nrows);
+  for (int i = 0; i < nrows; i++) rows[i] = i;
+  GrScale<double> xs, one;
+  xs.mod = mod;
+  one.mod = 1;
+  for (int k = 0; k < 4; k++) {
+    xs.v[k] = k < mod ? xScale[k] : 1.0;
+    one.v[k] = 1.0;
+  }
+  FMMG_CK(cudaMalloc(&p, (nx + nw + ny) * sizeof(double) + nrows * sizeof(int32_t)));
+  int32_t* dRows = (int32_t*)(p + nx + nw + ny);
+  cudaError_t e = cudaMemcpy(p, X, nx * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(p + nx, W, nw * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(dRows, rows.data(), nrows * sizeof(int32_t), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    gd_launch_tile(tile, 0, nrows, dRows, nullptr, 0, 0, p, K, p + nx, p + nx + nw, N, K, N, xs, one, 0.0, nullptr, 0);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(Y, p + nx + nw, ny * sizeof(double), cudaMemcpyDeviceToHost);
+  cudaFree(p);
+  if (e != cudaSuccess) return std::string("GEMM self-test: ") + cudaGetErrorString(e);
+  return std::string();
+}
+
 void gather_rows(cudaStream_t st, int64_t n, int dof, const int64_t* perm, const double* in, double* out) {
   if (n > 0) k_gather_den<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, dof, perm, in, out);
 }

@@ -255,6 +255,14 @@ fmmg_status fmmg_device_error(fmmg_handle* h, int* flag);
  * the device still usable.  Synchronises the device.  No counterpart in the
  * reference. */
 fmmg_status fmmg_selftest_wait(int device, int arrive, int64_t limit_ns);
+/* One product of the FP64 row GEMM, for tests of its order of sums: y[r][n] =
+ * sum over k of w[n][k] s[k mod `mod`] x[r][k], one multiply-add after another in
+ * ascending k.  Host arrays x [nrows][K], w [N][K], y [nrows][N]; x_scale holds
+ * `mod` (1, 3 or 4) powers of two; K even; tile 0..3 selects the kernel's 128 x
+ * 80, 64 x 80, 64 x 32 or 16 x 16 tiles.  nrows <= 4096, K, N <= 16384.  No
+ * counterpart in the reference. */
+fmmg_status fmmg_selftest_gemm(int device, int tile, int nrows, int K, int N, const double* x, const double* w,
+                               const double* x_scale, int mod, double* y);
 
 /* Autotuner (no counterpart in the reference): times `reps` evaluates of
  * (k, precision) on the caller's device buffers for each candidate launch
