@@ -1220,22 +1220,34 @@ static std::vector<double> pad_cols(const std::vector<double>& F, int m, int k) 
   return r;
 }
 
-// The operator layout's device staging, up to a few hundred MB once a handle:
-// given back at its end, when the stream has drained, on an error's return too.
+// The operator layout's device staging, one operator after another on the
+// handle's stream: the row GEMMs' split-K scratch (64 MB, used on that stream
+// only), and blocks of its own for what does not fit there (vector kernels at np
+// 7 and 8, once a handle), given back when the stream has drained, on an error's
+// return too.  Blocks for all of it cost the first mixed call 2 to 5 ms.
 struct OpStaging {
-  cudaStream_t st;
+  DevState& D;
+  size_t used = 0;
   std::vector<void*> held;
-  explicit OpStaging(cudaStream_t s) : st(s) {}
+  explicit OpStaging(DevState& d) : D(d) {}
   ~OpStaging() {
-    cudaStreamSynchronize(st);
+    if (held.empty()) return;
+    cudaStreamSynchronize(D.stream);
     for (void* p : held) cudaFree(p);
   }
   OpStaging(const OpStaging&) = delete;
   OpStaging& operator=(const OpStaging&) = delete;
+  void next() { used = 0; }  // the next operator: what the last one staged has been queued
   template <typename T>
   std::string get(T*& p, size_t n) {
+    const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+    if (D.gemmScratch && used + bytes <= D.gemmScratchBytes) {
+      p = (T*)((unsigned char*)D.gemmScratch + used);
+      used += bytes;
+      return std::string();
+    }
     void* q = nullptr;
-    cudaError_t e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
+    cudaError_t e = cudaMalloc(&q, bytes);
     if (e != cudaSuccess) return std::string("cudaMalloc: ") + cudaGetErrorString(e);
     held.push_back(q);
     p = (T*)q;
@@ -1423,10 +1435,11 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     // rank that is a multiple of 4 (zero rows of F1, zero columns of F2), so the
     // intermediate rows allow 16-byte tile fetches
     auto alloc = [&](float*& p, size_t n) { return dalloc(D, p, n); };
-    OpStaging tmp(D.stream);
+    OpStaging tmp(D);
     auto prep = [&](TcOp& op, DevState::OpT& wt, float* plain, const std::vector<double>& W, int n,
                     int k) -> std::string {
       double* dW = nullptr;
+      tmp.next();
       FMMG_TRY(tmp.get(dW, W.size()));
       FMMG_CK(cudaMemcpyAsync(dW, W.data(), W.size() * sizeof(double), cudaMemcpyHostToDevice, D.stream));
       return prepare_operator(D.stream, op, wt, plain, dW, n, k, alloc);
@@ -1444,6 +1457,7 @@ static std::string dev_prepare_mixed(const Plan& P, DevState& D, int kc) {
     FMMG_TRY(prep(D.cM2MUp, D.tM2MUp, D.m2mUp32, fold, (int)ue, (int)(8 * ue)));
     // the parent's part of a child's downward density: C2E down x L2L
     double* G = nullptr;
+    tmp.next();
     FMMG_TRY(tmp.get(G, 8 * de * de));
     FMMG_TRY(dn_fold(P, D, G, tmp));
     FMMG_TRY(prepare_operator(D.stream, D.cDnFold, D.tDnFold, D.dnFold32, G, (int)(8 * de), (int)de, alloc));
