@@ -437,14 +437,14 @@ def run_ours(args):
 
 
 # DRAM traffic of the dominant kernels from one ncu capture each (dram__bytes_read.sum +
-# dram__bytes_write.sum) on the 262,144-point case of this workload, with the
+# dram__bytes_write.sum) on 262,144 points of this workload's distribution, with the
 # algorithmic bytes of that launch; a full launch's traffic is scaled by the
 # algorithmic bytes (the units processed).  Summaries under profiles/.
 TRAFFIC = {
     ("m2l_had", "mixed", 8): {"dram_bytes": 859.948800e6 + 571.790592e6, "algorithmic_bytes": 1209899328,
                                "profile": "profiles/k_m2l_had_o4_laplace_sphere_clusters_262k_np6_k8.md"},
-    ("m2l_had", "fp64", 1): {"dram_bytes": 253.321472e6 + 175.060480e6, "algorithmic_bytes": 424424448,
-                              "profile": "profiles/k_m2l_had_pq_fp64_laplace_sphere_clusters_262k_np6.md"},
+    ("m2l_had", "fp64", 1): {"dram_bytes": 247.265536e6 + 178.162944e6, "algorithmic_bytes": 424972800,
+                              "profile": "profiles/fp64_kernels_laplace_262k_stokes_60k_np6.md"},
 }
 
 

@@ -84,9 +84,9 @@ __device__ __forceinline__ void hd_cmac(float2& a, float2 t, float2 x) {
 // 64 pairs of a neighbour unrolled by child offset.  The spectra of the next
 // neighbour's 8 children load while this one's are multiplied.  That matters:
 // with an index table between the offset and the translation and the spectra
-// loaded where they are used, the FP64 pipe, the shared-memory path (108 cycles
-// of reads a neighbour for 128 of multiply-adds) and L2 were all under half
-// busy.  FP64: 1M points 3.88 -> 3.42 ms, 131,072 points 0.50 -> 0.38 ms; FP32
+// loaded where they are used, the FP64 pipe was 49 % busy, the shared-memory path
+// (108 cycles of reads a neighbour for 128 of multiply-adds) 56 %, now 55 % and
+// 53 %, warps waiting for the pipe before all else.  FP64: 1M points 3.88 -> 3.42 ms, 131,072 points 0.50 -> 0.38 ms; FP32
 // k = 1, 100,000 points 0.235 -> 0.164 ms.
 //
 // Rows are output parents.  rowOut[8*b + c] is the spectrum row of child c of

@@ -282,8 +282,9 @@ __global__ void __launch_bounds__(SURF_THREADS)
 // all its outputs, with the N / 2 roots of unity it needs in registers (loops
 // unrolled, so each product names its root; the other half are their
 // negatives).  One thread an output read an input and a root from shared memory
-// for every product, and that path was 82 % busy.  1M points, np = 6: forward
-// 0.58 -> 0.24 ms, inverse 0.57 -> 0.24 ms.
+// for every product, and that path was 89 % busy in the forward and 79 % in the
+// inverse (now 48 and 61 %).  1M points, np = 6: forward 0.58 -> 0.24 ms, inverse
+// 0.57 -> 0.24 ms.
 template <int NP>
 constexpr int fft64_threads() {  // the z pass's lines in whole warps
   return (FftDims<NP>::NH * FftDims<NP>::N + 31) / 32 * 32;
