@@ -169,8 +169,10 @@ struct DevState {
   std::vector<Block> spare;
 };
 
-// FP32 near field: the blocks of tb targets that the fullest leaf takes (grid.y; a
+// FP32 near field: the leaves above which a warp a leaf fills the GPU (48 warps an
+// SM); and the blocks of tb targets that the fullest leaf takes (grid.y; a
 // leaf of more than 64 blocks loops)
+inline int near_warps(int numSMs) { return 48 * numSMs; }
 inline unsigned near_blocks(const DevState& D, int tb) {
   const int64_t b = (D.maxLeafTrg + tb - 1) / tb;
   return (unsigned)(b < 1 ? 1 : (b > 64 ? 64 : b));

@@ -145,11 +145,6 @@ __device__ __forceinline__ void mx_den(const float* __restrict__ s, float (&d)[N
 // alone, and as the lower-priority stream's work it held the SMs that the
 // chain of row GEMMs beside it was waiting for: Laplace double layer, 50,021
 // sources and 30,011 targets apart, k = 3: 1.06 -> 0.30 ms.
-// WS: the CTA's 4 warps share a leaf with fewer than 100 leaves an SM, 48 where a
-// source carries 24 densities or more (its staging, which a warp alone does once
-// for a leaf, weighs more).  ms with 1 and with 4: Stokes, k 4, 9,100 leaves 0.97
-// and 0.72, 21,600 leaves 1.73 and 1.90; Laplace double layer, k 4, 0.60 and 0.40,
-// 0.89 and 1.04, its k 8 0.61 and 0.54, 1.15 and 1.42; 312, k 8, 0.48 and 0.60.
 constexpr int NX_WARPS = 4, NX_CH = 32, NX_MAXE = 128, NX_R = 2;
 template <int KT, int KB, int WS>
 __global__ void __launch_bounds__(32 * NX_WARPS)
@@ -1582,7 +1577,7 @@ static void run_mixed_blocks(const Plan& P, DevState& D, int kc, int mask, bool 
   auto near = [&](const int64_t* ptr, const int32_t* idx, cudaStream_t sn) {
     if (nl == 0) return;
     constexpr int TB = 64;  // two targets a lane
-    const bool few = nl < (KT == LAP_S_U || KTraits<KT>::SD * KB >= 24 ? 48 : 100) * D.numSMs;  // see the kernels
+    const bool few = nl < near_warps(D.numSMs);
     const dim3 grid(few ? nl : (nl + NW_WARPS - 1) / NW_WARPS, near_blocks(D, few ? TB / 2 : TB), kb);
     if constexpr (KT == LAP_S_U) {  // packed FP32x2
       auto* k = few ? k_p2p_near32_lap2w<KB, NW_WARPS> : k_p2p_near32_lap2w<KB, 1>;
