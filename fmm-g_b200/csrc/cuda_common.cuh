@@ -60,14 +60,15 @@ struct FftDims32 {
 };
 
 // The sums over the S groups of TG lanes of a warp (lane = group TG + place) of
-// each value, in the first group's lanes: the upper half of the groups onto the
-// lower, a logarithmic number of times (one group after another took S - 1 steps:
-// with a point or two a leaf S is 32, and the sums took longer than the pairs).
+// each value, in the first group's lanes: the upper groups onto the lower ones, a
+// logarithmic number of times (one group after another took S - 1 steps: with a
+// point or two a leaf S is 32, and the sums took longer than the pairs).
 template <int A, int B>
 __device__ __forceinline__ void group_sum(double (&v)[A][B], int lane, int sp, int TG, int S) {
-  for (int n = S; n > 1;) {
-    const int h = (n + 1) >> 1;
-    const bool add = sp + h < n;
+#pragma unroll
+  for (int h = 16; h > 0; h >>= 1) {
+    if (h >= S) continue;
+    const bool add = sp < h && sp + h < S;
 #pragma unroll
     for (int a = 0; a < A; a++)
 #pragma unroll
@@ -75,7 +76,6 @@ __device__ __forceinline__ void group_sum(double (&v)[A][B], int lane, int sp, i
         const double o = __shfl_sync(0xffffffffu, v[a][b], (lane + h * TG) & 31);
         if (add) v[a][b] += o;
       }
-    n = h;
   }
 }
 

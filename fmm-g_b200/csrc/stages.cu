@@ -144,7 +144,17 @@ __global__ void __launch_bounds__(32 * WARPS)
         }
       }
     }
-    group_sum(acc, lane, sp, TG, S);
+    if (WPR == 1 || S > 4) {
+      group_sum(acc, lane, sp, TG, S);
+    } else {  // few groups, as M2T has: M2T 2 % faster than with group_sum alone
+#pragma unroll
+      for (int r = 0; r < PR; r++)
+#pragma unroll
+        for (int c = 0; c < TD; c++) {
+          const double own = acc[r][c];
+          for (int k = 1; k < S; k++) acc[r][c] += __shfl_sync(0xffffffffu, own, (lane + k * TG) & 31);
+        }
+    }
     if constexpr (WPR == 1) {
       if (sp == 0) {
 #pragma unroll
