@@ -170,9 +170,13 @@ struct DevState {
 };
 
 // FP32 near field: the leaves above which a warp a leaf fills the GPU (48 warps an
-// SM); and the blocks of tb targets that the fullest leaf takes (grid.y; a
-// leaf of more than 64 blocks loops)
+// SM).  The kernel alone is faster with a CTA a leaf up to about 100 leaves an SM
+// (Stokes, k 4, 9,100 leaves 0.72 and 0.97 ms), the calls are not: it holds the
+// SMs that the chain beside it waits for (kernel 312, 202,327 sources, 101,164
+// targets apart, k 3: 5.17 and 5.45 ms).
 inline int near_warps(int numSMs) { return 48 * numSMs; }
+// the blocks of tb targets that the fullest leaf takes (grid.y; a leaf of more
+// than 64 blocks loops)
 inline unsigned near_blocks(const DevState& D, int tb) {
   const int64_t b = (D.maxLeafTrg + tb - 1) / tb;
   return (unsigned)(b < 1 ? 1 : (b > 64 ? 64 : b));
