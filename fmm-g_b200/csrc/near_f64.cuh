@@ -19,7 +19,7 @@
 // as separate CTAs (grid.y).  No CTA-wide barrier in the loops.
 // Against one warp (evaluate) or one barrier-bound CTA (adjoint) a leaf with one
 // point a lane: 65,536 points in 554 leaves 2.58 -> 0.37 ms, Stokes 60,007 points
-// 1.28 -> 0.28, 1M points in 62,000 leaves 2.15 -> 1.54; target gradient of 131,072
+// 1.28 -> 0.28, 1M points in 62,000 leaves 2.15 -> 1.51; target gradient of 131,072
 // points 0.357 -> 0.293 ms, transposed sums 0.318 -> 0.225 ms.
 #pragma once
 

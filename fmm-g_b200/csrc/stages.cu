@@ -79,7 +79,7 @@ constexpr int P2P_MAXE = 256;
 // targets each, TG = ceil(targets / PR) a group, S = 32 / TG groups that split the
 // surface points.  The unit surface is staged for the CTA, a node's densities in
 // the warp's slice of shared memory; with WPR = 8 the warps' sums meet there in
-// warp order.  1M points M2T 0.67 -> 0.38 ms (8 warps a leaf 0.34), L2T 0.46 -> 0.41;
+// warp order.  1M points M2T 0.67 -> 0.37 ms (8 warps a leaf 0.34), L2T 0.46 -> 0.39;
 // Stokes 60,007 points M2T 0.64 -> 0.29 ms (8 warps 0.40).
 constexpr int E2T_L2T_WARPS = 4;
 template <int KM>
